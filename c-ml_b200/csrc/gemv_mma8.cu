@@ -381,6 +381,10 @@ int cmlb200_gemv_mma8_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const floa
     return quirk ? launch8<true>(W, W2, x, nw, eps, y, M, epi, st) : launch8<false>(W, W2, x, nw, eps, y, M, epi, st);
 }
 
+bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W);          // gemv_split.cu
+
 extern "C" int cmlb200_gemv_batched_from_planes(const cmlb200_qmat* W) {
-    return W && W->qs && W->scales && W->rows > 0 && W->cols > 0 && cmlb200_gemv_mma8_ok_(W, EPI_STORE) && cmlb200_gemv_mma8_ok_(W, EPI_SWIGLU) ? 1 : 0;
+    if (!W || !W->qs || !W->scales || W->rows <= 0 || W->cols <= 0) return 0;
+    if (W->type == CMLB200_Q8_0) return cmlb200_gemv_split_ok_(W) ? 1 : 0;
+    return cmlb200_gemv_mma8_ok_(W, EPI_STORE) && cmlb200_gemv_mma8_ok_(W, EPI_SWIGLU) ? 1 : 0;
 }

@@ -1,0 +1,760 @@
+// Decode GEMV, 1 to 32 rows of x, every block format C-ML reads (Q4_0, Q4_1, Q8_0, Q4_K, Q5_K, Q6_K of
+// src/core/gguf_quant.c:66-311 and NF4 of src/core/quantization.c:195-370), on fp16 tensor cores
+// (mma.sync m16n8k16, fp32 accumulation) with 32-bit accuracy:
+//   * the quants are small integers, which fp16 holds exactly: A = 16 weight rows x 16 quants, made in registers with
+//     one or two logic / packed-half operations per register;
+//   * x is split into two fp16 numbers, x = hi + lo, after scaling by a power of two that puts the largest value of its
+//     slice just below 2^9: 22 bits of every value, and nothing below 2^-32 of the largest is lost;
+//   * products and sums of one block are fp32 in the tensor core; block scales are applied to its sums in fp32, the
+//     minima of Q4_K / Q5_K by one more small product (sub-block minima times sums of x), those of Q4_1 in fp32.
+// Error against 64 bits on N(0,1) inputs: 1.2e-7 to 2e-7 of the result's norm, as the int8-digit kernels have.
+//
+// Work: item = 16 weight rows x 256 columns; the warps of a CTA share K (a warp takes every W-th 256-column unit), each
+// with a ring of its own that cp.async fills, the first items before the launch waits for its predecessor. Sums of the
+// warps meet in shared memory and are added in warp order, so results do not depend on timing.
+//
+//   gemv_split_kernel   up to 8 rows of x. NT = 0: up to 4 rows, made into hi / lo columns of ONE 8-column product by the
+//                       warp itself (columns 2r, 2r+1 = hi, lo of row r); NT = 1: 5 to 8 rows, planes from x_split_kernel.
+//                       A warp keeps the B operands of its unit in registers and walks the CTA's row tiles.
+//   gemv_split_wide_kernel   9 to 32 rows: B operands are loaded per block and used by T row tiles whose sums stay in registers;
+//                       16 columns of x a warp, from 17 rows on two warps share a part of K.
+//
+// What bounds it: instructions. 50 a block of 16 x 32 weights at M = 1 (10 to unpack, 6 to address and load, 2 products, 8 to apply the
+// scales, the rest the rows of x), 65 a warp and block at M = 32, at an issue rate of 0.42 to 0.66 a scheduler; tensor pipe 41 % busy
+// at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers) beat eight with 255: 8.2
+// against 10.4 us at M = 1, 16.1 against 14.7 at M = 32 but 9.9 against 11.4 at M = 16 (Q4_0 11008x4096, 4096x4096). More chains of
+// products (the block's halves apart) cost more additions than they hid: 14.3 against 12.9 us at M = 8. Times: gemv.cu.
+#pragma once
+#include "common.cuh"
+#include "mma_util.cuh"
+
+#ifndef UNROLL_B
+#define UNROLL_B 1
+#endif
+namespace {
+
+enum { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2 };
+
+// Shared memory of one weight row's 256-column unit: bytes of quants (and headers) as they lie in memory, block scales
+// behind them. Row strides are odd multiples of 16 bytes (mod 128), so eight rows hit eight bank groups.
+template <int F> struct Lay;
+template <> struct Lay<CMLB200_Q4_0> { static constexpr int ROW = 144, CH = 8, SC = 128; };
+template <> struct Lay<CMLB200_Q8_0> { static constexpr int ROW = 272, CH = 16, SC = 256; };
+template <> struct Lay<CMLB200_NF4> { static constexpr int ROW = 176, CH = 8, SC = 128; };
+template <> struct Lay<CMLB200_Q4_1> { static constexpr int ROW = 176, CH = 10, SC = 0; };
+template <> struct Lay<CMLB200_Q4_K> { static constexpr int ROW = 144, CH = 9, SC = 0; };
+template <> struct Lay<CMLB200_Q5_K> { static constexpr int ROW = 176, CH = 11, SC = 0; };
+template <> struct Lay<CMLB200_Q6_K> { static constexpr int ROW = 240, CH = 15, SC = 0; };   // the aligned window around 210 bytes
+template <int F> constexpr int kTileBytes = 16 * Lay<F>::ROW;
+template <int F> constexpr bool kMins = F == CMLB200_Q4_1 || F == CMLB200_Q4_K || F == CMLB200_Q5_K;     // formats with minima
+
+struct SplitArgs {
+    const uint8_t *qs, *qs2;       // weight, second weight (SwiGLU: gate, up)
+    const uint8_t *sc, *sc2;       // scales (Q4_0, Q8_0: fp16, NF4: fp32)
+    const float* x;                // fp32 rows (NT = 0)
+    const __half* nw;              // RMSNorm weight applied to them, or nullptr
+    const uint4* planes;           // split rows (NT > 0): [block][NT][hi, lo][lane]
+    const float* sums;             // their sums over blocks: [block][8 NT]
+    const float* xf;               // power of two that undoes the scaling, per row
+    float* y;
+    float eps;
+    int N, K, M, tiles, per_cta, stages, epi;
+    int nf4_shift;                 // log2 of how many 32-column blocks one NF4 scale covers, 3 at most
+    int nf4_units;                 // units one covers, 1 at least
+};
+
+// Shared memory through pointers, so that the compiler may order the loads as it likes between the waits
+typedef const uint8_t* Shared;
+__device__ __forceinline__ uint32_t lds32(Shared p) { return *reinterpret_cast<const uint32_t*>(p); }
+__device__ __forceinline__ uint32_t lds16(Shared p) { return *reinterpret_cast<const uint16_t*>(p); }
+__device__ __forceinline__ float ldsf(Shared p) { return *reinterpret_cast<const float*>(p); }
+__device__ __forceinline__ void cp_async16_part(uint32_t dst, const void* src, int bytes) {     // the rest is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4_part(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t m, uint32_t o) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(m), "r"(o));
+    return d;
+}
+__device__ __forceinline__ uint32_t hfma2u(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t hadd2u(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+constexpr float kNF4Unit = 16384.0f / 10000.0f;      // what a product of NF4 digits counts
+
+// ---- weights: global memory -> ring ---------------------------------------------------------------------------------
+template <int F> __device__ __forceinline__ size_t row_bytes(int nblk) {
+    return F == CMLB200_Q8_0 ? (size_t)nblk * 32 : F == CMLB200_Q4_1 ? (size_t)nblk * 20 : F == CMLB200_Q4_K ? (size_t)nblk * 18 :
+           F == CMLB200_Q5_K ? (size_t)nblk * 22 : F == CMLB200_Q6_K ? (size_t)nblk / 8 * 210 : (size_t)nblk * 16;
+}
+// Where a lane's 16-byte pieces of an item lie from its first row on (items whose 16 rows all exist)
+template <int F> struct Pieces {
+    static constexpr int CH = Lay<F>::CH, COUNT = (16 * CH + 31) / 32;
+    uint32_t off[F == CMLB200_Q6_K ? 1 : COUNT];
+    __device__ __forceinline__ void init(int nblk, int lane) {
+        if constexpr (F != CMLB200_Q6_K) {
+#pragma unroll
+            for (int i = 0; i < COUNT; i++) {
+                const int c = lane + 32 * i;
+                off[i] = (uint32_t)(c / CH) * (uint32_t)row_bytes<F>(nblk) + (uint32_t)(c % CH) * 16u;
+            }
+        }
+    }
+};
+// One item: rows row0 .. row0+15 (rows past N repeat row N-1; never written out), columns of unit `un`.
+template <int F>
+__device__ __forceinline__ void issue_tile(const SplitArgs& p, const Pieces<F>& pc, int which, int row0, int un, uint32_t dst, int lane) {
+    constexpr int ROW = Lay<F>::ROW, CH = Lay<F>::CH;
+    const int nblk = p.K / 32, last = p.N - 1;
+    const uint8_t *qs = which ? p.qs2 : p.qs, *sc = which ? p.sc2 : p.sc;
+    const size_t rb = row_bytes<F>(nblk);
+    if (F == CMLB200_Q6_K) {
+        const size_t total = rb * p.N;
+#pragma unroll
+        for (int i = 0; i < (16 * CH + 31) / 32; i++) {
+            const int c = lane + 32 * i, r = c / CH, ch = c % CH;
+            if (c < 16 * CH) {
+                const size_t o = (size_t)min(row0 + r, last) * rb + (size_t)un * 210, at = (o & ~(size_t)15) + 16 * ch;
+                const int n = at >= o + 210 ? 0 : (total - at < 16 ? (int)(total - at) : 16);
+                cp_async16_part(dst + r * ROW + ch * 16, n ? qs + at : qs, n);
+            }
+        }
+        return;
+    }
+    if (row0 + 16 <= p.N && (un + 1) * 8 <= nblk) {
+        const uint8_t* base = qs + (size_t)row0 * rb + (size_t)un * (CH * 16);
+#pragma unroll
+        for (int i = 0; i < Pieces<F>::COUNT; i++) {
+            const int c = lane + 32 * i;
+            if (16 * CH % 32 == 0 || c < 16 * CH) cp_async16(dst + (c / CH) * ROW + (c % CH) * 16, base + pc.off[F == CMLB200_Q6_K ? 0 : i]);
+        }
+    } else {
+        const int left = nblk - un * 8;                                      // blocks of the unit that exist
+        const int have = F == CMLB200_Q8_0 ? 2 * left : F == CMLB200_Q4_0 || F == CMLB200_NF4 ? left : CH;
+#pragma unroll 1
+        for (int c = lane; c < 16 * CH; c += 32) {
+            const int r = c / CH, ch = c % CH;
+            const uint8_t* src = qs + (size_t)min(row0 + r, last) * rb + (size_t)un * (CH * 16) + ch * 16;
+            cp_async16_part(dst + r * ROW + ch * 16, ch < have ? src : qs, ch < have ? 16 : 0);
+        }
+    }
+    if (F == CMLB200_Q4_0 || F == CMLB200_Q8_0) {
+        if (lane < 16) cp_async16(dst + lane * ROW + Lay<F>::SC, sc + 2 * ((size_t)min(row0 + lane, last) * nblk + (size_t)un * 8));
+    } else if (F == CMLB200_NF4) {                                          // absmax: one for a few blocks, or for units
+        const int ws = 3 - p.nf4_shift, words = 1 << ws, per_row = (nblk >> p.nf4_shift) / p.nf4_units, first = (un << ws) / p.nf4_units;
+        for (int c = lane; c < 16 * words; c += 32) {
+            const int r = c >> ws, k = c & (words - 1);
+            const bool ok = first + k < per_row;
+            const uint8_t* src = sc + 4 * ((size_t)min(row0 + r, last) * per_row + first + k);
+            cp_async4_part(dst + r * ROW + Lay<F>::SC + 4 * k, ok ? src : sc, ok ? 4 : 0);
+        }
+    }
+}
+
+// ---- weights: ring -> A operands --------------------------------------------------------------------------------------
+// A thread (g, t) = (lane / 4, lane % 4) of the product holds rows g and g + 8. Of a 32-column block it takes columns 4t .. 4t+3
+// and 16+4t .. 16+4t+3 (NF4: 8t .. 8t+7), in the order (0,2) (1,3) (4,6) (5,7) of the eight; the B operands have the same order,
+// and the order of columns inside a product is free. a[0], a[1]: the two m16n8k16 of the block; NF4: two digits of the value.
+template <int F> constexpr int kDigits = F == CMLB200_NF4 ? 2 : 1;
+
+// 4-bit formats: word w holds the eight nibbles of one row
+__device__ __forceinline__ void nibbles(uint32_t w, uint32_t magic, uint32_t (&h)[4]) {
+    const uint32_t v = w >> 8;
+    h[0] = and_or(w, 0x000f000fu, magic);
+    h[1] = and_or(v, 0x000f000fu, magic);
+    h[2] = and_or(w, 0x00f000f0u, magic);
+    h[3] = and_or(v, 0x00f000f0u, magic);
+}
+
+template <int F>
+__device__ __forceinline__ void row_regs(Shared at, int b, int t, uint32_t w0, uint32_t w1, uint32_t off, uint32_t (&h)[kDigits<F>][4]) {
+    if constexpr (F == CMLB200_Q4_0 || F == CMLB200_Q4_1 || F == CMLB200_Q4_K) {     // q - 8 from 1024 + q and 1024 + 16 q
+        uint32_t n[4];
+        nibbles(w0, 0x64006400u, n);
+        h[0][0] = hadd2u(n[0], 0xe408e408u);                     // - 1032
+        h[0][1] = hadd2u(n[1], 0xe408e408u);
+        h[0][2] = hfma2u(n[2], 0x2c002c00u, 0xd480d480u);        // / 16 - 72
+        h[0][3] = hfma2u(n[3], 0x2c002c00u, 0xd480d480u);
+    } else if constexpr (F == CMLB200_Q8_0) {                   // int8 from 1024 + (q + 128)
+        const uint32_t u0 = w0 ^ 0x80808080u, u1 = w1 ^ 0x80808080u;
+        h[0][0] = hadd2u(__byte_perm(u0, 0x64646464u, 0x4240), 0xe480e480u);
+        h[0][1] = hadd2u(__byte_perm(u0, 0x64646464u, 0x4341), 0xe480e480u);
+        h[0][2] = hadd2u(__byte_perm(u1, 0x64646464u, 0x4240), 0xe480e480u);
+        h[0][3] = hadd2u(__byte_perm(u1, 0x64646464u, 0x4341), 0xe480e480u);
+    } else if constexpr (F == CMLB200_Q5_K) {                   // bit 4 from the block's word of high bits: w1 = bits of columns 0..31
+        const uint32_t v = w0 >> 4, b4 = w1 >> (4 * t);          // bits 0-3: columns 4t.., bits 16-19: columns 16+4t..
+        // columns 0 and 2 (1 and 3) of the four: bits 0 and 2 (1 and 3) to bit 4 of the two halves, by a multiplication; q - 16 from 1024 + q
+        const uint32_t top = b4 >> 16;
+        h[0][0] = hadd2u(and_or((b4 & 5u) * 0x00040010u, 0x00100010u, and_or(w0, 0x000f000fu, 0x64006400u)), 0xe410e410u);
+        h[0][1] = hadd2u(and_or((b4 & 10u) * 0x00020008u, 0x00100010u, and_or(w0 >> 8, 0x000f000fu, 0x64006400u)), 0xe410e410u);
+        h[0][2] = hadd2u(and_or((top & 5u) * 0x00040010u, 0x00100010u, and_or(v, 0x000f000fu, 0x64006400u)), 0xe410e410u);
+        h[0][3] = hadd2u(and_or((top & 10u) * 0x00020008u, 0x00100010u, and_or(v >> 8, 0x000f000fu, 0x64006400u)), 0xe410e410u);
+    } else if constexpr (F == CMLB200_Q6_K) {                   // q - 32 from 1024 + q
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t q = lds16(at + off + 16 * b + 8 * k + 2 * t), hb = at[off + 128 + 8 * b + 4 * k + t];
+            const uint32_t w = __byte_perm(q, 0, 0x4140), hh = hb | (hb << 16);
+            const uint32_t e = and_or(w, 0x000f000fu, 0x64006400u), o = and_or(w >> 4, 0x000f000fu, 0x64006400u);
+            h[0][2 * k] = hadd2u(e | ((hh << 4) & 0x00000030u) | (hh & 0x00300000u), 0xe420e420u);              // - 1056
+            h[0][2 * k + 1] = hadd2u(o | ((hh << 2) & 0x00000030u) | ((hh >> 2) & 0x00300000u), 0xe420e420u);
+        }
+    } else {                                                    // NF4: 10000 times the code = 128 a + b, digits by byte table look-ups
+        // a + 128 and b + 128 of the 16 codes (|b| <= 64), four to a word
+        constexpr uint32_t A0 = 0x61574a32u, A1 = 0x8079726au, A2 = 0x9a938d86u, A3 = 0xceb8aca2u;
+        constexpr uint32_t B0 = 0x937d4e70u, B1 = 0x80714864u, B2 = 0xb39d499cu, B3 = 0x90be7ab7u;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t w = k ? w0 >> 16 : w0;
+            const uint32_t s = w & 0x7777u, pick = and_or(w >> 1, 0x4444u, 0x3210u);
+            const uint32_t va = __byte_perm(__byte_perm(A0, A1, s), __byte_perm(A2, A3, s), pick);
+            const uint32_t vb = __byte_perm(__byte_perm(B0, B1, s), __byte_perm(B2, B3, s), pick);
+            // bytes: columns 1, 0, 3, 2. 1024 + (a + 128) -> a * 2^-7, 1024 + (b + 128) -> b * 2^-14
+            h[0][2 * k] = hfma2u(__byte_perm(va, 0x64646464u, 0x4341), 0x20002000u, 0xc880c880u);
+            h[0][2 * k + 1] = hfma2u(__byte_perm(va, 0x64646464u, 0x4240), 0x20002000u, 0xc880c880u);
+            h[1][2 * k] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4341), 0x04000400u, 0xac80ac80u);
+            h[1][2 * k + 1] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4240), 0x04000400u, 0xac80ac80u);
+        }
+    }
+}
+
+// The words of block b that row_regs wants (row at shared address `at`)
+template <int F>
+__device__ __forceinline__ void row_words(Shared at, int b, int t, uint32_t& w0, uint32_t& w1) {
+    if (F == CMLB200_Q4_0 || F == CMLB200_NF4) w0 = lds32(at + 16 * b + 4 * t);
+    else if (F == CMLB200_Q8_0) { w0 = lds32(at + 32 * b + 4 * t); w1 = lds32(at + 32 * b + 16 + 4 * t); }
+    else if (F == CMLB200_Q4_1) w0 = lds32(at + 20 * b + 4 + 4 * t);
+    else if (F == CMLB200_Q4_K) w0 = lds32(at + 16 + 16 * b + 4 * t);
+    else if (F == CMLB200_Q5_K) { w0 = lds32(at + 48 + 16 * b + 4 * t); w1 = lds32(at + 16 + 4 * b); }
+}
+
+template <int F>
+__device__ __forceinline__ void block_regs(Shared lo, Shared hi, int b, int t, uint32_t off_lo, uint32_t off_hi, uint32_t (&a)[kDigits<F>][2][4]) {
+    uint32_t w0 = 0, w1 = 0, v0 = 0, v1 = 0, r[kDigits<F>][4], s[kDigits<F>][4];
+    row_words<F>(lo, b, t, w0, w1);
+    row_words<F>(hi, b, t, v0, v1);
+    row_regs<F>(lo, b, t, w0, w1, off_lo, r);
+    row_regs<F>(hi, b, t, v0, v1, off_hi, s);
+#pragma unroll
+    for (int d = 0; d < kDigits<F>; d++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            a[d][k][0] = r[d][2 * k];
+            a[d][k][1] = s[d][2 * k];
+            a[d][k][2] = r[d][2 * k + 1];
+            a[d][k][3] = s[d][2 * k + 1];
+        }
+}
+
+// What a row's header says, decoded once per item
+struct Head { float d, m; uint32_t s0, s1, m0, m1, off; };
+
+template <int F>
+__device__ __forceinline__ void head_of(const SplitArgs& p, Shared at, int row, int un, Head& h) {
+    if (F == CMLB200_Q4_K || F == CMLB200_Q5_K) {
+        const uint4 v = *reinterpret_cast<const uint4*>(at);
+        h.d = cml_half_to_float((uint16_t)(v.x & 0xffffu));
+        h.m = cml_half_to_float((uint16_t)(v.x >> 16));
+        h.s0 = v.y & 0x3f3f3f3fu;                                                  // scales of sub-blocks 0-3, 4-7, then minima
+        h.s1 = (v.w & 0x0f0f0f0fu) | ((v.y >> 2) & 0x30303030u);
+        h.m0 = v.z & 0x3f3f3f3fu;
+        h.m1 = ((v.w >> 4) & 0x0f0f0f0fu) | ((v.z >> 2) & 0x30303030u);
+    } else if (F == CMLB200_Q6_K) {
+        const size_t o = (size_t)min(row, p.N - 1) * ((size_t)p.K / 256 * 210) + (size_t)un * 210;
+        h.off = (uint32_t)(o & 15);
+        h.d = cml_half_to_float((uint16_t)lds16(at + h.off + 208));
+    }
+}
+
+// Scale of block b (Q6_K: of its half `k`)
+template <int F, bool QUIRK>
+__device__ __forceinline__ float scale_of(const SplitArgs& p, Shared at, const Head& h, int b, int k) {
+    if (F == CMLB200_Q4_0 || F == CMLB200_Q8_0) {
+        const uint16_t s = (uint16_t)lds16(at + Lay<F>::SC + 2 * b);
+        return QUIRK ? cml_half_to_float(s) : __half2float(__ushort_as_half(s));
+    }
+    if (F == CMLB200_NF4) return ldsf(at + Lay<F>::SC + 4 * (b >> p.nf4_shift)) * kNF4Unit;
+    if (F == CMLB200_Q4_1) return cml_half_to_float((uint16_t)lds16(at + 20 * b));
+    if (F == CMLB200_Q6_K) return h.d * (float)(int)(int8_t)at[h.off + 192 + 2 * b + k];
+    return h.d * (float)(((b < 4 ? h.s0 : h.s1) >> (8 * (b & 3))) & 255u);
+}
+
+// What block b adds per sum of x: its minimum, and what the centring of its quants took off
+template <int F>
+__device__ __forceinline__ float offset_of(Shared at, const Head& h, int b, float scale) {
+    if (F == CMLB200_Q4_1) return fmaf(8.0f, scale, cml_half_to_float((uint16_t)lds16(at + 20 * b + 2)));
+    const float mn = h.m * (float)(((b < 4 ? h.m0 : h.m1) >> (8 * (b & 3))) & 255u);
+    return fmaf(F == CMLB200_Q5_K ? 16.0f : 8.0f, scale, -mn);
+}
+
+// ---- activations --------------------------------------------------------------------------------------------------------
+// The power of two that brings values of magnitude up to `most` below 2^9, and its inverse
+__device__ __forceinline__ void scaling(float most, float& up, float& down) {
+    const int e = (int)(__float_as_uint(most) >> 23);
+    const int f = min(262 - e, 253);                            // exponent field of 2^(8 - floor(log2 most))
+    up = __uint_as_float((uint32_t)f << 23);
+    down = __uint_as_float((uint32_t)(254 - f) << 23);
+}
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// ---- up to 8 rows of x ------------------------------------------------------------------------------------------------------
+constexpr int kWarps = 16;
+template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 ? 2 : Lay<F>::ROW == 144 && NT ? 4 : 3;      // items per warp in flight
+constexpr int kOwnBytes = 16 + 4 * 8 * 4;                                // NT = 0: a warp's scaling and block sums of its rows, behind the operands
+constexpr int kXBytes = 2 * 8 * 4 * 16;                                  // operands of one row and unit: [hi, lo][block][t]
+
+template <int F, int NT, bool QUIRK>
+__global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitArgs p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, RING = kRing<F, NT>, COLS = NT == 0 ? 4 : 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // shared memory: rings [W][RING][TB] | NT = 0: operands [W][M][kXBytes], scaling and sums [W][kOwnBytes] | sums [per_cta][W][COLS][16] | squares [W][4]
+    Shared rings = smem + warp * (RING * TB);
+    const uint32_t ring = smem_u32(rings);
+    uint8_t* xs = smem + W * (RING * TB) + warp * (p.M * kXBytes);
+    float* own = reinterpret_cast<float*>(smem + W * (RING * TB) + W * (p.M * kXBytes) + warp * kOwnBytes);
+    float* part = reinterpret_cast<float*>(smem + W * (RING * TB) + (NT == 0 ? W * (p.M * kXBytes + kOwnBytes) : 0));
+    float* squares = part + (size_t)p.per_cta * W * COLS * 16;
+    const int units = (p.K + 255) / 256, nblk = p.K / 32, pairs = p.epi == EPI_SWIGLU;
+    const int tile0 = blockIdx.x * p.per_cta, mine = min(p.per_cta, p.tiles - tile0);
+    const int my_units = warp < units ? (units - warp + W - 1) / W : 0, items = my_units * mine;
+    Pieces<F> pc;
+    pc.init(nblk, lane);
+    int iss = 0, iss_tile = 0, iss_un = warp;
+    auto issue = [&](int buf) {
+        if (iss < items) {
+            const int tile = tile0 + iss_tile;
+            issue_tile<F>(p, pc, pairs ? tile & 1 : 0, (pairs ? tile >> 1 : tile) * 16, iss_un, ring + buf * TB, lane);
+            iss++;
+            if (++iss_tile == mine) { iss_tile = 0; iss_un += W; }
+        }
+        cp_async_commit();
+    };
+    // weights do not depend on the launch before (NF4 ones may: it may have quantized them)
+    if (F == CMLB200_NF4) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < RING; i++) issue(i);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    float ss[4] = {0.f, 0.f, 0.f, 0.f};
+    int buf = 0;
+    for (int u = 0; u < my_units; u++) {
+        const int un = warp + u * W;
+        uint32_t B[8][NT == 0 ? 4 : 8];                         // NT = 0: hi (even g) or lo (odd g) of row g/2; 1: hi, then lo of row g
+        float s32[kMins<F> ? 8 : 1][2];                         // sums of x over the unit's blocks, of the thread's two columns
+        float down = 1.f;
+        if (NT == 0) {
+            // one row at a time, eight columns a lane: block lane/4, the columns of thread t = lane%4 of the product
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                if (m >= p.M) break;
+                float e[8];
+                const int c0 = un * 256 + g * 32 + (F == CMLB200_NF4 ? 8 : 4) * t, c1 = F == CMLB200_NF4 ? c0 + 4 : c0 + 16;
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
+                if (un * 8 + g < nblk) {
+                    a = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c0));
+                    c = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c1));
+                }
+                e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w; e[4] = c.x; e[5] = c.y; e[6] = c.z; e[7] = c.w;
+                if (p.nw && un * 8 + g < nblk) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(p.nw + c0), w = *reinterpret_cast<const uint2*>(p.nw + c1);
+                    const uint32_t h[4] = {v.x, v.y, w.x, w.y};
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[k]));
+                        ss[m] = fmaf(e[2 * k], e[2 * k], fmaf(e[2 * k + 1], e[2 * k + 1], ss[m]));
+                        e[2 * k] *= f.x;
+                        e[2 * k + 1] *= f.y;
+                    }
+                }
+                float most = 0.f, up, dn, sum = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; k++) most = fmaxf(most, fabsf(e[k]));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+                scaling(most, up, dn);
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int k = 0; k < 8; k++) { e[k] *= up; sum += e[k]; }
+#pragma unroll
+                for (int k = 0; k < 4; k++) split2(e[4 * (k >> 1) + (k & 1)], e[4 * (k >> 1) + (k & 1) + 2], hi[k], lo[k]);
+                uint4* dst = reinterpret_cast<uint4*>(xs + m * kXBytes) + lane;
+                dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                dst[32] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                if (kMins<F>) {
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    if (t == 0) own[4 + m * 8 + g] = sum;
+                }
+                if (lane == 0) own[m] = dn;
+            }
+            __syncwarp();
+            const bool there = (g >> 1) < p.M;
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (there) v = reinterpret_cast<const uint4*>(xs + (g >> 1) * kXBytes)[(g & 1) * 32 + 4 * b + t];
+                B[b][0] = v.x; B[b][1] = v.y; B[b][2] = v.z; B[b][3] = v.w;
+                if (kMins<F>) s32[kMins<F> ? b : 0][0] = t < p.M ? own[4 + t * 8 + b] : 0.f;
+            }
+            down = t < p.M ? own[t] : 0.f;
+        } else {
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                const uint4* src = p.planes + (size_t)(un * 8 + b) * 64 + lane;
+                const uint4 h = __ldcg(src), l = __ldcg(src + 32);
+                B[b][0] = h.x; B[b][1] = h.y; B[b][2] = h.z; B[b][3] = h.w;
+                B[b][NT ? 4 : 0] = l.x; B[b][NT ? 5 : 0] = l.y; B[b][NT ? 6 : 0] = l.z; B[b][NT ? 7 : 0] = l.w;
+                if (kMins<F>) {
+                    const float2 v = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * 8 + 2 * t));
+                    s32[kMins<F> ? b : 0][0] = v.x;
+                    s32[kMins<F> ? b : 0][1] = v.y;
+                }
+            }
+        }
+        for (int i = 0; i < mine; i++) {
+            const int tile = tile0 + i, row0 = (pairs ? tile >> 1 : tile) * 16;
+            cp_async_wait<RING - 1>();
+            __syncwarp();
+            Shared lo = rings + buf * TB + g * ROW, hi = lo + 8 * ROW;
+            Head hl, hh;
+            head_of<F>(p, lo, row0 + g, un, hl);
+            head_of<F>(p, hi, row0 + g + 8, un, hh);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                uint32_t a[kDigits<F>][2][4];
+                block_regs<F>(lo, hi, b, t, hl.off, hh.off, a);
+                float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                constexpr int C1 = F == CMLB200_Q6_K ? 1 : 0;   // Q6_K: a scale for each half
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+#pragma unroll
+                    for (int d = 0; d < kDigits<F>; d++) {
+                        mma_f16(c[k * C1], a[d][k], B[b][2 * k], B[b][2 * k + 1]);
+                        if (NT) mma_f16(c[k * C1], a[d][k], B[b][NT ? 4 + 2 * k : 0], B[b][NT ? 5 + 2 * k : 0]);
+                    }
+#pragma unroll
+                for (int k = 0; k <= C1; k++) {
+                    const float sl = scale_of<F, QUIRK>(p, lo, hl, b, k), sh = scale_of<F, QUIRK>(p, hi, hh, b, k);
+                    acc[0] = fmaf(c[k][0], sl, acc[0]);
+                    acc[1] = fmaf(c[k][1], sl, acc[1]);
+                    acc[2] = fmaf(c[k][2], sh, acc[2]);
+                    acc[3] = fmaf(c[k][3], sh, acc[3]);
+                    if (kMins<F> && k == 0) {
+                        const float ml = offset_of<F>(lo, hl, b, sl), mh = offset_of<F>(hi, hh, b, sh);
+                        const float x0 = s32[kMins<F> ? b : 0][0], x1 = s32[kMins<F> ? b : 0][1];
+                        acc[0] = fmaf(x0, ml, acc[0]);
+                        acc[2] = fmaf(x0, mh, acc[2]);
+                        if (NT) { acc[1] = fmaf(x1, ml, acc[1]); acc[3] = fmaf(x1, mh, acc[3]); }
+                    }
+                }
+            }
+            __syncwarp();                                       // every lane is done with this buffer
+            issue(buf);
+            if (++buf == RING) buf = 0;
+            float* dst = part + ((size_t)i * W + warp) * (COLS * 16);
+            if (NT == 0) {
+                float v0 = (acc[0] + acc[1]) * down, v1 = (acc[2] + acc[3]) * down;
+                dst += t * 16 + g;
+                if (u) { v0 += dst[0]; v1 += dst[8]; }
+                dst[0] = v0;
+                dst[8] = v1;
+            } else {
+                dst += 2 * t * 16 + g;
+                if (u) { acc[0] += dst[0]; acc[1] += dst[16]; acc[2] += dst[8]; acc[3] += dst[24]; }
+                dst[0] = acc[0];
+                dst[16] = acc[1];
+                dst[8] = acc[2];
+                dst[24] = acc[3];
+            }
+        }
+    }
+    if (NT == 0 && p.nw) {
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss[m] += __shfl_xor_sync(0xffffffffu, ss[m], o);
+            if (lane == 0) squares[warp * 4 + m] = ss[m];
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    const int active = min(W, units), outs = mine >> pairs;
+    for (int idx = threadIdx.x; idx < outs * COLS * 16; idx += blockDim.x) {
+        const int r = idx & 15, m = (idx >> 4) & (COLS - 1), o = idx / (COLS * 16);
+        const int row = ((pairs ? tile0 >> 1 : tile0) + o) * 16 + r;
+        if (m >= p.M || row >= p.N) continue;
+        float f = 1.f;
+        if (NT) f = __ldcg(p.xf + m);
+        else if (p.nw) {
+            float q = 0.f;
+            for (int w = 0; w < active; w++) q += squares[w * 4 + m];
+            f = 1.0f / sqrtf(q / (float)p.K + p.eps);
+        }
+        const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
+        float v = 0.f, v2 = 0.f;
+        for (int w = 0; w < active; w++) v += src[w * (COLS * 16)];
+        v *= f;
+        float* out = p.y + (size_t)m * p.N + row;
+        if (pairs) {
+            for (int w = 0; w < active; w++) v2 += src[(W + w) * (COLS * 16)];
+            *out = (v / (1.0f + expf(-v))) * (v2 * f);
+        } else if (p.epi == EPI_ACCUM) *out += v;
+        else *out = v;
+    }
+}
+
+// ---- 9 to 32 rows of x --------------------------------------------------------------------------------------------------------
+// A warp has 16 columns (two products) of x and a share of K. CG = 1: sixteen shares; CG = 2 (17 rows of x and more): eight, whose
+// weights two warps read, each for its own columns.
+template <int F, int CG, int T, bool QUIRK>
+__global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, NT = 2, COLS = 16 * CG, W = kWarps / CG;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp / CG, cg = warp % CG, g = lane >> 2, t = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int stages = p.stages;
+    Shared rings = smem + share * (stages * T * TB);
+    const uint32_t ring = smem_u32(rings);
+    const int units = (p.K + 255) / 256, pairs = p.epi == EPI_SWIGLU, tile0 = blockIdx.x * T;
+    const int my_units = share < units ? (units - share + W - 1) / W : 0;
+    Pieces<F> pc;
+    pc.init(p.K / 32, lane);
+    int iss = 0;
+    auto issue = [&](int buf) {                                 // (the warps of a share bring every CG-th tile)
+        if (iss < my_units) {
+#pragma unroll
+            for (int i = 0; i < T; i++) {
+                if (CG > 1 && i % CG != cg) continue;
+                const int tile = min(tile0 + i, p.tiles - 1);
+                issue_tile<F>(p, pc, pairs ? tile & 1 : 0, (pairs ? tile >> 1 : tile) * 16, share + iss * W, ring + (buf * T + i) * TB, lane);
+            }
+            iss++;
+        }
+        cp_async_commit();
+    };
+    auto meet = [&]() {                                         // the warps of a share
+        if (CG == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(share + 1), "n"(32 * CG) : "memory");
+    };
+    if (F == CMLB200_NF4) asm volatile("griddepcontrol.wait;" ::: "memory");
+    issue(0);
+    if (stages > 1) issue(1);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    float acc[T][NT][4];
+#pragma unroll
+    for (int i = 0; i < T; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
+    uint4 nh[NT], nl[NT];                                       // B operands of the next block
+    auto fetch = [&](int blk) {
+        const uint4* src = p.planes + ((size_t)blk * CG + cg) * (NT * 64) + lane;
+#pragma unroll
+        for (int j = 0; j < NT; j++) { nh[j] = __ldcg(src + j * 64); nl[j] = __ldcg(src + j * 64 + 32); }
+    };
+    if (my_units) fetch(share * 8);
+    int buf = 0;
+    for (int u = 0; u < my_units; u++) {
+        const int un = share + u * W;
+        if (stages > 1) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        meet();
+        Shared base = rings + buf * T * TB + g * ROW;
+#pragma unroll 1
+        for (int b = 0; b < 8; b++) {
+            uint4 bh[NT], bl[NT];
+#pragma unroll
+            for (int j = 0; j < NT; j++) { bh[j] = nh[j]; bl[j] = nl[j]; }
+            if (b < 7) fetch(un * 8 + b + 1);
+            else if (u + 1 < my_units) fetch((un + W) * 8);
+            float2 s32[NT];
+            if (kMins<F>) {
+#pragma unroll
+                for (int j = 0; j < NT; j++) s32[j] = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * COLS + 16 * cg + 8 * j + 2 * t));
+            }
+#pragma unroll
+            for (int i = 0; i < T; i++) {
+                Shared lo = base + i * TB, hi = lo + 8 * ROW;
+                const int tile = min(tile0 + i, p.tiles - 1), row0 = (pairs ? tile >> 1 : tile) * 16;
+                Head hl, hh;
+                head_of<F>(p, lo, row0 + g, un, hl);
+                head_of<F>(p, hi, row0 + g + 8, un, hh);
+                uint32_t a[kDigits<F>][2][4];
+                block_regs<F>(lo, hi, b, t, hl.off, hh.off, a);
+                constexpr int C1 = F == CMLB200_Q6_K ? 1 : 0;
+                float c[C1 + 1][NT][4];
+#pragma unroll
+                for (int k = 0; k <= C1; k++)
+#pragma unroll
+                    for (int j = 0; j < NT; j++)
+#pragma unroll
+                        for (int v = 0; v < 4; v++) c[k][j][v] = 0.f;
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+#pragma unroll
+                    for (int d = 0; d < kDigits<F>; d++) {
+#pragma unroll
+                        for (int j = 0; j < NT; j++) mma_f16(c[k * C1][j], a[d][k], k ? bh[j].z : bh[j].x, k ? bh[j].w : bh[j].y);
+#pragma unroll
+                        for (int j = 0; j < NT; j++) mma_f16(c[k * C1][j], a[d][k], k ? bl[j].z : bl[j].x, k ? bl[j].w : bl[j].y);
+                    }
+#pragma unroll
+                for (int k = 0; k <= C1; k++) {
+                    const float sl = scale_of<F, QUIRK>(p, lo, hl, b, k), sh = scale_of<F, QUIRK>(p, hi, hh, b, k);
+                    float ml = 0.f, mh = 0.f;
+                    if (kMins<F> && k == 0) { ml = offset_of<F>(lo, hl, b, sl); mh = offset_of<F>(hi, hh, b, sh); }
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        acc[i][j][0] = fmaf(c[k][j][0], sl, acc[i][j][0]);
+                        acc[i][j][1] = fmaf(c[k][j][1], sl, acc[i][j][1]);
+                        acc[i][j][2] = fmaf(c[k][j][2], sh, acc[i][j][2]);
+                        acc[i][j][3] = fmaf(c[k][j][3], sh, acc[i][j][3]);
+                        if (kMins<F> && k == 0) {
+                            acc[i][j][0] = fmaf(s32[j].x, ml, acc[i][j][0]);
+                            acc[i][j][1] = fmaf(s32[j].y, ml, acc[i][j][1]);
+                            acc[i][j][2] = fmaf(s32[j].x, mh, acc[i][j][2]);
+                            acc[i][j][3] = fmaf(s32[j].y, mh, acc[i][j][3]);
+                        }
+                    }
+                }
+            }
+        }
+        meet();                                                 // every lane is done with this buffer
+        issue(buf);
+        if (++buf == stages) buf = 0;
+    }
+    cp_async_wait<0>();
+    __syncthreads();                                            // the rings become the place where the warps' sums meet
+    float* part = reinterpret_cast<float*>(smem);               // [T][W][COLS][16]
+#pragma unroll
+    for (int i = 0; i < T; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            float* dst = part + ((size_t)i * W + share) * (COLS * 16) + (16 * cg + 8 * j + 2 * t) * 16 + g;
+            dst[0] = acc[i][j][0];
+            dst[16] = acc[i][j][1];
+            dst[8] = acc[i][j][2];
+            dst[24] = acc[i][j][3];
+        }
+    __syncthreads();
+    const int active = min(W, units), mine = min(T, p.tiles - tile0), outs = mine >> pairs;
+    for (int idx = threadIdx.x; idx < outs * COLS * 16; idx += blockDim.x) {
+        const int r = idx & 15, m = (idx >> 4) % COLS, o = idx / (COLS * 16);
+        const int row = ((pairs ? tile0 >> 1 : tile0) + o) * 16 + r;
+        if (m >= p.M || row >= p.N) continue;
+        const float f = __ldcg(p.xf + m);
+        const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
+        float v = 0.f, v2 = 0.f;
+        for (int w = 0; w < active; w++) v += src[w * (COLS * 16)];
+        v *= f;
+        float* out = p.y + (size_t)m * p.N + row;
+        if (pairs) {
+            for (int w = 0; w < active; w++) v2 += src[(W + w) * (COLS * 16)];
+            *out = (v / (1.0f + expf(-v))) * (v2 * f);
+        } else if (p.epi == EPI_ACCUM) *out += v;
+        else *out = v;
+    }
+}
+
+// ---- host side ----------------------------------------------------------------------------------------------------------------------
+template <typename Kern>
+int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, const SplitArgs& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CMLB_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+    return CMLB200_OK;
+}
+
+constexpr size_t kSmemMost = 227 * 1024;
+
+template <int F, int NT, bool QUIRK>
+int run_narrow(SplitArgs& p, cudaStream_t st) {
+    constexpr int COLS = NT == 0 ? 4 : 8;
+    const int units = (p.K + 255) / 256, W = units < kWarps ? units : kWarps, sms = cmlb_num_sms();
+    // as many row tiles a CTA as fill the SMs once, or several times where that would be more than six (5 tiles of 11008 rows:
+    // 8.2 us at M = 1; 3: 11.4, 2: 13.3, for every CTA makes the operands of x again)
+    const int want = (p.tiles + sms - 1) / sms, rounds = (want + 5) / 6;
+    int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
+    if (p.epi == EPI_SWIGLU) per = (per + 1) & ~1;
+    p.per_cta = per;
+    const size_t smem = (size_t)W * kRing<F, NT> * kTileBytes<F> + (NT == 0 ? (size_t)W * (p.M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * COLS * 16 + W * 4) * sizeof(float);
+    auto kern = gemv_split_kernel<F, NT, QUIRK>;
+    static size_t done[kMaxDevices] = {};
+    CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
+    return launch_split(kern, (p.tiles + per - 1) / per, W, smem, st, p);
+}
+
+template <int F, int CG, int T, bool QUIRK>
+int run_wide(SplitArgs& p, cudaStream_t st) {
+    constexpr size_t stage = (size_t)(kWarps / CG) * T * kTileBytes<F>, sums = (size_t)T * kWarps * 16 * 16 * 4;
+    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage <= kSmemMost ? 2 : 1;
+    const size_t smem = p.stages * stage > sums ? p.stages * stage : sums;
+    auto kern = gemv_split_wide_kernel<F, CG, T, QUIRK>;
+    static size_t done[kMaxDevices] = {};
+    CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
+    return launch_split(kern, (p.tiles + T - 1) / T, kWarps, smem, st, p);
+}
+
+template <int F, int CG, bool QUIRK>
+int run_wide_t(SplitArgs& p, cudaStream_t st) {
+    constexpr int most = kSmemMost / (kWarps / CG * kTileBytes<F>);
+    const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
+    int best = 1;
+    double least = 1e30;
+    for (int i = 0; i < 4; i++) {
+        const int T = choice[i];
+        if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
+        const int ctas = (p.tiles + T - 1) / T;
+        const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
+        if (cost < least) { least = cost; best = T; }
+    }
+    if constexpr (most >= 5) if (best == 5) return run_wide<F, CG, 5, QUIRK>(p, st);
+    if constexpr (most >= 3) if (best == 3) return run_wide<F, CG, 3, QUIRK>(p, st);
+    if (best == 2) return run_wide<F, CG, 2, QUIRK>(p, st);
+    return run_wide<F, CG, 1, QUIRK>(p, st);
+}
+
+template <int F, bool QUIRK>
+int run_split(SplitArgs& p, int nt, cudaStream_t st) {
+    switch (nt) {
+        case 0: return run_narrow<F, 0, QUIRK>(p, st);
+        case 1: return run_narrow<F, 1, QUIRK>(p, st);
+        case 2: return run_wide_t<F, 1, QUIRK>(p, st);
+        default: return run_wide_t<F, 2, QUIRK>(p, st);
+    }
+}
+
+}  // namespace

@@ -1,0 +1,84 @@
+"""The fp16-split decode kernels (cmlb200_gemv for NF4, Q4_1, Q4_K, Q6_K, larger batches of the others) where their tiles, units
+of columns, warps and batches end, against the dequantised weight in 64 bits.
+
+Bound of an output's error: x enters as two fp16 numbers (2^-22 of every value, once more for what fp16's smallest steps
+cut off), sums of a block and of the blocks are fp32 (2^-24 for each of K / 32 + 32 additions, twice that in the tensor core,
+which truncates), all of it relative to the sum of the products' magnitudes."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import make_block_stream, make_weight, stream_ptr, to_dev
+
+pytestmark = pytest.mark.gpu
+STREAM_TYPES = {"q4_1": 3, "q4_k": 12, "q5_k": 13, "q6_k": 14}
+
+
+def _weight(pkg, synth, ob, orc, dev, rng, kind, N, K, block=64):
+    if kind in STREAM_TYPES:
+        return make_block_stream(pkg, synth, ob, orc, dev, rng, STREAM_TYPES[kind], N, K)
+    return make_weight(pkg, synth, ob, orc, dev, rng, kind, N, K, block)
+
+
+def _check(pkg, W, Wf, x, dev, y0=None):
+    M, K = x.shape
+    N = Wf.shape[0]
+    d_x = to_dev(x, dev)
+    d_y = torch.full((M, N), float("nan"), dtype=torch.float32, device=dev) if y0 is None else to_dev(y0, dev)
+    fn = pkg.lib.cmlb200_gemv if y0 is None else pkg.lib.cmlb200_gemv_accum
+    pkg.check(fn(W.q, d_x.data_ptr(), d_y.data_ptr(), M, stream_ptr()), "gemv")
+    got = d_y.cpu().numpy().astype(np.float64)
+    X, F = x.astype(np.float64), Wf.astype(np.float64)
+    want = X @ F.T + (0 if y0 is None else y0)
+    bound = (2.0 ** -21 + (K / 32 + 32) * 2.0 ** -23) * (np.abs(X) @ np.abs(F).T) + (0 if y0 is None else 2.0 ** -23 * np.abs(want))
+    assert (np.abs(got - want) <= bound + 1e-37).all(), np.max(np.abs(got - want) / (bound + 1e-37))
+
+
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0", "nf4", "q4_1", "q4_k", "q5_k", "q6_k"])
+@pytest.mark.parametrize("N,K", [(1, 256), (16, 512), (17, 4352), (161, 1024), (2400, 768)])
+def test_rows_columns_and_batches_at_their_edges(pkg, synth, ob, orc, torch_dev, kind, N, K):
+    rng = np.random.default_rng(N + K)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K)
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32):
+        _check(pkg, W, Wf, rng.standard_normal((M, K)).astype(np.float32), torch_dev)
+    _check(pkg, W, Wf, rng.standard_normal((16, K)).astype(np.float32), torch_dev, rng.standard_normal((16, N)).astype(np.float32))
+
+
+@pytest.mark.parametrize("block,K", [(32, 32), (32, 800), (64, 1088), (128, 384), (256, 768), (512, 1024)])
+@pytest.mark.parametrize("M", [1, 4, 8, 32])
+def test_nf4_blocks_and_partial_units(pkg, synth, ob, orc, torch_dev, block, K, M):
+    rng = np.random.default_rng(block + K + M)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", 83, K, block)
+    _check(pkg, W, Wf, rng.standard_normal((M, K)).astype(np.float32), torch_dev)
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-6, 1e6, 1e30])
+@pytest.mark.parametrize("M", [3, 7, 20])
+def test_any_range_of_x(pkg, synth, ob, orc, torch_dev, scale, M):
+    rng = np.random.default_rng(M)
+    for kind in ("nf4", "q4_k", "q8_0"):
+        W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, kind, 40, 1024)
+        x = (rng.standard_normal((M, 1024)) * scale).astype(np.float32)
+        x[1] = 0.0                                             # a row without a largest value
+        x[2, ::7] *= 1e-4                                      # values of very different sizes in one row
+        _check(pkg, W, Wf, x, torch_dev)
+
+
+def test_streams_keep_their_rows_apart(pkg, synth, ob, orc, torch_dev):
+    rng = np.random.default_rng(5)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", 4096, 4096)
+    xs = [to_dev(rng.standard_normal((16, 4096)).astype(np.float32), torch_dev) for _ in range(4)]
+    alone = []
+    for x in xs:
+        y = torch.empty(16, 4096, device=torch_dev)
+        pkg.check(pkg.lib.cmlb200_gemv(W.q, x.data_ptr(), y.data_ptr(), 16, stream_ptr()), "gemv")
+        alone.append(y)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    out = [torch.empty(16, 4096, device=torch_dev) for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, x, y in zip(streams, xs, out):
+            pkg.check(pkg.lib.cmlb200_gemv(W.q, x.data_ptr(), y.data_ptr(), 16, s.cuda_stream), "gemv")
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(alone, out))
