@@ -5,78 +5,64 @@
 // triple loop" (src/nn/qlora.c:264-317) and its dequantize-at-load + fp32 matmul
 // (src/core/gguf.c:271-295, src/ops/ir/execution.c:989-1052).
 //
-// One CTA owns a tile of 128 weight rows (the MMA "M" side, operand A) by MT <= 256 (or 512: two MMAs
-// per K step into two accumulators, so that a weight slab is expanded once for 512 activation rows;
-// chosen where a cost model says it saves CTA waves)
-// activation rows (the MMA "N" side, operand B) and walks K in slabs of 64:
-//   warp 0      one lane issues TMA tensor loads of the bf16 activation slab (128B swizzle)
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma (128 x MT x 16, kind::f16)
-//   warps 2..17 expand the packed weights to bf16 and store them in the canonical K-major
-//               128B-swizzled layout the MMA reads. Expanding a slab is a chain of dependent
-//               steps (wait, load, convert, store, fence, signal) of about a microsecond whatever
-//               the number of threads sharing it, so the sixteen warps form four groups and
-//               group g takes slabs g, g+4, g+8, ...: four slabs are in flight at once.
-//               Afterwards the same warps are the epilogue: tcgen05.ld the fp32 accumulators,
-//               round to bf16 and write Y
-//   warp 18     one lane issues TMA tensor loads of the PACKED weights (a [128 rows x 32 or 64
-//               byte] box per slab, into a ring) and of their scales (a [128 rows x 8 slabs]
-//               box per 8 slabs), so that no warp gathers 128 different cache lines per slab
-// Expansion cost decides this kernel (a slab of 8192 weights per 128 x 256 x 64 MMA group):
-//   Q4_0  no table: a byte permute drops two nibbles into the mantissas of two bf16 halves
-//         (0x43nn = 128 + n), one packed subtract gives n - 8 exactly, one packed multiply
-//         applies the block scale: 15 instructions per 8 weights, nothing read from shared memory
-//   NF4   one 4-byte table entry per packed BYTE (both code values as bf16), the table kept in
-//         8 copies so that lanes rarely meet in a bank, one packed multiply by the block scale
+// A CTA works on a tile of 128 weight rows (the MMA "M" side, operand A) by NX <= 512 activation rows (the MMA "N" side, operand B;
+// two MMAs and two halves of tensor memory above 256), K in slabs of 64. Where the tiles are fewer than the SMs, a cluster of 2, 4 or 8
+// CTAs shares the K of a tile: their sums meet in distributed shared memory, every CTA adds and finishes its part of the columns in
+// rank order (no scratch in global memory, no second launch, the same result every time).
+//   warp 0      one lane issues TMA tensor loads of the bf16 activation slab (128B swizzle, boxes of up to 256 rows)
+//   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma (128 x 256 x 16, kind::f16)
+//   warps 2..17 expand the packed weights to bf16 in the canonical K-major 128B-swizzled layout the MMA reads, two groups of eight
+//               the slabs in turn; they are the epilogue too: tcgen05.ld, then Y or the cluster's sum
+// What bounds it: the expansion up to 256 activation rows (a slab of 128 x 64 weights takes 0.37 us for Q4_0, 0.54 for NF4, 0.63 for
+// Q8_0, about as long as its instructions at half an instruction a cycle and scheduler), from 512 on expansion and MMA (0.54 us
+// for 128 x 512 x 64) about equally. Hence the tile: as many activation rows as fill the SMs in whole waves (pick_shape).
+// Packed weights and scales come by plain loads into registers, three slabs of the group ahead. Each thread keeps one
+// block index and no other address, and the issuing warp counts its stages: with 64-bit addresses, zeroed registers and a vote
+// in every wait a slab took 0.60 instead of 0.40 us, with a division per slab in the issuing warp 0.54.
+// us a call, before and after (before: 128 x 512 tiles, four groups fed by TMA, K splits through global memory), weights from memory:
+//   Q4_0 4096x4096    M = 77 22.4 14.6, 512 37.0 25.0, 2048 65.2 55.5      11008x4096  77 43.0 29.0, 512 64.0 55.6, 2048 201 156
+//   Q4_0 4096x11008   M = 77 35.0 24.2, 512 64.0 46.3, 2048 171 141        32000x4096  77 82.0 52.5, 512 130 110, 2048 477 397
+//   NF4 4096x4096     M = 77 22.8 17.4, 512 41.1 30.1, 2048 67.7 59.6      Q8_0 4096x4096  77 22.6 18.8, 512 39.6 33.4, 2048 94.3 68.0
+// Expansion:
+//   Q4_0  a byte permute drops two nibbles into the mantissas of two bf16 halves (0x43nn = 128 + n), one packed subtract gives
+//         n - 8 exactly, one packed multiply applies the block scale
+//   NF4   the two bytes of a code value by byte permutes over a table of 16 in registers, one packed multiply by the block scale
 //   Q8_0  convert, multiply in fp32, round once
 // Q4_0 and NF4 therefore round twice (scale or code value to bf16, then the product); the path's
 // tolerance is 1e-2 of the largest output. No cluster multicast is used. Every wait on an
 // mbarrier is bounded; on expiry the CTA raises a status flag (cmlb200_gemm_status), waits for
 // its copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
+#include <type_traits>
 #include "common.cuh"
 
 namespace {
 
-constexpr int BN = 128;             // weight rows per CTA (MMA M)
 constexpr int BK = 64;              // K slab: 64 bf16 = one 128-byte swizzle row
 constexpr int DQ_WARPS = 16;
-constexpr int DQ_GROUPS = 4;                    // slabs being expanded at once
-constexpr int GROUP_WARPS = DQ_WARPS / DQ_GROUPS;
 constexpr int DQ_THREADS = DQ_WARPS * 32;
-constexpr int THREADS = 64 + DQ_THREADS + 32;
-constexpr int A_BYTES = BN * BK * 2;            // 16 KB
-constexpr int B_HALF = 256 * BK * 2;            // 32 KB: 256 activation rows, what one MMA instruction takes
-constexpr int SC_SLABS = 8;                     // slabs per scale box (4 bytes per row and slab)
-constexpr int SC_BYTES = BN * SC_SLABS * 4;     // 4 KB
+constexpr int THREADS = 64 + DQ_THREADS;
+constexpr int A_BYTES = 128 * BK * 2;           // 16 KB: 128 expanded weight rows
+constexpr int BN = 128;             // weight rows of a tile
+constexpr int B_ROWS = 256;         // activation rows of a box and an MMA
+constexpr int B_BYTES = B_ROWS * BK * 2;        // 32 KB
+constexpr int AHEAD = 3;                        // slabs whose packed weights a thread has requested
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
-// WIDE: tiles of up to 512 activation rows (two MMA instructions per K step on the same expanded
-// weight slab, accumulators side by side in all 512 columns of tensor memory): the expansion, which
-// decides this kernel, is paid once per 512 instead of once per 256 activation rows. The activation
-// ring then holds two 64 KB stages; the narrow form keeps as many activation as weight stages.
+// A group always comes back to the same stages, so a parity wait is never two phases from its barrier.
+// WIDE (NX > 256): activations come in boxes of 256 rows of a ring of their own, two a slab; otherwise a stage holds both operands.
 template <int TYPE, bool WIDE> struct Cfg {
     static constexpr int RAWB = (TYPE == CMLB200_Q8_0) ? 64 : 32;       // packed bytes per row and slab
-    // The expanded-weight (A) stages and the packed-weight ring have exactly one slot per expansion
-    // group: group g then only ever reuses slot g, whose previous user was its own previous slab, so a
-    // parity wait can never be two phases away from the barrier (with fewer slots than groups a fast
-    // group could see "phase complete" for a phase that has not begun: a first Q8_0 configuration
-    // with three stages had that flaw).
-    static constexpr int STAGES = DQ_GROUPS;
-    static constexpr int RSTAGES = DQ_GROUPS;
-    // activation (B) stages: producer and consumer are one thread each and move in lockstep
-    static constexpr int BSTAGES = WIDE ? 2 : (TYPE == CMLB200_Q8_0 ? 3 : 4);
-    static constexpr int B_STAGE = WIDE ? 2 * B_HALF : B_HALF;
-    static constexpr int RAW_STAGE = BN * RAWB;
-    static constexpr int LUT_BYTES = (TYPE == CMLB200_NF4) ? 8 * 256 * 4 : 0;
+    static constexpr int GROUPS = 2, GROUP_WARPS = DQ_WARPS / GROUPS;
+    static constexpr int STAGES = 4;                                    // expanded weights
+    static constexpr int BSTAGES = WIDE ? 5 : STAGES;                   // boxes of activations
     // offsets from the 1024-byte aligned base
     static constexpr int a_off = 0;
     static constexpr int b_off = STAGES * A_BYTES;
-    static constexpr int raw_off = b_off + BSTAGES * B_STAGE;
-    static constexpr int sc_off = raw_off + RSTAGES * RAW_STAGE;
-    static constexpr int lut_off = sc_off + 2 * SC_BYTES;
-    static constexpr int bar_off = lut_off + LUT_BYTES;
-    static constexpr int nbars = 2 * STAGES + 2 * BSTAGES + 1 + 2 * RSTAGES + 2;
+    static constexpr int bar_off = b_off + BSTAGES * B_BYTES;
+    static constexpr int nbars = 2 * STAGES + 2 * BSTAGES + 2;
     static constexpr int total = bar_off + 8 * nbars + 32;
+    static_assert(total + 1024 <= 227 * 1024, "the stages do not fit shared memory");
 };
 
 __device__ int g_gemm_status = 0;   // 0 = ok; otherwise a code identifying the wait that expired
@@ -116,22 +102,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // Every lane waits on the barrier itself (each reader of bytes that a tensor load wrote has to
 // observe the barrier's phase on its own); the verdict is then made warp-uniform so that no lane
 // is left behind at a __syncwarp.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code, bool ok) {
-    bool mine = ok;
-    if (ok) {
-        mine = false;
-        for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
-            if (mbar_try(bar, parity)) { mine = true; break; }
-            if (it > 1024) {
-                if (*abort_flag) break;
-                __nanosleep(32);
-            }
+__device__ __noinline__ bool warp_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    bool mine = false;
+    for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
+        if (mbar_try(bar, parity)) { mine = true; break; }
+        if (it > 1024) {
+            if (*abort_flag) break;
+            __nanosleep(32);
         }
-        if (!mine && !*abort_flag) { *abort_flag = code; atomicCAS(&g_gemm_status, 0, code); }
     }
+    if (!mine && !*abort_flag) { *abort_flag = code; atomicCAS(&g_gemm_status, 0, code); }
     return __all_sync(0xffffffffu, mine);
 }
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    return warp_wait_slow(bar, parity, abort_flag, code);
+}
 
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -158,17 +150,16 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&f)[16]) {
+    uint32_t r[16];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; j++) f[j] = __uint_as_float(r[j]);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -187,32 +178,40 @@ __device__ __forceinline__ uint32_t bf162_sub(uint32_t a, uint32_t b) {
 // Expand the 32 weights this thread owns (row n, K offset k0 + 32*h) into four 16-byte
 // chunks of bf16, in element order. `raw`: the thread's packed bytes (16, or 32 for Q8_0).
 template <int TYPE>
-__device__ __forceinline__ void expand32(const uint4 (&raw)[2], float scale, const uint32_t* lut, int lane, uint4 (&out)[4]) {
+__device__ __forceinline__ void expand32(const uint4* raw, float scale, uint4 (&out)[4]) {
     if (TYPE == CMLB200_Q8_0) {
         const uint32_t w[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             uint32_t o[4];
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                const uint32_t word = w[2 * c + (p >> 1)];
-                const int sh = (p & 1) * 16;
-                const float a = (float)(int)(int8_t)((word >> sh) & 0xFF) * scale;
-                const float b = (float)(int)(int8_t)((word >> (sh + 8)) & 0xFF) * scale;
+            for (int p = 0; p < 4; p++) {                // 2^23 + (q + 128) as fp32 has the byte for its last mantissa bits
+                const uint32_t u = w[2 * c + (p >> 1)] ^ 0x80808080u;
+                const float a = (__uint_as_float(__byte_perm(u, 0x4b000000u, p & 1 ? 0x7442 : 0x7440)) - 8388736.0f) * scale;
+                const float b = (__uint_as_float(__byte_perm(u, 0x4b000000u, p & 1 ? 0x7443 : 0x7441)) - 8388736.0f) * scale;
                 o[p] = pack_bf16(a, b);
             }
             out[c] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     } else if (TYPE == CMLB200_NF4) {
-        // word i = bytes 4i..4i+3 = elements 8i..8i+7; lut[byte] = (bf16 of the high-nibble code, of the low-nibble code)
+        // word i = bytes 4i..4i+3 = elements 8i..8i+7, the even one in the high nibble. Low and high bytes of the 16 code values
+        // as bf16, four to a word; a permute looks up eight entries, a second one picks by the index's top bit
         const uint32_t w[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
         const uint32_t s2 = pack_bf16(scale, scale);
-        const uint32_t* tab = lut + (lane & 7);
+        constexpr uint32_t L0 = 0xca063280u, L1 = 0x00bb3d92u, L2 = 0xad7c25a3u, L3 = 0x803910e2u;
+        constexpr uint32_t H0 = 0xbebfbfbfu, H1 = 0x00bdbebeu, H2 = 0x3e3e3e3du, H3 = 0x3f3f3f3eu;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             uint32_t o[4];
 #pragma unroll
-            for (int p = 0; p < 4; p++) o[p] = bf162_mul(tab[((w[c] >> (8 * p)) & 0xFF) << 3], s2);
+            for (int p = 0; p < 2; p++) {
+                const uint32_t v = p ? w[c] >> 16 : w[c];
+                const uint32_t e = v & 0x7777u, pick = ((v >> 1) & 0x4444u) | 0x3210u;
+                const uint32_t lo = __byte_perm(__byte_perm(L0, L1, e), __byte_perm(L2, L3, e), pick);
+                const uint32_t hi = __byte_perm(__byte_perm(H0, H1, e), __byte_perm(H2, H3, e), pick);
+                o[2 * p] = bf162_mul(__byte_perm(lo, hi, 0x4051), s2);
+                o[2 * p + 1] = bf162_mul(__byte_perm(lo, hi, 0x6273), s2);
+            }
             out[c] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     } else {
@@ -244,60 +243,85 @@ __device__ __forceinline__ void expand32(const uint4 (&raw)[2], float scale, con
 //   GEMM_SWIGLU_BF16 silu(gate[i]) * value stored as bf16   (the up projection finishing SwiGLU,
 //                                                            src/nn/llama.c:126-155; gate may be the output array)
 enum { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_ACC_F32 = 2, GEMM_SWIGLU_BF16 = 3 };
-__device__ __forceinline__ void epilogue_store(void* out, const __nv_bfloat16* gate, int mode, size_t i, float v) {
-    if (mode == GEMM_OUT_BF16) static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
-    else if (mode == GEMM_OUT_F32) static_cast<float*>(out)[i] = v;
-    else if (mode == GEMM_ACC_F32) static_cast<float*>(out)[i] += v;
-    else {
-        const float g = __bfloat162float(gate[i]);
-        static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn((g / (1.0f + expf(-g))) * v);
+// CNT finished values of one weight row (neighbouring activation rows; `count` of them exist), `at` the first one's place. What
+// they are multiplied with is loaded first, so that the loads are in flight together; what they are added to is not loaded at all.
+template <int CNT>
+__device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int mode, size_t at, int N, int count, const float (&v)[CNT]) {
+    if (mode == GEMM_SWIGLU_BF16) {
+        __nv_bfloat16 o[CNT];
+#pragma unroll
+        for (int j = 0; j < CNT; j++)
+            if (j < count) o[j] = gate[at + (size_t)j * N];
+#pragma unroll
+        for (int j = 0; j < CNT; j++)
+            if (j < count) {
+                const float g = __bfloat162float(o[j]);
+                static_cast<__nv_bfloat16*>(out)[at + (size_t)j * N] = __float2bfloat16_rn((g / (1.0f + expf(-g))) * v[j]);
+            }
+    } else if (mode == GEMM_OUT_BF16) {
+        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+#pragma unroll
+        for (int j = 0; j < CNT; j++, o += N)
+            if (j < count) *o = __float2bfloat16_rn(v[j]);
+    } else {
+        float* o = static_cast<float*>(out) + at;
+#pragma unroll
+        for (int j = 0; j < CNT; j++, o += N)
+            if (j < count) {
+                if (mode == GEMM_ACC_F32) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"(v[j]) : "memory");
+                else *o = v[j];
+            }
     }
 }
 
-// grid = (ceil(N/128), ceil(M/MT), splits); MT <= 256, or 512 in the WIDE form. With splits > 1 each z-slice covers a K range and
-// writes fp32 partial sums [split][M][N] to `partial`; a second kernel reduces them.
-// SCTMA: the scales come as 4 bytes per row and slab (two fp16 of Q4_0 / Q8_0, or one fp32 of NF4
-// with block 64) through the tensor map `smap`; otherwise every expansion thread loads its own.
-template <int TYPE, bool SCTMA, bool WIDE>
+__device__ __forceinline__ uint4 ld_weights(const uint4* p) {        // the row's next slabs come into L2 along with it
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+struct GemmArgs {
+    const uint8_t* qs;
+    const void* scales;
+    void* out;
+    const __nv_bfloat16* gate;
+    int mode, M, N, K, NX, tiles_m, tiles, nf4_block, nf4_shift;
+};
+
+template <int TYPE, bool WIDE>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-            const __grid_constant__ CUtensorMap smap, const void* __restrict__ scales, void* __restrict__ out,
-            const __nv_bfloat16* __restrict__ gate, int mode, float* __restrict__ partial, int M, int N, int K, int MT,
-            int nf4_block, int kb_per_split) {
+gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
     using C = Cfg<TYPE, WIDE>;
-    constexpr int STAGES = C::STAGES, BST = C::BSTAGES, RS = C::RSTAGES, RAWB = C::RAWB;
+    constexpr int STAGES = C::STAGES, BST = C::BSTAGES, RAWB = C::RAWB;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t sbase = smem_u32(smem);
-    const uint32_t bars = sbase + C::bar_off;
-    // barrier slots (8 B each)
-    constexpr int NB0 = 2 * STAGES + 2 * BST;
+    const uint32_t sbase = smem_u32(smem), bars = sbase + C::bar_off;
     auto full_a = [&](int s) { return bars + 8 * s; };
-    auto empty = [&](int s) { return bars + 8 * (STAGES + s); };
+    auto empty_a = [&](int s) { return bars + 8 * (STAGES + s); };
     auto full_b = [&](int s) { return bars + 8 * (2 * STAGES + s); };
-    // (slots 2 * STAGES + BST .. 2 * STAGES + 2 * BST - 1 of the barrier area are spare)
-    const uint32_t accum_bar = bars + 8 * NB0;
-    auto raw_full = [&](int s) { return bars + 8 * (NB0 + 1 + s); };
-    auto raw_empty = [&](int s) { return bars + 8 * (NB0 + 1 + RS + s); };
-    auto sc_full = [&](int s) { return bars + 8 * (NB0 + 1 + 2 * RS + s); };
+    auto empty_b = [&](int s) { return bars + 8 * (2 * STAGES + BST + s); };
+    const uint32_t done_bar = bars + 8 * (C::nbars - 2), free_bar = bars + 8 * (C::nbars - 1);      // accumulators finished / read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::bar_off + 8 * C::nbars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::bar_off + 8 * C::nbars + 8);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.x * BN, m0 = blockIdx.y * MT;
-    const int total_kb = (K + BK - 1) / BK;          // K % 64 == 32: the last slab's upper half is zero
-    const int kb_begin = blockIdx.z * kb_per_split;
-    const int kb_end = min(total_kb, kb_begin + kb_per_split);
-    const int nkb = kb_end - kb_begin;
+    const int KB = (p.K + BK - 1) / BK;                 // K % 64 == 32: the last slab's upper half is zero
+    const int n_lo = min(p.NX, B_ROWS), n_hi = p.NX - n_lo;              // activation rows of the first and the second MMA
+    // a cluster shares the K of a tile; CTAs without one walk over several tiles
+    uint32_t rank, ranks;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    const int first_tile = blockIdx.x / ranks, step = gridDim.x / ranks;
+    const int kb0 = KB * rank / ranks, kb1 = KB * (rank + 1) / ranks, nkb = kb1 - kb0;
+    const int my_tiles = first_tile < p.tiles ? (p.tiles - first_tile + step - 1) / step : 0, slabs = my_tiles * nkb;
     uint32_t tmem_cols = 32;
-    while ((int)tmem_cols < MT) tmem_cols <<= 1;
+    while ((int)tmem_cols < p.NX) tmem_cols <<= 1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), GROUP_WARPS); mbar_init(empty(s), 1); }
-        for (int s = 0; s < BST; s++) mbar_init(full_b(s), 1);
-        mbar_init(accum_bar, 1);
-        for (int s = 0; s < RS; s++) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), GROUP_WARPS); }
-        for (int s = 0; s < 2; s++) mbar_init(sc_full(s), 1);
+        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), C::GROUP_WARPS + (WIDE ? 0 : 1)); mbar_init(empty_a(s), 1); }
+        for (int s = 0; s < BST; s++) { mbar_init(full_b(s), 1); mbar_init(empty_b(s), 1); }
+        mbar_init(done_bar, 1);
+        mbar_init(free_bar, DQ_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -306,14 +330,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                      ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (TYPE == CMLB200_NF4 && threadIdx.x >= 64 && threadIdx.x < 64 + 256) {
-        // byte -> (high-nibble code, low-nibble code) as two bf16, eight copies interleaved
-        uint32_t* lut = reinterpret_cast<uint32_t*>(smem + C::lut_off);
-        const int b = threadIdx.x - 64;
-        const uint32_t e = pack_bf16(kNF4[b >> 4], kNF4[b & 15]);
-#pragma unroll
-        for (int c = 0; c < 8; c++) lut[b * 8 + c] = e;
-    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -322,184 +339,195 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
     if (warp == 0) {
         // ---------------- TMA producer: activation slabs (operand B) ----------------
         if (lane == 0) {
-            int issued = 0;
-            for (int i = 0; i < nkb; i++) {
-                const int s = i % BST;
-                // stage s was last read by the MMAs of slab i - BST, whose completion the issuer signals
-                // on that slab's weight-stage barrier (one commit per slab serves both rings)
-                if (i >= BST && !mbar_wait(empty((i - BST) % STAGES), ((i - BST) / STAGES) & 1, abort_flag, 1)) break;
-                mbar_expect_tx(full_b(s), (uint32_t)MT * BK * 2);
-                tma_load_2d(sbase + C::b_off + s * C::B_STAGE, &xmap, (kb_begin + i) * BK, m0, full_b(s));
-                if (WIDE && MT > 256)                              // rows 256.. of the tile: the second MMA's operand
-                    tma_load_2d(sbase + C::b_off + s * C::B_STAGE + B_HALF, &xmap, (kb_begin + i) * BK, m0 + 256, full_b(s));
-                issued = i + 1;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            // not WIDE: the box of a slab goes with its expanded weights, in the stage's barriers; counters instead of divisions
+            const int boxes = WIDE ? 2 : 1, total = slabs * boxes;
+            int bi = 0, s = 0, kb = kb0, tile = first_tile, upper = 0;
+            uint32_t phase = 1;
+            for (; bi < total; bi++) {
+                const uint32_t bar = WIDE ? full_b(s) : full_a(s);
+                if (!mbar_wait(WIDE ? empty_b(s) : empty_a(s), phase, abort_flag, 1)) break;
+                mbar_expect_tx(bar, (uint32_t)n_lo * BK * 2);
+                tma_load_2d(sbase + C::b_off + s * B_BYTES, &xmap, kb * BK, (tile % p.tiles_m) * p.NX + upper * B_ROWS, bar);
+                if (++s == BST) { s = 0; phase ^= 1; }
+                if (WIDE) upper ^= 1;
+                if (upper == 0 && ++kb == kb1) { kb = kb0; tile += step; }
             }
-            // never leave a bulk copy in flight behind an exiting CTA
-            for (int i = max(0, issued - BST); i < issued; i++)
-                mbar_wait(full_b(i % BST), (i / BST) & 1, abort_flag, 2);
+            for (int i = max(0, bi - BST); i < bi; i++) mbar_wait(WIDE ? full_b(i % BST) : full_a(i % BST), (i / BST) & 1, abort_flag, 2);   // no copy outlives its CTA
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const int n_lo = MT < 256 ? MT : 256, n_hi = MT - n_lo;       // activation rows of the first / second MMA
-            const uint32_t ibase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 4) << 24);
-            const uint32_t idesc = ibase | ((uint32_t)(n_lo >> 3) << 17), idesc_hi = ibase | ((uint32_t)(n_hi >> 3) << 17);
-            bool ok = true;
+        // ---------------- MMA issuer: the warp stays converged, an elected lane issues ----
+        const uint32_t ibase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 4) << 24);
+        const uint32_t idesc = ibase | ((uint32_t)(n_lo >> 3) << 17), idesc_hi = ibase | ((uint32_t)(n_hi >> 3) << 17);
+        bool ok = true;
+        int s = 0, sb = 0;
+        uint32_t phase = 0, phase_b = 0;
+        for (int seg = 0; seg < my_tiles && ok; seg++) {
+            if (seg) ok = warp_wait(free_bar, (seg - 1) & 1, abort_flag, 7);
             for (int i = 0; i < nkb && ok; i++) {
-                const int s = i % STAGES, sb = i % BST;
-                ok = mbar_wait(full_a(s), (i / STAGES) & 1, abort_flag, 3) && mbar_wait(full_b(sb), (i / BST) & 1, abort_flag, 4);
+                ok = warp_wait(full_a(s), phase, abort_flag, 3);
                 if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t adesc = make_desc_sw128(sbase + C::a_off + s * A_BYTES);
-                const uint64_t bdesc = make_desc_sw128(sbase + C::b_off + sb * C::B_STAGE);
-                const uint64_t bdesc_hi = make_desc_sw128(sbase + C::b_off + sb * C::B_STAGE + B_HALF);
+                auto half = [&](int b, uint32_t acc, uint32_t id) {
+                    const uint64_t bdesc = make_desc_sw128(sbase + C::b_off + b * B_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < BK / 16; kk++) {  // advance 32 bytes inside the swizzle row per K=16 step
-                    umma_f16(tmem_base, adesc + (uint64_t)(2 * kk), bdesc + (uint64_t)(2 * kk), idesc, (i | kk) ? 1u : 0u);
-                    if (WIDE && n_hi > 0)
-                        umma_f16(tmem_base + 256u, adesc + (uint64_t)(2 * kk), bdesc_hi + (uint64_t)(2 * kk), idesc_hi, (i | kk) ? 1u : 0u);
+                    for (int kk = 0; kk < BK / 16; kk++)               // 32 bytes inside the swizzle row per K=16 step
+                        umma_f16(acc, adesc + (uint64_t)(2 * kk), bdesc + (uint64_t)(2 * kk), id, (i | kk) ? 1u : 0u);
+                };
+                if (WIDE) {
+#pragma unroll
+                    for (int upper = 0; upper < 2; upper++) {
+                        ok = ok && warp_wait(full_b(sb), phase_b, abort_flag, 4);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (ok && elect_one()) {
+                            half(sb, tmem_base + (uint32_t)(upper * B_ROWS), upper ? idesc_hi : idesc);
+                            umma_commit(empty_b(sb));
+                            if (upper) umma_commit(empty_a(s));
+                        }
+                        __syncwarp();
+                        if (++sb == BST) { sb = 0; phase_b ^= 1; }
+                    }
+                } else {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elect_one()) {
+                        half(s, tmem_base, idesc);
+                        umma_commit(empty_a(s));
+                    }
+                    __syncwarp();
                 }
-                umma_commit(empty(s));
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
-            umma_commit(accum_bar);   // arrives once every MMA issued so far has retired
-        }
-    } else if (warp == 2 + DQ_WARPS) {
-        // ---------------- TMA producer: packed weights and their scales ----------------
-        if (lane == 0) {
-            int issued = 0, sc_issued = 0;
-            const int c_first = kb_begin / SC_SLABS;
-            for (int i = 0; i < nkb; i++) {
-                // Slot of slab i - RS free: its group has read that slab's bytes AND its scales. Waits
-                // happen in slab order, so by now every slab up to i - RS is done with the scale box
-                // that the box loaded below replaces (it ended at least RS + 1 slabs ago).
-                const int rs = i % RS;
-                if (!mbar_wait(raw_empty(rs), ((i / RS) & 1) ^ 1, abort_flag, 8)) break;
-                if (SCTMA && (i == 0 || (kb_begin + i) % SC_SLABS == 0)) {
-                    const int cs = sc_issued & 1;
-                    mbar_expect_tx(sc_full(cs), SC_BYTES);
-                    tma_load_2d(sbase + C::sc_off + cs * SC_BYTES, &smap, (c_first + sc_issued) * (SC_SLABS * 4), n0, sc_full(cs));
-                    sc_issued++;
-                }
-                mbar_expect_tx(raw_full(rs), C::RAW_STAGE);
-                tma_load_2d(sbase + C::raw_off + rs * C::RAW_STAGE, &wmap, (kb_begin + i) * RAWB, n0, raw_full(rs));
-                issued = i + 1;
-            }
-            for (int i = max(0, issued - RS); i < issued; i++) mbar_wait(raw_full(i % RS), (i / RS) & 1, abort_flag, 9);
-            for (int c = max(0, sc_issued - 2); c < sc_issued; c++) mbar_wait(sc_full(c & 1), (c >> 1) & 1, abort_flag, 10);
+            if (elect_one()) umma_commit(done_bar);      // arrives once every MMA issued so far has retired
+            __syncwarp();
         }
     } else {
         // ---------------- weight expansion (operand A), then epilogue ----------------
-        // group = which slabs (i % 4), tg = thread within the group; a thread expands two (row, half)
-        // items of its group's slab: rows tg/2 and 64 + tg/2, half tg & 1
-        const int dqw = warp - 2, grp = dqw % DQ_GROUPS, tg = (dqw / DQ_GROUPS) * 32 + lane;
-        const int h = tg & 1;
-        const int row_blocks = K / 32;
-        const uint32_t* lut = reinterpret_cast<const uint32_t*>(smem + C::lut_off);
-        const int c_first = kb_begin / SC_SLABS;
-        int chunk_seen = -1;
-
+        const int dqw = warp - 2, grp = dqw / C::GROUP_WARPS, tg = (dqw % C::GROUP_WARPS) * 32 + lane;
+        const int h = tg & 1, row = tg >> 1;                         // this thread's 32 weights of a slab: row, half
+        const int row_blocks = p.K / 32;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint8_t* a_row[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) a_row[c] = smem + C::a_off + (row >> 3) * 1024 + (row & 7) * 128 + (((4 * h + c) ^ (row & 7)) << 4);
+        // packed weights come straight into registers, AHEAD slabs before they are expanded (by TMA, in rows of 32 and 16 bytes, they
+        // came at a slab in two microseconds)
+        // place in the weight of the next slab to request: its slab within the tile, its block index (32 weights); the last slab's
+        // upper half may lie past the row's end (K % 64 == 32): a scale of zero stands for it
+        int ftile = first_tile, fkb = kb0 + grp;
+        const int flim = min(kb1, h ? row_blocks / 2 : (row_blocks + 1) / 2);
+        uint32_t fblk = 0;
+        auto place = [&]() {
+            while (fkb >= kb1) { fkb -= nkb; ftile += step; }
+            fblk = (uint32_t)min(ftile / p.tiles_m * BN + row, p.N - 1) * (uint32_t)row_blocks + 2u * (uint32_t)fkb + (uint32_t)h;
+        };
+        place();
+        uint4 raw[AHEAD][RAWB / 32];
+        typedef typename std::conditional<TYPE == CMLB200_NF4, float, uint16_t>::type Scale;
+        Scale scale[AHEAD];
+#pragma unroll
+        for (int d = 0; d < AHEAD; d++)
+#pragma unroll
+            for (int i = 0; i < RAWB / 32; i++) raw[d][i] = make_uint4(0u, 0u, 0u, 0u);
+        auto fetch = [&](uint4 (&r)[RAWB / 32], Scale& sc) {
+            if (fkb < flim && ftile < p.tiles) {
+                const uint4* src = reinterpret_cast<const uint4*>(p.qs) + (size_t)fblk * (RAWB / 32);
+#pragma unroll
+                for (int i = 0; i < RAWB / 32; i++) r[i] = ld_weights(src + i);
+                if (TYPE == CMLB200_NF4) {
+                    const uint32_t at = p.nf4_shift >= 0 ? fblk >> p.nf4_shift : (uint32_t)((size_t)fblk * 32 / (size_t)p.nf4_block);
+                    sc = __ldg(reinterpret_cast<const float*>(p.scales) + at);
+                } else sc = __ldg(reinterpret_cast<const uint16_t*>(p.scales) + fblk);
+            } else sc = 0;
+            fblk += 2 * C::GROUPS;
+            fkb += C::GROUPS;
+            if (fkb >= kb1) place();
+        };
         bool ok = true;
-        for (int i = grp; i < nkb; i += DQ_GROUPS) {
-            const int kb = kb_begin + i;
-            const size_t kblk = (size_t)kb * 2 + h;               // 32-element block index in the row
-            const bool in_row = kblk < (size_t)row_blocks;
-            // scales that do not come by tensor load are fetched before the waits, which hide part of the latency
-            float scale[2] = {0.f, 0.f};
-            if (!SCTMA && in_row) {
+        // one slab: out of the registers of its slot (known when compiling: nothing moves between registers, which would wait for loads)
+        auto slab = [&](uint4 (&r)[RAWB / 32], Scale& sc, int it) {
+            uint4 out[4];
+            float f;
+            if constexpr (TYPE == CMLB200_NF4) f = sc;
+            else f = cml_half_to_float(sc);
+            expand32<TYPE>(r, f, out);                                // (past the end of a row: zeros meet zero-filled activations)
+            fetch(r, sc);
+            const int s = it % STAGES;
+            ok = warp_wait(empty_a(s), ((it / STAGES) & 1) ^ 1, abort_flag, 5);
+            if (!ok) return;
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int n = min(n0 + 64 * e + (tg >> 1), N - 1);
-                    if (TYPE == CMLB200_NF4) scale[e] = reinterpret_cast<const float*>(scales)[((size_t)n * K + kblk * 32) / (size_t)nf4_block];
-                    else scale[e] = cml_half_to_float(reinterpret_cast<const uint16_t*>(scales)[(size_t)n * row_blocks + kblk]);
-                }
-            }
-            const int rs = i % RS;
-            ok = warp_wait(raw_full(rs), (i / RS) & 1, abort_flag, 11, ok);
-            const int cl = kb / SC_SLABS - c_first, cs = cl & 1;
-            if (SCTMA && cl != chunk_seen) { ok = warp_wait(sc_full(cs), (cl >> 1) & 1, abort_flag, 12, ok); chunk_seen = cl; }
-            if (!ok) break;
-            uint4 raw[2][2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const uint8_t* src = smem + C::raw_off + rs * C::RAW_STAGE + (64 * e + (tg >> 1)) * RAWB + h * (RAWB / 2);
-                raw[e][0] = *reinterpret_cast<const uint4*>(src);
-                if (RAWB == 64) raw[e][1] = *reinterpret_cast<const uint4*>(src + 16);
-                if (SCTMA) {
-                    const uint32_t sw = *reinterpret_cast<const uint32_t*>(smem + C::sc_off + cs * SC_BYTES + (64 * e + (tg >> 1)) * (SC_SLABS * 4) + (kb % SC_SLABS) * 4);
-                    if (TYPE == CMLB200_NF4) scale[e] = __uint_as_float(sw);
-                    else scale[e] = cml_half_to_float((uint16_t)(h ? (sw >> 16) : (sw & 0xFFFF)));
-                }
-            }
-            uint4 out[2][4];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                if (in_row) expand32<TYPE>(raw[e], scale[e], lut, lane, out[e]);
-                else {                                            // past the end of the row: zeros meet the zero-filled activations
-#pragma unroll
-                    for (int c = 0; c < 4; c++) out[e][c] = make_uint4(0u, 0u, 0u, 0u);
-                }
-            }
-            // The slot is handed back only now, after the arithmetic above has consumed every loaded
-            // register. Signalling right behind the load instructions is not enough: the arrival can
-            // overtake loads that are still queued in a busy shared-memory pipe, the producer then
-            // refills the slot, and those loads return the bytes of a later slab (seen as whole 16-row
-            // bands carrying the weights of slab i + ring depth, more often with the NF4 table traffic).
-            __syncwarp();
-            if (lane == 0) mbar_arrive(raw_empty(rs));
-            const int s = i % STAGES;
-            ok = warp_wait(empty(s), ((i / STAGES) & 1) ^ 1, abort_flag, 5, ok);
-            if (!ok) break;
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int r = 64 * e + (tg >> 1);
-                uint8_t* arow = smem + C::a_off + s * A_BYTES + (r >> 3) * 1024 + (r & 7) * 128;
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    *reinterpret_cast<uint4*>(arow + (((4 * h + c) ^ (r & 7)) << 4)) = out[e][c];
-            }
+            for (int c = 0; c < 4; c++) *reinterpret_cast<uint4*>(a_row[c] + s * A_BYTES) = out[c];
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(full_a(s));
-        }
-
-        // ---- epilogue: D[n][m] (lane = weight row, column = activation row) -> Y[m][n]
-        ok = warp_wait(accum_bar, 0, abort_flag, 6, ok);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok) {
-            const int q = warp & 3;                 // the TMEM lane quadrant this warp may read
-            const int part = (warp - 2) >> 2;       // four warps share a quadrant and split the columns
-            const int nrow = n0 + q * 32 + lane;
-            for (int c0 = part * 32; c0 < MT; c0 += 32 * GROUP_WARPS) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-                if (nrow < N) {
+        };
+        static_assert(AHEAD == 3, "the loop below names the slots");
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int m = m0 + c0 + j;
-                        if (m < M && c0 + j < MT) {
-                            if (partial) partial[((size_t)blockIdx.z * M + m) * N + nrow] = __uint_as_float(v[j]);
-                            else epilogue_store(out, gate, mode, (size_t)m * N + nrow, __uint_as_float(v[j]));
-                        }
+        for (int d = 0; d < AHEAD; d++) fetch(raw[d], scale[d]);
+        const int q = warp & 3, part = dqw >> 2;                     // epilogue: tensor memory lanes 32q.., columns 16 part + 64 i
+        float* const own = reinterpret_cast<float*>(smem);           // [NX][128]: this CTA's sums, where the stages were
+        int it = grp, slot = 0, ends = 0;                            // this group's next slab, its slot, the slab behind the tile
+        for (int seg = 0; seg < my_tiles && ok; seg++) {
+            const int tile = first_tile + seg * step, n0 = tile / p.tiles_m * BN, m0 = (tile % p.tiles_m) * p.NX;
+            ends += nkb;
+            for (; it < ends && ok; it += C::GROUPS) {
+                if (slot == 0) slab(raw[0], scale[0], it);
+                else if (slot == 1) slab(raw[1], scale[1], it);
+                else slab(raw[2], scale[2], it);
+                slot = slot == 2 ? 0 : slot + 1;
+            }
+            ok = ok && warp_wait(done_bar, seg & 1, abort_flag, 6);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // ---- D[n][m] (lane = weight row, column = activation row) -> Y[m][n], or into shared memory for the cluster
+            if (ok) {
+                for (int c0 = part * 16; c0 < p.NX; c0 += 64) {
+                    float f[16];
+                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, f);
+                    const int r = q * 32 + lane;
+                    if (ranks == 1) {
+                        if (n0 + r < p.N) finish(p.out, p.gate, p.mode, (size_t)(m0 + c0) * p.N + n0 + r, p.N, min(p.NX - c0, p.M - m0 - c0), f);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) own[(c0 + j) * 128 + r] = f[j];
                     }
                 }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(free_bar);
+        }
+    }
+    if (ranks > 1) {                                                 // one tile, its K over the cluster: CTA r adds and finishes its share of the columns
+        __syncthreads();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int n0 = first_tile / p.tiles_m * BN, m0 = (first_tile % p.tiles_m) * p.NX;
+        if (warp >= 2 && !*abort_flag) {
+            const int q = warp & 3, part = (warp - 2) >> 2, r = q * 32 + lane;
+            const int per = ((p.NX + (int)ranks - 1) / (int)ranks + 1) & ~1, c_end = min(p.NX, ((int)rank + 1) * per);
+            for (int c0 = (int)rank * per + part * 8; c0 < c_end; c0 += 32) {
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = 0.f;
+                for (uint32_t k = 0; k < ranks; k++) {
+                    uint32_t at;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(sbase + (uint32_t)(c0 * 128 + r) * 4u), "r"(k));
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (c0 + j < c_end) {
+                            float x;
+                            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at + (uint32_t)j * 512u) : "memory");
+                            v[j] += x;
+                        }
+                }
+                if (n0 + r < p.N) finish(p.out, p.gate, p.mode, (size_t)(m0 + c0) * p.N + n0 + r, p.N, min(min(8, c_end - c0), p.M - m0 - c0), v);
             }
         }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
-    }
-}
-
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, void* __restrict__ out, const __nv_bfloat16* __restrict__ gate,
-                                     int mode, size_t mn, int splits) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < mn; i += stride) {
-        float s = 0.f;
-        for (int z = 0; z < splits; z++) s += partial[(size_t)z * mn + i];
-        epilogue_store(out, gate, mode, i, s);
     }
 }
 
@@ -520,130 +548,99 @@ int get_encoder(EncodeTiledFn* out) {
     return CMLB200_OK;
 }
 
-// Scratch for split-K partial sums, grown on demand, one per device in use.
-struct Workspace { float* ptr; size_t bytes; };
-Workspace g_ws[16] = {};
+// A call's shape: tiles of 128 weight rows by NX activation rows, the K of a tile shared by `ranks` CTAs
+struct Shape { int NX, ranks; };
 
-// K splits for a grid of gx x gy tiles: few tiles are split so that every SM gets a CTA, with at
-// least 8 slabs per CTA.
-inline int auto_splits(int gx, int gy, int total_kb, int sms) {
-    int splits = 1;
-    while (gx * gy * splits * 2 <= sms && total_kb / (splits * 2) >= 8) splits *= 2;
-    return splits;
+// Estimated time (us) of a shape, fitted to 4096x4096, 11008x4096, 4096x11008, 32000x4096 and 1024x4096 at M = 40 .. 2048: waves of
+// tiles, each K / 64 / ranks slabs of `expand` us for the weights and 0.115 for every 256 activation rows, 2.5 us to fill the
+// pipeline and the epilogue; a cluster's sum takes a few us more (NX = 80: 15.0 us with four ranks, 19.1 with two, 27.1 without, 4096x4096). A cluster lies in one
+// GPC, so fewer fit than the SMs would hold: 1024x4096 at M = 40 takes 11.3 us as 8 clusters of 8 CTAs and 20.9 as 16 of them
+inline double shape_cost(const Shape& s, int M, int N, int KB, int sms, double expand) {
+    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN), at_once = s.ranks == 8 ? sms / 16 : s.ranks == 4 ? sms * 7 / 32 : sms / s.ranks;
+    if (s.ranks > 1 && (tiles > at_once || s.NX > B_ROWS)) return 1e30;
+    const double slab = expand + 0.115 * s.NX / 256;
+    const int waves = (tiles + at_once - 1) / at_once;
+    return waves * (((KB + s.ranks - 1) / s.ranks) * slab + 2.5 + 0.006 * s.NX) + (s.ranks > 1 ? 3.2 + 0.02 * s.NX + 0.13 * s.ranks : 0.0);
+}
+inline Shape pick_shape(int M, int N, int KB, int sms, double expand) {
+    Shape best = {16, 1};
+    double least = 1e300;
+    const int tm0 = (M + 511) / 512, tm1 = (M + 255) / 256;
+    for (int tm = tm0; tm <= tm1 + min(tm1 + 1, 8); tm++)
+        for (int ranks = 1; ranks <= 8; ranks *= 2) {
+            if (ranks > 1 && KB < 2 * ranks) continue;
+            const Shape s = {((M + tm - 1) / tm + 15) / 16 * 16, ranks};
+            const double c = shape_cost(s, M, N, KB, sms, expand);
+            if (c < least) { least = c; best = s; }
+        }
+    return best;
 }
 
-// Estimated time (us) of one launch with tiles of mt activation rows: per 64-wide K slab a 256-row
-// tile takes SLAB_N us (bound by the weight expansion), a 512-row tile SLAB_W (bound by the 64 KB of
-// activations it pulls from L2), plus 8 us per wave of CTAs for pipeline fill and epilogue, plus
-// the split-K partial sums going out and back in at about 5 TB/s.
-constexpr double SLAB_N = 0.6, SLAB_W = 0.95;     // fitted to 4096x4096, 11008x4096, 4096x11008 at M = 512 .. 4096
-inline double tile_cost_us(int M, int N, int K, int mt, int sms) {
-    const int gx = (N + BN - 1) / BN, gy = (M + mt - 1) / mt, total_kb = (K + BK - 1) / BK;
-    const int splits = auto_splits(gx, gy, total_kb, sms);
-    const int waves = (gx * gy * splits + sms - 1) / sms;
-    return waves * ((double)((total_kb + splits - 1) / splits) * (mt > 256 ? SLAB_W : SLAB_N) + 8.0) +
-           (splits > 1 ? (double)splits * M * N * 8.0 / 5e6 : 0.0);
-}
-
-template <int TYPE>
-int launch_gemm(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, float* ws, int splits_forced,
-                cudaStream_t st) {
+template <int TYPE, bool WIDE>
+int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, const Shape& shape, cudaStream_t st) {
+    using C = Cfg<TYPE, WIDE>;
     const int N = W->rows, K = W->cols;
-    // more than 256 activation rows: 512-row tiles (the weight slab is expanded once for both halves)
-    const bool wide = M > 256 && splits_forced <= 0 && Cfg<TYPE, true>::total + 1024 <= 227 * 1024 &&
-                      tile_cost_us(M, N, K, 512, cmlb_num_sms()) < tile_cost_us(M, N, K, 256, cmlb_num_sms());    // (Q8_0's 8 KB packed slabs leave no room for it)
-    const int MT = wide ? 512 : (M >= 256 ? 256 : ((M + 15) / 16) * 16);
+    GemmArgs a = {};
+    a.NX = shape.NX;
+    a.tiles_m = (M + a.NX - 1) / a.NX;
+    a.tiles = (N + BN - 1) / BN * a.tiles_m;
+    a.qs = (const uint8_t*)W->qs;
+    a.scales = W->scales;
+    a.out = y;
+    a.gate = (const __nv_bfloat16*)gate;
+    a.mode = mode;
+    a.M = M;
+    a.N = N;
+    a.K = K;
+    a.nf4_block = W->block;
+    a.nf4_shift = W->block == 32 ? 0 : W->block == 64 ? 1 : W->block == 128 ? 2 : W->block == 256 ? 3 : -1;
     EncodeTiledFn enc;
     int rc = get_encoder(&enc);
     if (rc) return rc;
     CUtensorMap xmap;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)(MT > 256 ? 256 : MT)};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)min(a.NX, B_ROWS)};
     const cuuint32_t estr[2] = {1, 1};
     CUresult cr = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)x, dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CMLB_REQUIRE(cr == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with %d (x must be 16-byte aligned, K*2 a multiple of 16)", (int)cr);
-    // the packed weights as bytes [N][row_bytes], a box of 128 rows by one slab's bytes
-    using C = Cfg<TYPE, false>;
-    CUtensorMap wmap, smap;
-    const cuuint64_t row_bytes = (cuuint64_t)K * C::RAWB / BK;
-    const cuuint64_t wdims[2] = {row_bytes, (cuuint64_t)N};
-    const cuuint64_t wstr[1] = {row_bytes};
-    const cuuint32_t wbox[2] = {(cuuint32_t)C::RAWB, (cuuint32_t)BN};
-    cr = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, W->qs, wdims, wstr, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    CMLB_REQUIRE(cr == CUDA_SUCCESS, "cuTensorMapEncodeTiled (weights) failed with %d", (int)cr);
-    // scales as bytes [N][4 per slab] when every row and slab has exactly four of them on a 16-byte row pitch:
-    // the two fp16 of Q4_0 / Q8_0, or the fp32 of NF4 with block 64; K % 256 == 0
-    const bool sctma = K % 256 == 0 && ((uintptr_t)W->scales & 15) == 0 && (TYPE != CMLB200_NF4 || W->block == 64);
-    smap = wmap;
-    if (sctma) {
-        const cuuint64_t sdims[2] = {(cuuint64_t)K / 16, (cuuint64_t)N};
-        const cuuint64_t sstr[1] = {(cuuint64_t)K / 16};
-        const cuuint32_t sbox[2] = {(cuuint32_t)(SC_SLABS * 4), (cuuint32_t)BN};
-        cr = enc(&smap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, W->scales, sdims, sstr, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        CMLB_REQUIRE(cr == CUDA_SUCCESS, "cuTensorMapEncodeTiled (scales) failed with %d", (int)cr);
-    }
-
-    const int gx = (N + BN - 1) / BN, gy = (M + MT - 1) / MT;
-    const int total_kb = (K + BK - 1) / BK;
-    int splits = 1;
-    if (splits_forced > 0) splits = splits_forced;
-    else {
-        splits = auto_splits(gx, gy, total_kb, cmlb_num_sms());
-    }
-    if (splits > total_kb) splits = total_kb;
-    const int kb_per_split = (total_kb + splits - 1) / splits;
-    splits = (total_kb + kb_per_split - 1) / kb_per_split;
-    float* partial = nullptr;
-    if (splits > 1) {
-        const size_t need = (size_t)splits * M * N * sizeof(float);
-        if (ws) partial = ws;
-        else {
-            int dev = 0;
-            CMLB_CUDA(cudaGetDevice(&dev));
-            CMLB_REQUIRE(dev < 16, "device index %d out of range", dev);
-            if (g_ws[dev].bytes < need) {
-                if (g_ws[dev].ptr) CMLB_CUDA(cudaFree(g_ws[dev].ptr));
-                g_ws[dev].ptr = nullptr;
-                g_ws[dev].bytes = 0;
-                CMLB_CUDA(cudaMalloc((void**)&g_ws[dev].ptr, need));
-                g_ws[dev].bytes = need;
-            }
-            partial = g_ws[dev].ptr;
-        }
-    }
-    static_assert(Cfg<TYPE, false>::total + 1024 <= 227 * 1024, "the stages do not fit shared memory");
-    static size_t attr[4][kMaxDevices] = {};
-#define GEMM_LAUNCH(SC, WD, slot)                                                                                                     \
-    do {                                                                                                                             \
-        auto kern = gemm_kernel<TYPE, SC, WD>;                                                                                       \
-        const int smem = Cfg<TYPE, WD>::total + 1024;                                                                                \
-        CMLB_CUDA(cmlb_ensure_smem(kern, (size_t)smem, attr[slot]));                                                                 \
-        kern<<<dim3(gx, gy, splits), THREADS, smem, st>>>(xmap, wmap, smap, W->scales, y, (const __nv_bfloat16*)gate, mode, partial, M, N, \
-                                                          K, MT, W->block, kb_per_split);                                           \
-    } while (0)
-    constexpr bool kWideFits = Cfg<TYPE, true>::total + 1024 <= 227 * 1024;
-    if (sctma && wide) GEMM_LAUNCH(true, kWideFits, 0);
-    else if (sctma) GEMM_LAUNCH(true, false, 1);
-    else if (wide) GEMM_LAUNCH(false, kWideFits, 2);
-    else GEMM_LAUNCH(false, false, 3);
-#undef GEMM_LAUNCH
-    CMLB_LAUNCH_CHECK();
-    if (splits > 1) {
-        const size_t mn = (size_t)M * N;
-        int grid = (int)((mn + 255) / 256);
-        if (grid > cmlb_num_sms() * 8) grid = cmlb_num_sms() * 8;
-        splitk_reduce_kernel<<<grid, 256, 0, st>>>(partial, y, (const __nv_bfloat16*)gate, mode, mn, splits);
-        CMLB_LAUNCH_CHECK();
-    }
+    auto kern = gemm_kernel<TYPE, WIDE>;
+    static size_t attr[kMaxDevices] = {};
+    const size_t smem = C::total + 1024;
+    CMLB_CUDA(cmlb_ensure_smem(kern, smem, attr));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(shape.ranks > 1 ? a.tiles * shape.ranks : min(a.tiles, cmlb_num_sms())));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = shape.ranks;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    CMLB_CUDA(cudaLaunchKernelEx(&cfg, kern, xmap, a));
     return CMLB200_OK;
 }
 
-int gemm_entry(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, float* ws, int splits, void* stream) {
+template <int TYPE>
+int launch_gemm(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, int splits, cudaStream_t st) {
+    const int KB = (W->cols + BK - 1) / BK;
+    Shape s = pick_shape(M, W->rows, KB, cmlb_num_sms(), TYPE == CMLB200_Q8_0 ? 0.63 : TYPE == CMLB200_NF4 ? 0.54 : 0.37);
+    if (splits > 0) {                                                    // the caller's choice, as far as a cluster and the slabs go
+        const int tm = (M + 255) / 256;
+        s.NX = ((M + tm - 1) / tm + 15) / 16 * 16;
+        s.ranks = 1;
+        while (2 * s.ranks <= splits && 2 * s.ranks <= KB && s.ranks < 8) s.ranks *= 2;
+    }
+    return s.NX > B_ROWS ? launch_tiles<TYPE, true>(W, x, y, gate, mode, M, s, st) : launch_tiles<TYPE, false>(W, x, y, gate, mode, M, s, st);
+}
+
+int gemm_entry(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, int ctas, void* stream) {
     CMLB_REQUIRE(W && W->qs && W->scales && x && y, "cmlb200_gemm_bf16: NULL argument");
     CMLB_REQUIRE(mode >= GEMM_OUT_BF16 && mode <= GEMM_SWIGLU_BF16 && (mode != GEMM_SWIGLU_BF16 || gate), "cmlb200_gemm_bf16_ex: bad output mode %d", mode);
     CMLB_REQUIRE(M >= 1, "cmlb200_gemm_bf16: M=%d must be positive", M);
@@ -652,12 +649,12 @@ int gemm_entry(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t
                  "cmlb200_gemm_bf16: x and the weight planes must be 16-byte aligned");
     cudaStream_t st = as_stream(stream);
     switch (W->type) {
-        case CMLB200_Q8_0: return launch_gemm<CMLB200_Q8_0>(W, x, y, gate, mode, M, ws, splits, st);
-        case CMLB200_Q4_0: return launch_gemm<CMLB200_Q4_0>(W, x, y, gate, mode, M, ws, splits, st);
+        case CMLB200_Q8_0: return launch_gemm<CMLB200_Q8_0>(W, x, y, gate, mode, M, ctas, st);
+        case CMLB200_Q4_0: return launch_gemm<CMLB200_Q4_0>(W, x, y, gate, mode, M, ctas, st);
         case CMLB200_NF4:
             CMLB_REQUIRE(W->block >= 32 && W->block % 32 == 0 && W->cols % W->block == 0,
                          "cmlb200_gemm_bf16: NF4 block size %d must be a multiple of 32 that divides cols", W->block);
-            return launch_gemm<CMLB200_NF4>(W, x, y, gate, mode, M, ws, splits, st);
+            return launch_gemm<CMLB200_NF4>(W, x, y, gate, mode, M, ctas, st);
         default: CMLB_REQUIRE(false, "cmlb200_gemm_bf16: unsupported weight type %d", W->type);
     }
     return CMLB200_EINVAL;
@@ -666,18 +663,18 @@ int gemm_entry(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t
 }  // namespace
 
 extern "C" int cmlb200_gemm_bf16(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t* d_y_bf16, int M, void* stream) {
-    return gemm_entry(W, d_x_bf16, d_y_bf16, nullptr, GEMM_OUT_BF16, M, nullptr, 0, stream);
+    return gemm_entry(W, d_x_bf16, d_y_bf16, nullptr, GEMM_OUT_BF16, M, 0, stream);
 }
 
 extern "C" int cmlb200_gemm_bf16_ex(const cmlb200_qmat* W, const uint16_t* d_x_bf16, int M, int mode, void* d_out, const uint16_t* d_gate_bf16,
                                     void* stream) {
-    return gemm_entry(W, d_x_bf16, d_out, d_gate_bf16, mode, M, nullptr, 0, stream);
+    return gemm_entry(W, d_x_bf16, d_out, d_gate_bf16, mode, M, 0, stream);
 }
 
 extern "C" int cmlb200_gemm_bf16_splitk(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t* d_y_bf16, int M,
                                         int splits, void* stream) {
     CMLB_REQUIRE(splits >= 1, "cmlb200_gemm_bf16_splitk: splits must be >= 1");
-    return gemm_entry(W, d_x_bf16, d_y_bf16, nullptr, GEMM_OUT_BF16, M, nullptr, splits, stream);
+    return gemm_entry(W, d_x_bf16, d_y_bf16, nullptr, GEMM_OUT_BF16, M, splits, stream);
 }
 
 extern "C" int cmlb200_gemm_status(int* status, int reset) {

@@ -206,8 +206,8 @@ int cmlb200_gemm_bf16(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t*
 #define CMLB200_GEMM_SWIGLU_BF16 3
 int cmlb200_gemm_bf16_ex(const cmlb200_qmat* W, const uint16_t* d_x_bf16, int M, int mode, void* d_out, const uint16_t* d_gate_bf16,
                          void* stream);
-/* Same, with the number of K splits chosen by the caller (1 = none). With more than one
- * split the partial sums pass through an fp32 scratch buffer owned by the library. */
+/* Same, with the number of K splits chosen by the caller (1 = none): a cluster of the largest power of two CTAs up to
+ * `splits`, 8 and half the 64-wide slabs of K shares a tile; the partial sums meet in distributed shared memory. */
 int cmlb200_gemm_bf16_splitk(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t* d_y_bf16, int M,
                              int splits, void* stream);
 /* Synchronises the device and reports whether a bounded wait inside the tensor-core kernel

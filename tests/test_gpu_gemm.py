@@ -99,6 +99,26 @@ def test_gemm_k_tail_of_half_a_slab(pkg, synth, ob, orc, torch_dev, kind, K, M):
         assert rel_err_inf(got2, ob.linear_nt(orc, xr.reshape(x.shape), Wf)) <= TOL
 
 
+@pytest.mark.parametrize("kind,N,K,M", [
+    ("q4_0", 130, 544, 15), ("q8_0", 127, 1088, 17), ("nf4", 129, 1088, 80), ("q4_0", 1024, 4096, 77),     # clusters, ragged tiles
+    ("q4_0", 1030, 1056, 255), ("nf4", 1030, 1088, 257), ("q8_0", 1030, 1056, 272),                        # 256 | 257: one MMA a slab or two
+    ("q4_0", 20000, 160, 511), ("q8_0", 20000, 160, 512), ("nf4", 20000, 160, 513), ("q4_0", 20000, 64, 1025)])   # several tiles a CTA
+@pytest.mark.parametrize("splits", [0, 2, 8])
+def test_gemm_tiles_and_clusters(pkg, synth, ob, orc, torch_dev, kind, N, K, M, splits):
+    """The shapes pick_shape and a caller's split come to, at the edges of tiles, slabs and clusters, twice with the same bits. Each
+    output is bf16 (2^-9) of a sum over weights that were rounded twice (2^-9 each, as rms over K terms at most that of one):
+    3 x 2^-9 of the norm of the outputs."""
+    rng = np.random.default_rng(1100 + N + M)
+    W, Wf = make_weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K, block=32)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    _, xr = synth.bf16_round(x)
+    want = xr.reshape(x.shape).astype(np.float64) @ Wf.T.astype(np.float64)
+    got = _gemm(pkg, synth, W, x, N, torch_dev, splits=splits)
+    assert np.linalg.norm(got - want) <= 3 * 2.0 ** -9 * np.linalg.norm(want)
+    assert rel_err_inf(got, want) <= TOL
+    assert np.array_equal(got, _gemm(pkg, synth, W, x, N, torch_dev, splits=splits))
+
+
 @pytest.mark.parametrize("M", [48, 300])
 def test_gemm_output_modes(pkg, synth, ob, orc, torch_dev, M):
     """The epilogues the LLaMA prefill uses: fp32 output, accumulation onto an fp32 residual, and
