@@ -251,6 +251,17 @@ def test_sink_outweighs_weak_keys(pkg, torch_dev, f32):
                 assert np.allclose(want, mean * (seen / (1 + seen))[:, None])
 
 
+@pytest.mark.parametrize("sequences", [7, 8])
+def test_tile_edges_and_heads_per_cta(pkg, torch_dev, sequences):
+    """Prompts that end at, before and behind a tile of 64, then a token of each sequence: 7 x 20 heads are at most one CTA each,
+    8 x 20 share keys within a CTA."""
+    lengths = [64, 65, 66, 128, 129, 130, 2, 193][:sequences]
+    L = Layer(pkg, torch_dev, mixer(20, 4, 64, 96, 0, coef=0.1, every=50), lengths, False)
+    got = L.run([[(s, 0, n - 1) for s, n in enumerate(lengths) if n > 2], [(6, 0, 1)], [(s, n - 1, n) for s, n in enumerate(lengths)]])
+    for s in range(sequences):
+        assert np.abs(L.want(s) - got[s]).max() < tol(False)
+
+
 def test_long_decode_splits_keys_over_a_cluster(pkg, torch_dev):
     """Few rows and thousands of keys: up to eight CTAs share a row's keys; the split must not show."""
     n = 3000
