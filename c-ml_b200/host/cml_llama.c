@@ -53,6 +53,8 @@ typedef struct DevModel {
     float arb_ms[2];                       /* start-up timing of one sum: peer memory, ncclAllReduce + add */
     size_t arb_probe_floats;
     float* lineup;                         /* 4 zero floats for tp_line_up */
+    int tc_w;                              /* some weight has a tile-major copy: batches may run the kernel that cmlb200_gemv_tiles_status is about */
+    float* h_logits;                       /* page-locked: logits of up to SKINNY_ROWS rows on their way to the caller's tensor */
     int generic_w;                         /* some projection is Q4_1 / Q4_K / Q5_K / Q6_K: fp32 row-block path for every call */
     int hd, heads_l, kvh_l, qw_l, kvw_l, inter_l;
     DevLayer* L;
@@ -153,6 +155,7 @@ static void dm_destroy(DevModel* d) {
                     d->logits, d->logits_l, d->logits_g, d->pairs, d->att_scratch, d->rope_cs, d->b_a, d->b_b, d->b_c, d->b_d, d->d_tokens, d->d_cur, d->row_seq,
                     d->row_pos, d->row_limit, d->d_hist};
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++) cmlb200_free(bufs[i]);
+    cmlb200_host_free_pinned(d->h_logits);
     free(d->h_cur);
     for (int r = 0; r < 8; r++) {
         if (d->arb_ws[r]) { if (r == d->rank) cmlb200_free(d->arb_ws[r]); else cmlb200_ipc_close(d->arb_ws[r]); }
@@ -472,6 +475,7 @@ static int dm_alloc_buffers(DevModel* d) {
     DEV(cmlb200_malloc((void**)&d->u, (size_t)SKINNY_ROWS * d->inter_l * 4));
     DEV(cmlb200_malloc((void**)&d->tmp, R * H * 4));
     DEV(cmlb200_malloc((void**)&d->logits, R * c->vocab_size * 4));
+    DEV(cmlb200_host_alloc_pinned((void**)&d->h_logits, (size_t)SKINNY_ROWS * c->vocab_size * 4));
     d->vocab_l = (d->tp > 1 && c->vocab_size % d->tp == 0) ? c->vocab_size / d->tp : c->vocab_size;
     if (d->vocab_l != c->vocab_size) {
         DEV(cmlb200_malloc((void**)&d->logits_l, R * d->vocab_l * 4));
@@ -510,7 +514,7 @@ static int upload_qmat(DevModel* d, int type, const uint8_t* blocks, int rows, i
     out->block = 32;
     if (type != GGUF_TENSOR_Q4_0 && type != GGUF_TENSOR_Q8_0) {
         /* Q4_1 / Q4_K / Q5_K / Q6_K: the block stream goes to the device as it is; the model then runs
-         * every call on the fp32 row-block path (no fused or tensor-core kernels for these types) */
+         * every call in blocks of up to 32 fp32 rows (no prefill GEMM for these types) */
         const size_t bs = gguf_quant_block_size((GGUFTensorType)type), bytes = (size_t)rows * ((size_t)cols / bs) * gguf_quant_type_size((GGUFTensorType)type);
         out->block = (int)bs;
         if (CML_DEV_FAIL(cmlb200_malloc(&out->qs, bytes), "upload") || CML_DEV_FAIL(cmlb200_memcpy_h2d(out->qs, blocks, bytes, d->stream), "upload") ||
@@ -528,14 +532,15 @@ static int upload_qmat(DevModel* d, int type, const uint8_t* blocks, int rows, i
     if (CML_DEV_FAIL(cmlb200_malloc(&out->qs, qb), "upload") || CML_DEV_FAIL(cmlb200_malloc(&out->scales, sb), "upload")) goto done;
     if (CML_DEV_FAIL(cmlb200_memcpy_h2d(out->qs, h_qs, qb, d->stream), "upload") ||
         CML_DEV_FAIL(cmlb200_memcpy_h2d(out->scales, h_sc, sb, d->stream), "upload")) goto done;
-    /* the tcgen05 decode path serves batches of 3..32 from a tile-major copy, unless the 8-row
-     * mma.sync kernel takes this weight from the planes (Q4_0, cols % 256 == 0) */
+    /* the tcgen05 decode path serves batches of 5..32 from a tile-major copy, unless the
+     * mma.sync kernels take this weight from the planes (cols % 256 == 0) */
     if (cols % 128 == 0 && d->max_batch > 2 && !cmlb200_gemv_batched_from_planes(out)) {
         const size_t tb = cmlb200_tiles_bytes(type, rows, cols);
         h_t = malloc(tb);
         if (!h_t) goto done;
         if (CML_DEV_FAIL(cmlb200_repack_tiles(type, blocks, rows, cols, h_t), "upload")) goto done;
         if (CML_DEV_FAIL(cmlb200_malloc(&out->tiles, tb), "upload")) goto done;
+        d->tc_w = 1;
         if (CML_DEV_FAIL(cmlb200_memcpy_h2d(out->tiles, h_t, tb, d->stream), "upload")) goto done;
     }
     if (CML_DEV_FAIL(cmlb200_stream_sync(d->stream), "upload")) goto done;
@@ -767,9 +772,11 @@ int cml_llama_load_gguf(CMLLLaMAModel* model, const char* filepath) {
  * stream-K fix-up, and the peer-memory all-reduce, whose launch then left the residual without the
  * projection.) Returns -1 and logs; a failed all-reduce also retires the peer path, because the
  * ranks' sequence counters may no longer agree, and NCCL serves every size from then on. */
-static int dm_check_waits(DevModel* d, const char* who) {
+static int dm_check_waits(DevModel* d, int rows, const char* who) {
     int st = 0;
-    if (cmlb200_gemm_status(&st, 1) == CMLB200_OK && st == 0) cmlb200_gemv_tiles_status(&st, 1);
+    /* each status costs two synchronous copies: only those of kernels that a call of so many rows can have run */
+    if (rows > SKINNY_ROWS) cmlb200_gemm_status(&st, 1);
+    if (st == 0 && d->tc_w) cmlb200_gemv_tiles_status(&st, 1);
     if (st) { LOG_ERROR("%s: a bounded device-side wait expired (code %d)", who, st); return -1; }
     if (d->ar_ok && d->ar_ws[d->rank]) {
         if (cmlb200_tp_ar_status(d->ar_ws[d->rank], &st) != CMLB200_OK) { LOG_ERROR("%s: %s", who, cmlb200_last_error()); return -1; }
@@ -1009,14 +1016,17 @@ static Tensor* run_forward(CMLLLaMAModel* model, const int* token_ids, int rows,
     int shape[2] = {with_logits ? rows : 1, with_logits ? c->vocab_size : 1};
     Tensor* out = cml_tensor_alloc(DTYPE_FLOAT32, shape, 2, !with_logits);
     if (!out) return NULL;
+    const size_t bytes = (size_t)rows * c->vocab_size * 4;
+    const int staged = with_logits && rows <= SKINNY_ROWS;   /* through page-locked memory: a pageable copy of one row costs as much as a layer */
     if (CML_DEV_FAIL(cmlb200_memcpy_h2d(d->d_tokens, token_ids, (size_t)rows * 4, d->stream), who) || tp_line_up(d) ||
         enqueue_forward_ex(d, rows, mode, seq, max_pos - 1, -1, with_logits) ||
-        (with_logits && CML_DEV_FAIL(cmlb200_memcpy_d2h(out->data, d->logits, (size_t)rows * c->vocab_size * 4, d->stream), who)) ||
+        (with_logits && CML_DEV_FAIL(cmlb200_memcpy_d2h(staged ? d->h_logits : out->data, d->logits, bytes, d->stream), who)) ||
         CML_DEV_FAIL(cmlb200_stream_sync(d->stream), who)) {
         tensor_free(out);
         return NULL;
     }
-    if (dm_check_waits(d, who)) { tensor_free(out); return NULL; }
+    if (staged) memcpy(out->data, d->h_logits, bytes);
+    if (dm_check_waits(d, rows, who)) { tensor_free(out); return NULL; }
     if (mode == 0) d->h_cur[seq] += rows;
     else for (int b = 0; b < rows; b++) d->h_cur[b] += 1;
     model->current_seq_len = d->h_cur[0];
@@ -1113,7 +1123,7 @@ int cml_llama_decode_greedy(CMLLLaMAModel* model, const int* first_tokens, int b
     DEV(cmlb200_stream_sync(st));
     cmlb200_event_destroy(e0);
     cmlb200_event_destroy(e1);
-    if (dm_check_waits(d, "cml_llama_decode_greedy")) return -1;
+    if (dm_check_waits(d, batch, "cml_llama_decode_greedy")) return -1;
     if (elapsed_ms) *elapsed_ms = ms;
     for (int b = 0; b < batch; b++) d->h_cur[b] += steps;
     model->current_seq_len = d->h_cur[0];
@@ -1210,7 +1220,7 @@ Tensor* cml_llama_layer_forward(CMLLLaMAModel* model, CMLLLaMALayer* layer, Tens
              !CML_DEV_FAIL(cmlb200_memcpy_d2h(out->data, d->h, bytes, d->stream), who);
     /* put the model's own position back whatever happened */
     if (CML_DEV_FAIL(cmlb200_memcpy_h2d(d->d_cur, &saved, sizeof(int), d->stream), who) || CML_DEV_FAIL(cmlb200_stream_sync(d->stream), who)) ok = 0;
-    if (dm_check_waits(d, who)) ok = 0;
+    if (dm_check_waits(d, rows, who)) ok = 0;
     if (!ok) { tensor_free(out); return NULL; }
     return out;
 }

@@ -19,6 +19,7 @@
 #define TILE_ROWS 64
 #define SMALL_ROWS 64              /* steps up to this many rows share one compact upload layout, and may be captured */
 #define HEAD_ROWS 256              /* rows of logits per pass of the vocabulary projection */
+#define STAGED_ROWS 32             /* rows of logits that go through page-locked memory */
 #define MAX_CLASSES 16
 #define MAX_GRAPHS 32
 
@@ -39,6 +40,7 @@ struct CMLLanguageModel {
     size_t meta_cap;
     int *h_table, *d_table;        /* block table, host mirror page-locked */
     float* d_logits;
+    float* h_logits;               /* page-locked: STAGED_ROWS rows on their way to the caller */
     int *d_picked, *h_picked;
     int *d_hist, *d_step;
     size_t hist_cap;
@@ -85,6 +87,7 @@ static int make_buffers(CMLLanguageModel* lm) {
     memset(lm->h_table, 0, table);
     DEV(cmlb200_memset(lm->d_table, 0, table, lm->stream));
     DEV(cmlb200_malloc((void**)&lm->d_logits, (size_t)HEAD_ROWS * (size_t)lm->info.vocab * sizeof(float)));
+    DEV(cmlb200_host_alloc_pinned((void**)&lm->h_logits, (size_t)STAGED_ROWS * (size_t)lm->info.vocab * sizeof(float)));
     DEV(cmlb200_malloc((void**)&lm->d_picked, HEAD_ROWS * sizeof(int)));
     DEV(cmlb200_host_alloc_pinned((void**)&lm->h_picked, HEAD_ROWS * sizeof(int)));
     DEV(cmlb200_malloc((void**)&lm->d_step, sizeof(int)));
@@ -141,6 +144,7 @@ void cml_lm_free(CMLLanguageModel* lm) {
     cmlb200_host_free_pinned(lm->h_meta);
     cmlb200_host_free_pinned(lm->h_table);
     cmlb200_host_free_pinned(lm->h_picked);
+    cmlb200_host_free_pinned(lm->h_logits);
     if (lm->stream) cmlb200_stream_destroy(lm->stream);
     free(lm->in_step);
     free(lm->portions);
@@ -366,6 +370,10 @@ static int run_step(CMLLanguageModel* lm, const CMLLMEntry* entries, int n, floa
             DEV(cmlb200_memcpy_d2h(lm->h_picked, lm->d_picked, (size_t)k * sizeof(int), lm->stream));
             DEV(cmlb200_stream_sync(lm->stream));
             memcpy(picked + at, lm->h_picked, (size_t)k * sizeof(int));
+        } else if (k <= STAGED_ROWS) {                        /* (a pageable copy of a few rows costs as much as their step) */
+            DEV(cmlb200_memcpy_d2h(lm->h_logits, lm->d_logits, (size_t)k * V * sizeof(float), lm->stream));
+            DEV(cmlb200_stream_sync(lm->stream));
+            memcpy(logits + (size_t)at * V, lm->h_logits, (size_t)k * V * sizeof(float));
         } else {
             DEV(cmlb200_memcpy_d2h(logits + (size_t)at * V, lm->d_logits, (size_t)k * V * sizeof(float), lm->stream));
         }
