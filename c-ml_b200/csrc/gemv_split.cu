@@ -162,3 +162,14 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
         default: return cmlb200_split_k_(W->type, &p, nt, st);
     }
 }
+
+// Projections of RMS-normalised rows in one or two launches, for the LLaMA's decode steps beyond what cmlb200_gemv_rmsnorm takes:
+// any block format the kernels take, up to 32 rows; epi 2 (SwiGLU) up to 8, where a CTA's row tiles come in pairs at no cost.
+extern "C" int cmlb200_gemv_norm_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M) {
+    if (M < 1 || M > (W2 ? 8 : 32) || W->rows <= 0 || W->cols <= 0 || !cmlb200_gemv_split_ok_(W)) return 0;
+    return !W2 || (W2->type == W->type && W2->rows == W->rows && W2->cols == W->cols && W2->block == W->block && cmlb200_gemv_split_ok_(W2));
+}
+extern "C" int cmlb200_gemv_norm_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* d_x, const uint16_t* d_norm_w, float eps, float* d_y, int M,
+                                  void* stream) {
+    return cmlb200_gemv_split_(W, W2, d_x, d_norm_w, eps, d_y, M, W2 ? EPI_SWIGLU : EPI_STORE, as_stream(stream));
+}

@@ -24,6 +24,9 @@
 
 #define DEV(call) do { if (CML_DEV_FAIL((call), __func__)) return -1; } while (0)
 #define SKINNY_ROWS 32
+/* csrc/gemv_split.cu: RMS norm and projection (W2: gate and up with their SwiGLU) of up to 32 rows, any block format */
+int cmlb200_gemv_norm_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M);
+int cmlb200_gemv_norm_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* d_x, const uint16_t* d_norm_w, float eps, float* d_y, int M, void* stream);
 #define ATT_DECODE_CHUNK 32
 #define ATT_CHUNK 64
 
@@ -903,6 +906,8 @@ static int enqueue_forward_ex(DevModel* d, int rows, int mode, int seq, int plan
         /* ---- attention block: norm -> fused QKV projection -> RoPE + cache append -> attention */
         if (tiny) {
             DEV(cmlb200_gemv_rmsnorm(&L->wqkv, NULL, d->h, (const uint16_t*)L->n1, c->rms_norm_eps, d->qkv, rows, 0, st));
+        } else if (skinny && cmlb200_gemv_norm_ok_(&L->wqkv, NULL, rows)) {
+            DEV(cmlb200_gemv_norm_(&L->wqkv, NULL, d->h, (const uint16_t*)L->n1, c->rms_norm_eps, d->qkv, rows, st));
         } else if (skinny) {
             DEV(cmlb200_rmsnorm(d->h, (const uint16_t*)L->n1, rows, H, c->rms_norm_eps, d->nrm, NULL, st));
             if (lin_f32(d, &L->wqkv, d->nrm, d->qkv, rows, 0)) return -1;
@@ -931,6 +936,16 @@ static int enqueue_forward_ex(DevModel* d, int rows, int mode, int seq, int plan
         if (tiny) {
             if (proj_residual_f32(d, &L->wo, d->att, rows)) return -1;
             DEV(cmlb200_gemv_rmsnorm(&L->wg, &L->wu, d->h, (const uint16_t*)L->n2, c->rms_norm_eps, d->ffn, rows, 2, st));
+            if (proj_residual_f32(d, &L->wd, d->ffn, rows)) return -1;
+        } else if (skinny && cmlb200_gemv_norm_ok_(&L->wg, &L->wu, rows)) {
+            if (proj_residual_f32(d, &L->wo, d->att, rows)) return -1;
+            DEV(cmlb200_gemv_norm_(&L->wg, &L->wu, d->h, (const uint16_t*)L->n2, c->rms_norm_eps, d->ffn, rows, st));
+            if (proj_residual_f32(d, &L->wd, d->ffn, rows)) return -1;
+        } else if (skinny && cmlb200_gemv_norm_ok_(&L->wg, NULL, rows) && cmlb200_gemv_norm_ok_(&L->wu, NULL, rows)) {
+            if (proj_residual_f32(d, &L->wo, d->att, rows)) return -1;
+            DEV(cmlb200_gemv_norm_(&L->wg, NULL, d->h, (const uint16_t*)L->n2, c->rms_norm_eps, d->g, rows, st));
+            DEV(cmlb200_gemv_norm_(&L->wu, NULL, d->h, (const uint16_t*)L->n2, c->rms_norm_eps, d->u, rows, st));
+            DEV(cmlb200_swiglu_f32(d->g, d->u, d->ffn, (size_t)rows * d->inter_l, st));
             if (proj_residual_f32(d, &L->wd, d->ffn, rows)) return -1;
         } else if (skinny) {
             if (proj_residual_f32(d, &L->wo, d->att, rows)) return -1;
@@ -966,6 +981,8 @@ static int enqueue_forward_ex(DevModel* d, int rows, int mode, int seq, int plan
     float* lg = split_head ? d->logits_l : d->logits;          /* [rows, vocab_l] */
     if (tiny) {
         DEV(cmlb200_gemv_rmsnorm(&d->lm_head, NULL, d->h, (const uint16_t*)d->fnorm, c->rms_norm_eps, lg, rows, 0, st));
+    } else if (skinny && cmlb200_gemv_norm_ok_(&d->lm_head, NULL, rows)) {
+        DEV(cmlb200_gemv_norm_(&d->lm_head, NULL, d->h, (const uint16_t*)d->fnorm, c->rms_norm_eps, lg, rows, st));
     } else if (skinny) {
         DEV(cmlb200_rmsnorm(d->h, (const uint16_t*)d->fnorm, rows, H, c->rms_norm_eps, d->nrm, NULL, st));
         if (lin_f32(d, &d->lm_head, d->nrm, lg, rows, 0)) return -1;
