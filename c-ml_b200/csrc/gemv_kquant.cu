@@ -9,6 +9,7 @@
 // sub-block costs 24 dp4a per row of x; the fp16 / 6-bit / int8 scales, minima and offsets of the
 // formats are applied once per sub-block in fp32. Q4_K / Q5_K follow C-ML's own nibble order (each
 // 32-element sub-block in 16 consecutive bytes, src/core/gguf_quant.c:174-187), not ggml's.
+// Left with columns that are no whole 256 and very long rows: the fp16-split kernels (gemv_split.cuh) take the others.
 #include "common.cuh"
 
 namespace {

@@ -28,9 +28,6 @@
 #include "common.cuh"
 #include "mma_util.cuh"
 
-#ifndef UNROLL_B
-#define UNROLL_B 1
-#endif
 namespace {
 
 enum { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2 };
