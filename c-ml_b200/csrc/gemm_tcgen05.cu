@@ -6,7 +6,7 @@
 // (src/core/gguf.c:271-295, src/ops/ir/execution.c:989-1052).
 //
 // A CTA works on a tile of 128 weight rows (the MMA "M" side, operand A) by NX <= 512 activation rows (the MMA "N" side, operand B;
-// two MMAs and two halves of tensor memory above 256), K in slabs of 64. Where the tiles are fewer than the SMs, a cluster of 2, 4 or 8
+// two MMAs and two halves of tensor memory above 256), K in slabs of 64. Where the tiles are fewer than the SMs, a cluster of 2 to 8
 // CTAs shares the K of a tile: their sums meet in distributed shared memory, every CTA adds and finishes its part of the columns in
 // rank order (no scratch in global memory, no second launch, the same result every time).
 //   warp 0      one lane issues TMA tensor loads of the bf16 activation slab (128B swizzle, boxes of up to 256 rows)
@@ -409,8 +409,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         uint8_t* a_row[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) a_row[c] = smem + C::a_off + (row >> 3) * 1024 + (row & 7) * 128 + (((4 * h + c) ^ (row & 7)) << 4);
-        // packed weights come straight into registers, AHEAD slabs before they are expanded (by TMA, in rows of 32 and 16 bytes, they
-        // came at a slab in two microseconds)
+        // packed weights come straight into registers, AHEAD slabs before they are expanded
         // place in the weight of the next slab to request: its slab within the tile, its block index (32 weights); the last slab's
         // upper half may lie past the row's end (K % 64 == 32): a scale of zero stands for it
         int ftile = first_tile, fkb = kb0 + grp;
@@ -554,9 +553,10 @@ struct Shape { int NX, ranks; };
 // Estimated time (us) of a shape, fitted to 4096x4096, 11008x4096, 4096x11008, 32000x4096 and 1024x4096 at M = 40 .. 2048: waves of
 // tiles, each K / 64 / ranks slabs of `expand` us for the weights and 0.115 for every 256 activation rows, 2.5 us to fill the
 // pipeline and the epilogue; a cluster's sum takes a few us more (NX = 80: 15.0 us with four ranks, 19.1 with two, 27.1 without, 4096x4096). A cluster lies in one
-// GPC, so fewer fit than the SMs would hold: 1024x4096 at M = 40 takes 11.3 us as 8 clusters of 8 CTAs and 20.9 as 16 of them
+// GPC (18 SMs, eight of them, counted as seven), so fewer fit than the SMs would hold: 1024x4096 at M = 40 takes 11.3 us as 8 clusters
+// of 8 CTAs and 20.9 as 16 of them
 inline double shape_cost(const Shape& s, int M, int N, int KB, int sms, double expand) {
-    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN), at_once = s.ranks == 8 ? sms / 16 : s.ranks == 4 ? sms * 7 / 32 : sms / s.ranks;
+    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN), at_once = s.ranks == 1 ? sms : s.ranks > 6 ? sms / 16 : 7 * (sms / 8 / s.ranks);
     if (s.ranks > 1 && (tiles > at_once || s.NX > B_ROWS)) return 1e30;
     const double slab = expand + 0.115 * s.NX / 256;
     const int waves = (tiles + at_once - 1) / at_once;
@@ -567,7 +567,7 @@ inline Shape pick_shape(int M, int N, int KB, int sms, double expand) {
     double least = 1e300;
     const int tm0 = (M + 511) / 512, tm1 = (M + 255) / 256;
     for (int tm = tm0; tm <= tm1 + min(tm1 + 1, 8); tm++)
-        for (int ranks = 1; ranks <= 8; ranks *= 2) {
+        for (int ranks = 1; ranks <= 8; ranks++) {
             if (ranks > 1 && KB < 2 * ranks) continue;
             const Shape s = {((M + tm - 1) / tm + 15) / 16 * 16, ranks};
             const double c = shape_cost(s, M, N, KB, sms, expand);
