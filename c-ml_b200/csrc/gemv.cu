@@ -258,14 +258,16 @@ int check_qmat(const cmlb200_qmat* W, const char* who) {
 //   Q8_0  4096x4096: 1 5.6 | 4.6, 2 6.3 | 5.1 (4096x11008: 13.5 | 17.9, two launches), 3 6.8 | 9.3, 8 8.8 | 14.1, 32 16.8 | 82.6
 //   NF4 4096x4096: 1 9.5 | 63.5, 4 11.2 | 70.5, 32 26.5 | 562; Q4_K: 1 5.9 | 7.4, 8 9.6 | 22.9, 32 21.0 | 83.8; Q6_K: 1 7.8 | 9.7, 8 10.6 | 27.3,
 //         32 21.6 | 109.9; Q4_1: 1 5.6 | 7.3, 32 18.4 | 79.9 (the alternative of the GGUF types, gemv_kquant.cu, is left with columns
-//         that are no whole 256)
+//         that are no whole 256 and short rows at M = 1: 16 warps share the 256-column units of a row, Q6_K 4608x1536 6.3 | 5.5).
+//         Q8_0 7424x3840: 4 9.3 | 8.7
 //   Q5_K  11008x4096: 1 15.2 | 14.9, 2 15.8 | 23.5, 32 49.8 | 189.5; 1024x4096: 1 4.6 | 5.5
 bool split_is_faster(const cmlb200_qmat* W, int M, int epi) {
     if (!cmlb200_gemv_split_ok_(W)) return false;
     switch (W->type) {
         case CMLB200_Q4_0: return M > 8 || M == 3;
-        case CMLB200_Q8_0: return M > 2 || (M == 2 && cmlb200_gemv_mma_rows_(W, epi) < 2);
-        default: return true;
+        case CMLB200_Q8_0: return M > 4 || M == 3 || (M > 1 && cmlb200_gemv_mma_rows_(W, epi) < M);
+        case CMLB200_NF4: return true;
+        default: return M > 1 || (W->type != CMLB200_Q5_K && W->cols >= 4096);
     }
 }
 
