@@ -1,7 +1,6 @@
 // Choice of the kernels of gemv_split.cuh and the rows of x as their B operands.
-#include <mutex>
 #include "gemv_split.cuh"
-#include "stream_scratch.cuh"
+#include "call_scratch.cuh"
 
 int cmlb200_split_q4_(void* args, int nt, int quirk, cudaStream_t st);
 int cmlb200_split_q8_(void* args, int nt, int quirk, cudaStream_t st);
@@ -89,11 +88,7 @@ x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float
     }
 }
 
-
-// Scratch of a stream for the split rows, the sums of their blocks and their scaling
 constexpr int kMaxUnits = 512;                               // K < 131072
-constexpr size_t kPlaneBytes = (size_t)kMaxUnits * 8 * 4 * 64 * sizeof(uint4), kSumBytes = (size_t)kMaxUnits * 8 * 32 * 4;
-std::mutex g_pair_mutex;                                     // the two launches of a call stay together on their stream
 
 }  // namespace
 
@@ -132,14 +127,14 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
     p.nf4_shift = W->type != CMLB200_NF4 ? 0 : W->block >= 256 ? 3 : W->block == 128 ? 2 : W->block == 64 ? 1 : 0;
     p.nf4_units = W->type == CMLB200_NF4 && W->block > 256 ? W->block / 256 : 1;
     const int nt = M <= 4 ? 0 : M <= 8 ? 1 : M <= 16 ? 2 : 4;
-    std::unique_lock<std::mutex> lock(g_pair_mutex, std::defer_lock);
-    if (nt) lock.lock();
+    CallScratch scratch;                                     // the split rows, the sums of their blocks, their scaling
     if (nt) {
+        const size_t blocks = (size_t)((p.K + 255) / 256) * 8, plane_bytes = blocks * nt * 64 * sizeof(uint4), sum_bytes = blocks * 8 * nt * sizeof(float);
         uint8_t* base = nullptr;
-        int rc = cmlb_stream_scratch(st, kPlaneBytes + kSumBytes + 32 * sizeof(float), (void**)&base);
+        int rc = scratch.get(st, plane_bytes + sum_bytes + 8 * nt * sizeof(float), (void**)&base);
         if (rc) return rc;
         uint4* planes = reinterpret_cast<uint4*>(base);
-        float *sums = reinterpret_cast<float*>(base + kPlaneBytes), *xf = reinterpret_cast<float*>(base + kPlaneBytes + kSumBytes);
+        float *sums = reinterpret_cast<float*>(base + plane_bytes), *xf = reinterpret_cast<float*>(base + plane_bytes + sum_bytes);
         p.planes = planes;
         p.sums = sums;
         p.xf = xf;

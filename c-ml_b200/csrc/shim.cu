@@ -2,7 +2,6 @@
 #include <stdarg.h>
 #include <string.h>
 #include "common.cuh"
-#include "stream_scratch.cuh"
 
 static thread_local char g_err[512] = "";
 
@@ -72,9 +71,7 @@ extern "C" int cmlb200_stream_create(void** stream) {
     return CMLB200_OK;
 }
 extern "C" int cmlb200_stream_destroy(void* stream) {
-    if (!stream) return CMLB200_OK;
-    cmlb_stream_scratch_release(as_stream(stream));
-    CMLB_CUDA(cudaStreamDestroy(as_stream(stream)));
+    if (stream) CMLB_CUDA(cudaStreamDestroy(as_stream(stream)));
     return CMLB200_OK;
 }
 extern "C" int cmlb200_stream_sync(void* stream) {
