@@ -8,34 +8,7 @@
 // bytes in registers, multiplies with activations staged in shared memory,
 // and rows are reduced with warp shuffles.
 #include "common.cuh"
-
-// gemv_dp4a.cu: the integer-dot kernels for Q4_0 / Q8_0 at small M
-int cmlb200_gemv_dp4a_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps,
-                       const uint32_t* xq, float* y, int M, int epi, cudaStream_t st);
-size_t cmlb200_xq_bytes_(int M, int K);
-int cmlb200_x_digits_(const float* x, int M, int K, uint32_t* xq, cudaStream_t st);
-
-// gemv_mma.cu: the tensor-core decode kernel (mma.sync int8) for up to 4 rows of x per launch
-int cmlb200_gemv_mma_rows_(const cmlb200_qmat* W, int epi);
-int cmlb200_gemv_mma_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps,
-                      const uint32_t* xq, float* y, int M, int epi, cudaStream_t st);
-
-// gemv_mma8.cu: the same for 5 to 8 rows of x per launch (Q4_0)
-bool cmlb200_gemv_mma8_ok_(const cmlb200_qmat* W, int epi);
-int cmlb200_gemv_mma8_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps, float* y, int M,
-                       int epi, cudaStream_t st);
-
-// gemv_kquant.cu: Q4_1 / Q4_K / Q5_K / Q6_K weights straight from the GGUF block stream
-bool cmlb200_is_kquant_type_(int type);
-int cmlb200_gemv_kquant_(const cmlb200_qmat* W, const float* x, float* y, int M, int accumulate, cudaStream_t st);
-
-// gemv_tc.cu: tcgen05 integer tensor-core path over the tile-major copy of the weight
-int cmlb200_gemv_tc_(const cmlb200_qmat* W, const float* x, float* y, int M, int accumulate, cudaStream_t st);
-
-// gemv_split.cu: fp16 tensor cores with x in two fp16 parts, every block format, up to 32 rows of x per launch
-bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W);
-int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps, float* y, int M, int epi,
-                        cudaStream_t st);
+#include "gemv_paths.cuh"
 
 namespace {
 
@@ -261,11 +234,11 @@ int check_qmat(const cmlb200_qmat* W, const char* who) {
 //         that are no whole 256 and short rows at M = 1: 16 warps share the 256-column units of a row, Q6_K 4608x1536 6.3 | 5.5).
 //         Q8_0 7424x3840: 4 9.3 | 8.7
 //   Q5_K  11008x4096: 1 15.2 | 14.9, 2 15.8 | 23.5, 32 49.8 | 189.5; 1024x4096: 1 4.6 | 5.5
-bool split_is_faster(const cmlb200_qmat* W, int M, int epi) {
-    if (!cmlb200_gemv_split_ok_(W)) return false;
+bool split_is_faster(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M, int epi) {
+    if (!cmlb200_gemv_split_ok_(W, W2)) return false;
     switch (W->type) {
         case CMLB200_Q4_0: return M > 8 || M == 3;
-        case CMLB200_Q8_0: return M > 4 || M == 3 || (M > 1 && cmlb200_gemv_mma_rows_(W, epi) < M);
+        case CMLB200_Q8_0: return M > 4 || M == 3 || (M > 1 && cmlb200_gemv_mma_rows_(W, W2, epi) < M);
         case CMLB200_NF4: return true;
         default: return M > 1 || (W->type != CMLB200_Q5_K && W->cols >= 4096);
     }
@@ -288,12 +261,12 @@ int gemv_dispatch(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x,
     cudaStream_t st = as_stream(stream);
     const bool kquant = cmlb200_is_kquant_type_(W->type);
     if (kquant) CMLB_REQUIRE(EPI != EPI_SWIGLU, "%s: GGUF type %d has no fused SwiGLU kernel; use cmlb200_gemv twice and cmlb200_swiglu_f32", who, W->type);
-    if (split_is_faster(W, M, EPI)) return cmlb200_gemv_split_(W, W2, x, nullptr, 0.f, y, M, EPI, st);
+    if (split_is_faster(W, W2, M, EPI)) return cmlb200_gemv_split_(W, W2, x, nullptr, 0.f, y, M, EPI, st);
     if (kquant) {
         return cmlb200_gemv_kquant_(W, x, y, M, EPI == EPI_ACCUM, st);
     }
     const bool tc_ok = W->type != CMLB200_NF4 && M > kDp4aMaxM && W->tiles && EPI != EPI_SWIGLU && W->cols % 128 == 0 && ((uintptr_t)y & 15) == 0;
-    if (W->type == CMLB200_Q4_0 && M > 2 && (M > 4 || cmlb200_gemv_mma_rows_(W, EPI) < M) && cmlb200_gemv_mma8_ok_(W, EPI)) {
+    if (W->type == CMLB200_Q4_0 && M > 2 && (M > 4 || cmlb200_gemv_mma_rows_(W, W2, EPI) < M) && cmlb200_gemv_mma8_ok_(W, W2, EPI)) {
         // eight rows of x per launch of the plane-major mma.sync kernel: the weight is streamed once per eight rows
         for (int m0 = 0; m0 < M && rc == 0; m0 += 8)
             rc = cmlb200_gemv_mma8_(W, W2, x + (size_t)m0 * W->cols, nullptr, 0.f, y + (size_t)m0 * W->rows, M - m0 < 8 ? M - m0 : 8, EPI, st);
@@ -302,7 +275,7 @@ int gemv_dispatch(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x,
     if (W->type != CMLB200_NF4 && M <= kMmaMaxM) {
         // the mma.sync kernel streams the weight once per launch: take it while two launches cover M
         // (or when there is no tile-major copy for the tcgen05 kernel)
-        const int per = cmlb200_gemv_mma_rows_(W, EPI);
+        const int per = cmlb200_gemv_mma_rows_(W, W2, EPI);
         if (per > 0 && ((M + per - 1) / per <= 2 || !tc_ok)) return cmlb200_gemv_mma_(W, W2, x, nullptr, 0.f, nullptr, y, M, EPI, st);
     }
     if (W->type != CMLB200_NF4 && M > kDp4aMaxM && W->tiles && EPI != EPI_SWIGLU && W->cols % 128 == 0 &&

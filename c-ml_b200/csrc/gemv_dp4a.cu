@@ -22,20 +22,7 @@
 // gemv_mma.cu takes the shapes it can (K % 256 == 0 and a digit table that fits shared memory) and
 // is tried first.
 #include "common.cuh"
-
-int cmlb200_x_digits_(const float* x, int M, int K, uint32_t* xq, cudaStream_t st);
-// gemv_mma.cu: the tensor-core kernel for the shapes it takes
-bool cmlb200_gemv_mma_ok_(const cmlb200_qmat* W, int epi, int M);
-int cmlb200_gemv_mma_rows_(const cmlb200_qmat* W, int epi);
-int cmlb200_gemv_mma_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps,
-                      const uint32_t* xq, float* y, int M, int epi, cudaStream_t st);
-// gemv_mma8.cu: its sibling for 5 to 8 rows of x in one launch (Q4_0, fp32 x)
-bool cmlb200_gemv_mma8_ok_(const cmlb200_qmat* W, int epi);
-bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W);
-int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps, float* y, int M, int epi,
-                        cudaStream_t st);
-int cmlb200_gemv_mma8_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps, float* y, int M,
-                       int epi, cudaStream_t st);
+#include "gemv_paths.cuh"
 
 namespace {
 
@@ -339,10 +326,10 @@ int cmlb200_x_digits_(const float* x, int M, int K, uint32_t* xq, cudaStream_t s
 int cmlb200_gemv_dp4a_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps,
                        const uint32_t* xq, float* y, int M, int epi, cudaStream_t st) {
     // three rows (the 4-row kernel would need two launches or pad), and Q8_0 from three on: as in gemv.cu
-    if (!xq && M > 2 && (M == 3 || W->type == CMLB200_Q8_0) && cmlb200_gemv_split_ok_(W)) return cmlb200_gemv_split_(W, W2, x, norm_w, eps, y, M, epi, st);
+    if (!xq && M > 2 && (M == 3 || W->type == CMLB200_Q8_0) && cmlb200_gemv_split_ok_(W, W2)) return cmlb200_gemv_split_(W, W2, x, norm_w, eps, y, M, epi, st);
     // more rows of x than one launch of the 4-row kernel takes for this shape: the 8-row kernel streams the weight once
-    if (!xq && M > 2 && M <= 8 && (M > 4 || cmlb200_gemv_mma_rows_(W, epi) < M) && cmlb200_gemv_mma8_ok_(W, epi)) return cmlb200_gemv_mma8_(W, W2, x, norm_w, eps, y, M, epi, st);
-    if (cmlb200_gemv_mma_ok_(W, epi, M)) return cmlb200_gemv_mma_(W, W2, xq ? nullptr : x, norm_w, eps, xq, y, M, epi, st);
+    if (!xq && M > 2 && M <= 8 && (M > 4 || cmlb200_gemv_mma_rows_(W, W2, epi) < M) && cmlb200_gemv_mma8_ok_(W, W2, epi)) return cmlb200_gemv_mma8_(W, W2, x, norm_w, eps, y, M, epi, st);
+    if (cmlb200_gemv_mma_ok_(W, W2, epi)) return cmlb200_gemv_mma_(W, W2, xq ? nullptr : x, norm_w, eps, xq, y, M, epi, st);
     uint32_t* ws = nullptr;
     if (xq) x = nullptr;
     else {                            // the register kernel reads digits from the library's scratch
@@ -494,5 +481,6 @@ extern "C" int cmlb200_gemv_rmsnorm(const cmlb200_qmat* W, const cmlb200_qmat* W
     if (epi == EPI_SWIGLU)
         CMLB_REQUIRE(W2 && W2->qs && W2->scales && W2->type == W->type && W2->rows == W->rows && W2->cols == W->cols,
                      "cmlb200_gemv_rmsnorm: SwiGLU needs a second weight of the same type and shape");
+    CMLB_REQUIRE(((uintptr_t)W->qs & 15) == 0 && (epi != EPI_SWIGLU || ((uintptr_t)W2->qs & 15) == 0), "cmlb200_gemv_rmsnorm: weight planes must be 16-byte aligned");
     return cmlb200_gemv_dp4a_(W, epi == EPI_SWIGLU ? W2 : nullptr, d_x, d_norm_w_f16, eps, nullptr, d_y, M, epi, as_stream(stream));
 }

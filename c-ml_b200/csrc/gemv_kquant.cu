@@ -11,6 +11,7 @@
 // 32-element sub-block in 16 consecutive bytes, src/core/gguf_quant.c:174-187), not ggml's.
 // Left with columns that are no whole 256 and very long rows: the fp16-split kernels (gemv_split.cuh) take the others.
 #include "common.cuh"
+#include "gemv_paths.cuh"
 
 namespace {
 

@@ -33,6 +33,7 @@
 // (src/core/gguf.c:271-295 + src/ops/ir/execution.c:989-1052, 3090-3134) like the other GEMV
 // kernels.
 #include "common.cuh"
+#include "gemv_paths.cuh"
 #include "mma_util.cuh"
 
 namespace {
@@ -557,18 +558,18 @@ bool fits(int nblk, int epi, int mt) {
 
 // Shapes the tensor-core decode kernel takes: whole 8-block slices of K with 16-byte aligned
 // scale rows, and room in shared memory for the digit table of two rows of x next to the rings.
-bool cmlb200_gemv_mma_ok_(const cmlb200_qmat* W, int epi, int M) {
+bool cmlb200_gemv_mma_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int epi) {
     if (W->type != CMLB200_Q4_0 && W->type != CMLB200_Q8_0) return false;
     if (W->cols % 256 != 0 || ((uintptr_t)W->qs & 15) || ((uintptr_t)W->scales & 15)) return false;
-    const int nblk = W->cols / 32;
-    (void)M;                                   // rows of x go four, two or one per launch, whatever fits
+    if (W2 && (((uintptr_t)W2->qs | (uintptr_t)W2->scales) & 15)) return false;
+    const int nblk = W->cols / 32;             // (rows of x go four, two or one per launch, whatever fits)
     return W->type == CMLB200_Q8_0 ? fits<CMLB200_Q8_0>(nblk, epi, 1) : fits<CMLB200_Q4_0>(nblk, epi, 1);
 }
 
 // Rows of x one launch of the tensor-core decode kernel takes for this weight: 4, 2, 1, or 0 when
 // the shape is outside the kernel.
-int cmlb200_gemv_mma_rows_(const cmlb200_qmat* W, int epi) {
-    if (!cmlb200_gemv_mma_ok_(W, epi, 1)) return 0;
+int cmlb200_gemv_mma_rows_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int epi) {
+    if (!cmlb200_gemv_mma_ok_(W, W2, epi)) return 0;
     const int nblk = W->cols / 32;
     const bool q8 = W->type == CMLB200_Q8_0;
     for (int mt = 4; mt >= 2; mt >>= 1)
@@ -603,7 +604,7 @@ extern "C" int cmlb200_gemv_tp_allreduce(const cmlb200_qmat* W, const float* d_x
     CMLB_REQUIRE(W && W->qs && W->scales && d_x && d_h && ws, "cmlb200_gemv_tp_allreduce: NULL argument");
     CMLB_REQUIRE(M >= 1 && M <= 4, "cmlb200_gemv_tp_allreduce: M=%d outside 1..4", M);
     CMLB_REQUIRE(tp >= 2 && tp <= kTpMaxRanks && rank >= 0 && rank < tp, "cmlb200_gemv_tp_allreduce: tp=%d rank=%d (tp must be 2..8)", tp, rank);
-    CMLB_REQUIRE(cmlb200_gemv_mma_ok_(W, EPI_STORE, M), "cmlb200_gemv_tp_allreduce: weight %dx%d type %d is outside the tensor-core decode kernel", W->rows, W->cols, W->type);
+    CMLB_REQUIRE(cmlb200_gemv_mma_ok_(W, nullptr, EPI_STORE), "cmlb200_gemv_tp_allreduce: weight %dx%d type %d is outside the tensor-core decode kernel", W->rows, W->cols, W->type);
     CMLB_REQUIRE((size_t)M * W->rows * 2 <= max_floats, "cmlb200_gemv_tp_allreduce: M*rows = %zu exceeds the workspace (max_floats / 2)", (size_t)M * W->rows);
     CMLB_REQUIRE(cmlb_num_sms() <= kTpGemvSlices, "cmlb200_gemv_tp_allreduce: more than %d SMs", kTpGemvSlices);
     CMLB_REQUIRE(((uintptr_t)d_x & 15) == 0, "cmlb200_gemv_tp_allreduce: x must be 16-byte aligned");
@@ -618,5 +619,5 @@ extern "C" int cmlb200_gemv_tp_allreduce(const cmlb200_qmat* W, const float* d_x
 }
 
 extern "C" int cmlb200_gemv_tp_fused_ok(const cmlb200_qmat* W, int M) {
-    return W && W->qs && W->scales && M >= 1 && M <= 4 && cmlb200_gemv_mma_ok_(W, EPI_STORE, M) && cmlb_num_sms() <= kTpGemvSlices ? 1 : 0;
+    return W && W->qs && W->scales && M >= 1 && M <= 4 && cmlb200_gemv_mma_ok_(W, nullptr, EPI_STORE) && cmlb_num_sms() <= kTpGemvSlices ? 1 : 0;
 }

@@ -25,6 +25,7 @@
 // grid = one CTA per SM. Replaces C-ML's dequantize-then-fp32-matmul
 // (src/core/gguf.c:271-295 + src/ops/ir/execution.c:989-1052, 3090-3134) for batched decode.
 #include "common.cuh"
+#include "gemv_paths.cuh"
 #include "mma_util.cuh"
 
 namespace {
@@ -366,8 +367,9 @@ int launch8(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const
 // Shapes the 8-row kernel takes: Q4_0, whole 8-block slices of K with 16-byte aligned scale rows,
 // and (for K of more than one phase) few enough items per CTA for their sums to fit in shared
 // memory next to the rings.
-bool cmlb200_gemv_mma8_ok_(const cmlb200_qmat* W, int epi) {
+bool cmlb200_gemv_mma8_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int epi) {
     if (W->type != CMLB200_Q4_0 || W->cols % 256 != 0 || W->cols / 256 > kMaxUnits || ((uintptr_t)W->qs & 15) || ((uintptr_t)W->scales & 15)) return false;
+    if (W2 && (((uintptr_t)W2->qs | (uintptr_t)W2->scales) & 15)) return false;
     return plan_of(W, epi == EPI_SWIGLU ? 2 : 1).smem <= kSmemLimit;
 }
 
@@ -381,10 +383,8 @@ int cmlb200_gemv_mma8_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const floa
     return quirk ? launch8<true>(W, W2, x, nw, eps, y, M, epi, st) : launch8<false>(W, W2, x, nw, eps, y, M, epi, st);
 }
 
-bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W);          // gemv_split.cu
-
 extern "C" int cmlb200_gemv_batched_from_planes(const cmlb200_qmat* W) {
     if (!W || !W->qs || !W->scales || W->rows <= 0 || W->cols <= 0) return 0;
-    if (W->type == CMLB200_Q8_0) return cmlb200_gemv_split_ok_(W) ? 1 : 0;
-    return cmlb200_gemv_mma8_ok_(W, EPI_STORE) && cmlb200_gemv_mma8_ok_(W, EPI_SWIGLU) ? 1 : 0;
+    if (W->type == CMLB200_Q8_0) return cmlb200_gemv_split_ok_(W, nullptr) ? 1 : 0;
+    return cmlb200_gemv_mma8_ok_(W, nullptr, EPI_STORE) && cmlb200_gemv_mma8_ok_(W, nullptr, EPI_SWIGLU) ? 1 : 0;
 }

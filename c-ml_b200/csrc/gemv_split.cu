@@ -1,6 +1,7 @@
 // Choice of the kernels of gemv_split.cuh and the rows of x as their B operands.
 #include "gemv_split.cuh"
 #include "call_scratch.cuh"
+#include "gemv_paths.cuh"
 
 int cmlb200_split_q4_(void* args, int nt, int quirk, cudaStream_t st);
 int cmlb200_split_q8_(void* args, int nt, int quirk, cudaStream_t st);
@@ -94,7 +95,8 @@ constexpr int kMaxUnits = 512;                               // K < 131072
 
 // Weights the kernels take: whole 16-byte rows of quants and whole 256-column units of scales, or (NF4) blocks of 32, 64, 128
 // or a multiple of 256 columns
-bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W) {
+bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2) {
+    if (W2 && !cmlb200_gemv_split_ok_(W2, nullptr)) return false;
     if (W->cols / 256 >= kMaxUnits || ((uintptr_t)W->qs & 15)) return false;
     switch (W->type) {
         case CMLB200_Q4_0:
@@ -161,8 +163,8 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
 // Projections of RMS-normalised rows in one or two launches, for the LLaMA's decode steps beyond what cmlb200_gemv_rmsnorm takes:
 // any block format the kernels take, up to 32 rows; epi 2 (SwiGLU) up to 8, where a CTA's row tiles come in pairs at no cost.
 extern "C" int cmlb200_gemv_norm_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M) {
-    if (M < 1 || M > (W2 ? 8 : 32) || W->rows <= 0 || W->cols <= 0 || !cmlb200_gemv_split_ok_(W)) return 0;
-    return !W2 || (W2->type == W->type && W2->rows == W->rows && W2->cols == W->cols && W2->block == W->block && cmlb200_gemv_split_ok_(W2));
+    if (M < 1 || M > (W2 ? 8 : 32) || W->rows <= 0 || W->cols <= 0 || !cmlb200_gemv_split_ok_(W, W2)) return 0;
+    return !W2 || (W2->type == W->type && W2->rows == W->rows && W2->cols == W->cols && W2->block == W->block);
 }
 extern "C" int cmlb200_gemv_norm_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* d_x, const uint16_t* d_norm_w, float eps, float* d_y, int M,
                                   void* stream) {

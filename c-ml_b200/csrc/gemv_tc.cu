@@ -36,6 +36,7 @@
 // bounded and reports through cmlb200_gemm_status.
 #include <string.h>
 #include "common.cuh"
+#include "gemv_paths.cuh"
 
 __device__ int g_tc_status = 0;   // 0 = ok; otherwise the code of the bounded wait that expired
 
