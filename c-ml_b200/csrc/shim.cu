@@ -1,6 +1,7 @@
 // Device plumbing of the cmlb200 C-ABI: errors, memory, copies, streams.
 #include <stdarg.h>
 #include <string.h>
+#include "call_scratch.cuh"
 #include "common.cuh"
 
 static thread_local char g_err[512] = "";
@@ -71,7 +72,9 @@ extern "C" int cmlb200_stream_create(void** stream) {
     return CMLB200_OK;
 }
 extern "C" int cmlb200_stream_destroy(void* stream) {
-    if (stream) CMLB_CUDA(cudaStreamDestroy(as_stream(stream)));
+    if (!stream) return CMLB200_OK;
+    cmlb_scratch_release(as_stream(stream));
+    CMLB_CUDA(cudaStreamDestroy(as_stream(stream)));
     return CMLB200_OK;
 }
 extern "C" int cmlb200_stream_sync(void* stream) {

@@ -145,7 +145,7 @@ def test_graph_outlives_its_capture_stream(pkg, weights, torch_dev):
 
 
 def test_graphs_give_their_scratch_back(pkg, weights, torch_dev):
-    """200 graphs, of 600 KB of scratch each, one after another: what stays is no more than the pool may keep."""
+    """200 graphs, of 2 MB of scratch each, one after another: what stays is no more than the pool may keep."""
     rng = np.random.default_rng(5)
     W = weights("nf4", 2048, 4096)
     x, y = rows(rng, 32, 4096, torch_dev), torch.empty(32, 2048, device=torch_dev)
