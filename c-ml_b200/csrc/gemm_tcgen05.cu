@@ -30,8 +30,8 @@
 //   Q8_0  convert, multiply in fp32, round once
 // Q4_0 and NF4 therefore round twice (scale or code value to bf16, then the product); the path's
 // tolerance is 1e-2 of the largest output. No cluster multicast is used. Every wait on an
-// mbarrier is bounded; on expiry the CTA raises a status flag (cmlb200_gemm_status), waits for
-// its copies in flight, frees its tensor memory and returns.
+// mbarrier is bounded; on expiry the CTA raises a status flag (cmlb200_gemm_status), waits for its
+// copies and MMAs in flight (each has a barrier of its own), frees its tensor memory and returns.
 #include <cuda.h>
 #include <type_traits>
 #include "common.cuh"
@@ -47,7 +47,11 @@ constexpr int BN = 128;             // weight rows of a tile
 constexpr int B_ROWS = 256;         // activation rows of a box and an MMA
 constexpr int B_BYTES = B_ROWS * BK * 2;        // 32 KB
 constexpr int AHEAD = 3;                        // slabs whose packed weights a thread has requested
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
+#ifndef CML_GEMM_SPIN_LIMIT
+#define CML_GEMM_SPIN_LIMIT (1u << 22)          // (a test builds this file with a limit that runs out)
+#endif
+constexpr uint32_t SPIN_LIMIT = CML_GEMM_SPIN_LIMIT;
+constexpr uint32_t DRAIN_LIMIT = 1u << 22;
 
 // A group always comes back to the same stages, so a parity wait is never two phases from its barrier.
 // WIDE (NX > 256): activations come in boxes of 256 rows of a ring of their own, two a slab; otherwise a stage holds both operands.
@@ -98,6 +102,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = code;
     atomicCAS(&g_gemm_status, 0, code);
     return false;
+}
+// Waits for something that is under way whoever has aborted: a copy of this CTA, or its last MMAs.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    for (uint32_t it = 0; it < DRAIN_LIMIT && !mbar_try(bar, parity); ++it)
+        if (it > 1024) __nanosleep(32);
 }
 // Every lane waits on the barrier itself (each reader of bytes that a tensor load wrote has to
 // observe the barrier's phase on its own); the verdict is then made warp-uniform so that no lane
@@ -318,7 +327,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
     while ((int)tmem_cols < p.NX) tmem_cols <<= 1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), C::GROUP_WARPS + (WIDE ? 0 : 1)); mbar_init(empty_a(s), 1); }
+        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), C::GROUP_WARPS); mbar_init(empty_a(s), 1); }
         for (int s = 0; s < BST; s++) { mbar_init(full_b(s), 1); mbar_init(empty_b(s), 1); }
         mbar_init(done_bar, 1);
         mbar_init(free_bar, DQ_WARPS);
@@ -340,12 +349,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         // ---------------- TMA producer: activation slabs (operand B) ----------------
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            // not WIDE: the box of a slab goes with its expanded weights, in the stage's barriers; counters instead of divisions
+            // not WIDE: a stage's box and expanded weights are free together; counters instead of divisions
             const int boxes = WIDE ? 2 : 1, total = slabs * boxes;
             int bi = 0, s = 0, kb = kb0, tile = first_tile, upper = 0;
             uint32_t phase = 1;
             for (; bi < total; bi++) {
-                const uint32_t bar = WIDE ? full_b(s) : full_a(s);
+                const uint32_t bar = full_b(s);
                 if (!mbar_wait(WIDE ? empty_b(s) : empty_a(s), phase, abort_flag, 1)) break;
                 mbar_expect_tx(bar, (uint32_t)n_lo * BK * 2);
                 tma_load_2d(sbase + C::b_off + s * B_BYTES, &xmap, kb * BK, (tile % p.tiles_m) * p.NX + upper * B_ROWS, bar);
@@ -353,19 +362,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                 if (WIDE) upper ^= 1;
                 if (upper == 0 && ++kb == kb1) { kb = kb0; tile += step; }
             }
-            for (int i = max(0, bi - BST); i < bi; i++) mbar_wait(WIDE ? full_b(i % BST) : full_a(i % BST), (i / BST) & 1, abort_flag, 2);   // no copy outlives its CTA
+            for (int i = max(0, bi - BST); i < bi; i++) mbar_drain(full_b(i % BST), (i / BST) & 1);   // no copy outlives its CTA
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: the warp stays converged, an elected lane issues ----
         const uint32_t ibase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 4) << 24);
         const uint32_t idesc = ibase | ((uint32_t)(n_lo >> 3) << 17), idesc_hi = ibase | ((uint32_t)(n_hi >> 3) << 17);
         bool ok = true;
-        int s = 0, sb = 0;
+        int s = 0, sb = 0, seg = 0;
         uint32_t phase = 0, phase_b = 0;
-        for (int seg = 0; seg < my_tiles && ok; seg++) {
+        for (; seg < my_tiles && ok; seg++) {
             if (seg) ok = warp_wait(free_bar, (seg - 1) & 1, abort_flag, 7);
             for (int i = 0; i < nkb && ok; i++) {
-                ok = warp_wait(full_a(s), phase, abort_flag, 3);
+                // (the box first: it is there earlier, so its wait hides behind the expansion's)
+                ok = (WIDE || warp_wait(full_b(s), phase, abort_flag, 4)) && warp_wait(full_a(s), phase, abort_flag, 3);
                 if (!ok) break;
                 const uint64_t adesc = make_desc_sw128(sbase + C::a_off + s * A_BYTES);
                 auto half = [&](int b, uint32_t acc, uint32_t id) {
@@ -400,6 +410,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
             if (elect_one()) umma_commit(done_bar);      // arrives once every MMA issued so far has retired
             __syncwarp();
         }
+        if (!ok && seg > 0) mbar_drain(done_bar, (seg - 1) & 1);          // tensor memory and the stages outlive the MMAs
     } else {
         // ---------------- weight expansion (operand A), then epilogue ----------------
         const int dqw = warp - 2, grp = dqw / C::GROUP_WARPS, tg = (dqw % C::GROUP_WARPS) * 32 + lane;

@@ -1,6 +1,11 @@
 """GPU parity of the tcgen05 prefill dequant-GEMM (bf16 activations/outputs, fp32 accumulate
 in tensor memory). Tolerance 1e-2 relative to max|y| (bf16 tensor-core prefill), as the path
 is specified; the oracle is fed the fp32 values of the bf16-rounded activations."""
+import ctypes as C
+import shutil
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -152,3 +157,38 @@ def test_gemm_output_modes(pkg, synth, ob, orc, torch_dev, M):
     assert pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, 3, buf.data_ptr(), None, stream_ptr()) == -1      # SwiGLU needs the gate
     assert pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, 7, buf.data_ptr(), None, stream_ptr()) == -1
 
+
+
+@pytest.fixture(scope="module")
+def impatient(tmp_path_factory, pkg):
+    """The same source with waits that give up after a single poll."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    root = Path(__file__).resolve().parents[1]
+    src, out = root / "c-ml_b200" / "csrc", tmp_path_factory.mktemp("impatient") / "gemm.so"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-DCML_GEMM_SPIN_LIMIT=1u", "-Xcompiler", "-fPIC", "-shared",
+                    "-I", str(root / "include"), "-I", str(src), *(str(src / f) for f in ("gemm_tcgen05.cu", "shim.cu", "call_scratch.cu")),
+                    "-Xlinker", "-Bsymbolic", "-o", str(out)], check=True, capture_output=True)
+    lib = C.CDLL(str(out))
+    for name in ("cmlb200_gemm_bf16", "cmlb200_gemm_status"):
+        getattr(lib, name).argtypes = getattr(pkg.lib, name).argtypes
+    return lib
+
+
+@pytest.mark.parametrize("kind,N,K,M", [("q4_0", 4096, 4096, 77), ("nf4", 1024, 2048, 200), ("q8_0", 2048, 4096, 512), ("q4_0", 20000, 1024, 513)])
+def test_gemm_waits_that_expire(pkg, synth, ob, orc, torch_dev, impatient, kind, N, K, M):
+    """Launches whose waits run out report it and return with nothing of theirs under way: launches in front of and behind them,
+    which share their SMs, are right, and so is the next call."""
+    rng = np.random.default_rng(1200 + N)
+    W, _ = make_weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K)
+    x = to_dev(synth.bf16_round(rng.standard_normal((M, K)).astype(np.float32))[0].reshape(M, K), torch_dev)
+    y, want, lost = [torch.zeros((M, N), dtype=torch.uint16, device=torch_dev) for _ in range(3)]
+    st = C.c_int(0)
+    pkg.check(pkg.lib.cmlb200_gemm_bf16(W.q, x.data_ptr(), want.data_ptr(), M, stream_ptr()), "gemm")
+    for _ in range(20):
+        y.zero_()
+        assert impatient.cmlb200_gemm_bf16(W.q, x.data_ptr(), lost.data_ptr(), M, stream_ptr()) == 0
+        pkg.check(pkg.lib.cmlb200_gemm_bf16(W.q, x.data_ptr(), y.data_ptr(), M, stream_ptr()), "gemm")
+        torch.cuda.synchronize()
+        assert torch.equal(y.view(torch.int16), want.view(torch.int16))
+        assert impatient.cmlb200_gemm_status(C.byref(st), 1) == 0 and st.value != 0
+    assert gemm_status(pkg) == 0
