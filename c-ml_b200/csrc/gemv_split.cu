@@ -11,11 +11,13 @@ int cmlb200_split_k_(int type, void* args, int nt, cudaStream_t st);
 namespace {
 
 // Rows of x as B operands in global memory. One CTA per row of x (rows from M on: zeros); RMSNorm (src/nn/llama.c:71-124) first
-// when a weight is given. CONTIG: a thread of the product takes 8 neighbouring columns (NF4).
+// when a weight is given. CONTIG: a thread of the product takes 8 neighbouring columns (NF4). follow: scalings of a row lie no further
+// apart than 2^40, so that sums may follow them from unit to unit.
+constexpr int kKept = 3;
 template <bool CONTIG>
 __global__ void __launch_bounds__(512)
-x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float eps, int K, int M, int NT, uint4* __restrict__ planes,
-               float* __restrict__ sums, float* __restrict__ xf) {
+x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float eps, int K, int M, int NT, bool follow,
+               uint4* __restrict__ planes, float* __restrict__ sums, float* __restrict__ xf) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float red[2][16];
@@ -44,39 +46,55 @@ x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float
             e[2 * k + 1] *= f.y;
         }
     };
-    float most = 0.f, ss = 0.f;
-    for (int i = tid; i < items; i += 512) {
-        float e[8];
-        load(i, e);
+    float inv = 1.f, least = 0.f, kept[kKept][8];                   // a thread's first items stay in registers
+#pragma unroll
+    for (int n = 0; n < kKept; n++) load(tid + 512 * n, kept[n]);
+    if (nw || follow) {
+        float ss = 0.f, most = 0.f;
+        auto look = [&](int i, float (&e)[8]) {
+            if (nw) {
+#pragma unroll
+                for (int k = 0; k < 8; k++) ss = fmaf(e[k], e[k], ss);
+                weigh(i, e);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) most = fmaxf(most, fabsf(e[k]));
+        };
+#pragma unroll
+        for (int n = 0; n < kKept; n++) look(tid + 512 * n, kept[n]);
+        for (int i = tid + 512 * kKept; i < items; i += 512) {
+            float e[8];
+            load(i, e);
+            look(i, e);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        if (lane == 0) { red[0][warp] = most; red[1][warp] = ss; }
+        __syncthreads();
+        most = 0.f, ss = 0.f;
+#pragma unroll
+        for (int w = 0; w < 16; w++) { most = fmaxf(most, red[0][w]); ss += red[1][w]; }
+        if (nw) inv = 1.0f / sqrtf(ss / (float)K + eps);
+        if (follow) least = most * inv * 0x1p-40f;
+    }
+    auto put = [&](int i, float (&e)[8]) {                          // 32 items are a unit, a warp's
+        float s = 0.f, most = least, up, down;
         if (nw) {
 #pragma unroll
-            for (int k = 0; k < 8; k++) ss = fmaf(e[k], e[k], ss);
-            weigh(i, e);
+            for (int k = 0; k < 8; k++) e[k] *= inv;
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) most = fmaxf(most, fabsf(e[k]));
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-        ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    }
-    if (lane == 0) { red[0][warp] = most; red[1][warp] = ss; }
-    __syncthreads();
-    most = 0.f, ss = 0.f;
-#pragma unroll
-    for (int w = 0; w < 16; w++) { most = fmaxf(most, red[0][w]); ss += red[1][w]; }
-    const float inv = nw ? 1.0f / sqrtf(ss / (float)K + eps) : 1.f;
-    float up, down;
-    scaling(most * inv, up, down);
-    if (tid == 0) xf[row] = down;
-    for (int i = tid; i < items; i += 512) {
-        float e[8], s = 0.f;
-        load(i, e);
-        if (nw) weigh(i, e);
+        for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        scaling(most, up, down);
+        if (lane == 0) xf[(size_t)(i >> 5) * (8 * NT) + row] = down;
         uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int k = 0; k < 8; k++) { e[k] = e[k] * inv * up; s += e[k]; }
+        for (int k = 0; k < 8; k++) { e[k] *= up; s += e[k]; }
 #pragma unroll
         for (int k = 0; k < 4; k++) split2(e[4 * (k >> 1) + (k & 1)], e[4 * (k >> 1) + (k & 1) + 2], hi[k], lo[k]);
         const int blk = i >> 2, t = i & 3;
@@ -86,6 +104,15 @@ x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         if (t == 0) sums[(size_t)blk * (8 * NT) + row] = s;
+    };
+#pragma unroll
+    for (int n = 0; n < kKept; n++)
+        if (tid + 512 * n < items) put(tid + 512 * n, kept[n]);
+    for (int i = tid + 512 * kKept; i < items; i += 512) {
+        float e[8];
+        load(i, e);
+        if (nw) weigh(i, e);
+        put(i, e);
     }
 }
 
@@ -133,13 +160,16 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
     if (nt) {
         const size_t blocks = (size_t)((p.K + 255) / 256) * 8, plane_bytes = blocks * nt * 64 * sizeof(uint4), sum_bytes = blocks * 8 * nt * sizeof(float);
         uint8_t* base = nullptr;
-        int rc = scratch.get(st, plane_bytes + sum_bytes + 8 * nt * sizeof(float), (void**)&base);
+        int rc = scratch.get(st, plane_bytes + sum_bytes + sum_bytes / 8, (void**)&base);
         if (rc) return rc;
         uint4* planes = reinterpret_cast<uint4*>(base);
-        float *sums = reinterpret_cast<float*>(base + plane_bytes), *xf = reinterpret_cast<float*>(base + plane_bytes + sum_bytes);
+        float* sums = reinterpret_cast<float*>(base + plane_bytes);
+        float* xf = reinterpret_cast<float*>(base + plane_bytes + sum_bytes);
         p.planes = planes;
         p.sums = sums;
         p.xf = xf;
+        const int shares = nt == 4 ? kWarps / 2 : kWarps, units = (p.K + 255) / 256;
+        const bool follow = nt > 1 && units > shares && !split_deep(W->type, units, shares);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(8 * nt);
         cfg.blockDim = dim3(512);
@@ -149,7 +179,7 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CMLB_CUDA(cudaLaunchKernelEx(&cfg, W->type == CMLB200_NF4 ? x_split_kernel<true> : x_split_kernel<false>, x, p.nw, eps, p.K, M, nt, planes, sums, xf));
+        CMLB_CUDA(cudaLaunchKernelEx(&cfg, W->type == CMLB200_NF4 ? x_split_kernel<true> : x_split_kernel<false>, x, p.nw, eps, p.K, M, nt, follow, planes, sums, xf));
     }
     const int quirk = (W->flags & CMLB200_QMAT_SUBNORMAL_SCALES) || (W2 && (W2->flags & CMLB200_QMAT_SUBNORMAL_SCALES));
     switch (W->type) {

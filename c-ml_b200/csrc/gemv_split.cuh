@@ -4,7 +4,7 @@
 //   * the quants are small integers, which fp16 holds exactly: A = 16 weight rows x 16 quants, made in registers with
 //     one or two logic / packed-half operations per register;
 //   * x is split into two fp16 numbers, x = hi + lo, after scaling by a power of two that puts the largest value of its
-//     slice just below 2^9: 22 bits of every value, and nothing below 2^-32 of the largest is lost;
+//     256-column unit just below 2^15: 23 bits of every value, and nothing below 2^-39 of the largest is lost;
 //   * products and sums of one block are fp32 in the tensor core; block scales are applied to its sums in fp32, the
 //     minima of Q4_K / Q5_K by one more small product (sub-block minima times sums of x), those of Q4_1 in fp32.
 // Error against 64 bits on N(0,1) inputs: 1.2e-7 to 2e-7 of the result's norm, as the int8-digit kernels have.
@@ -52,10 +52,11 @@ struct SplitArgs {
     const __half* nw;              // RMSNorm weight applied to them, or nullptr
     const uint4* planes;           // split rows (NT > 0): [block][NT][hi, lo][lane]
     const float* sums;             // their sums over blocks: [block][8 NT]
-    const float* xf;               // power of two that undoes the scaling, per row
+    const float* xf;               // power of two that undoes the scaling: [unit][8 NT]
     float* y;
     float eps;
     int N, K, M, tiles, per_cta, stages, epi;
+    int extra;                     // 9 rows and more: where in shared memory the address of tensor memory and the scalings go
     int nf4_shift;                 // log2 of how many 32-column blocks one NF4 scale covers, 3 at most
     int nf4_units;                 // units one covers, 1 at least
 };
@@ -298,19 +299,43 @@ __device__ __forceinline__ float offset_of(Shared at, const Head& h, int b, floa
 }
 
 // ---- activations --------------------------------------------------------------------------------------------------------
-// The power of two that brings values of magnitude up to `most` below 2^9, and its inverse
+// The power of two that brings values of magnitude up to `most` below 2^15, and its inverse
 __device__ __forceinline__ void scaling(float most, float& up, float& down) {
     const int e = (int)(__float_as_uint(most) >> 23);
-    const int f = min(262 - e, 253);                            // exponent field of 2^(8 - floor(log2 most))
+    const int f = min(268 - e, 253);                            // exponent field of 2^(14 - floor(log2 most))
     up = __uint_as_float((uint32_t)f << 23);
     down = __uint_as_float((uint32_t)(254 - f) << 23);
 }
+__device__ __forceinline__ float power(uint32_t field) { return __uint_as_float((field & 255u) << 23); }
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(a, b);
     const float2 f = __half22float2(h);
     const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// One output's sums of the warps, in four chains: fewer roundings one upon the other than in a row
+template <int COLS> __device__ __forceinline__ float warp_sums(const float* src, int active) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int w = 0; w < 16; w++)
+        if (w < active) v[w & 3] += src[w * (COLS * 16)];
+    return (v[0] + v[1]) + (v[2] + v[3]);
+}
+
+// Eight sums of a thread to and from eight columns of tensor memory
+__device__ __forceinline__ void tmem_put8(uint32_t at, const float (&v)[2][4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+                 ::"f"(v[0][0]), "f"(v[0][1]), "f"(v[0][2]), "f"(v[0][3]), "f"(v[1][0]), "f"(v[1][1]), "f"(v[1][2]), "f"(v[1][3]), "r"(at) : "memory");
+}
+__device__ __forceinline__ void tmem_add8(uint32_t at, float (&v)[2][4]) {
+    float r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "r"(at));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k >> 2][k & 3] += r[k];
 }
 
 // ---- up to 8 rows of x ------------------------------------------------------------------------------------------------------
@@ -359,7 +384,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         const int un = warp + u * W;
         uint32_t B[8][NT == 0 ? 4 : 8];                         // NT = 0: hi (even g) or lo (odd g) of row g/2; 1: hi, then lo of row g
         float s32[kMins<F> ? 8 : 1][2];                         // sums of x over the unit's blocks, of the thread's two columns
-        float down = 1.f;
+        float down = 1.f, down1 = 1.f;                          // undo the unit's scaling, of the thread's (two) columns
         if (NT == 0) {
             // one row at a time, eight columns a lane: block lane/4, the columns of thread t = lane%4 of the product
             __syncwarp();
@@ -429,6 +454,9 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
                     s32[kMins<F> ? b : 0][1] = v.y;
                 }
             }
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(p.xf + (size_t)un * 8 + 2 * t));
+            down = v.x;
+            down1 = v.y;
         }
         for (int i = 0; i < mine; i++) {
             const int tile = tile0 + i, row0 = (pairs ? tile >> 1 : tile) * 16;
@@ -446,12 +474,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
                 float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 constexpr int C1 = F == CMLB200_Q6_K ? 1 : 0;   // Q6_K: a scale for each half
 #pragma unroll
-                for (int k = 0; k < 2; k++)
+                for (int d = kDigits<F> - 1; d >= 0; d--) {     // small products first: the tensor core truncates, relative to the sum so far
+                    if (NT) {
 #pragma unroll
-                    for (int d = 0; d < kDigits<F>; d++) {
-                        mma_f16(c[k * C1], a[d][k], B[b][2 * k], B[b][2 * k + 1]);
-                        if (NT) mma_f16(c[k * C1], a[d][k], B[b][NT ? 4 + 2 * k : 0], B[b][NT ? 5 + 2 * k : 0]);
+                        for (int k = 0; k < 2; k++) mma_f16(c[k * C1], a[d][k], B[b][NT ? 4 + 2 * k : 0], B[b][NT ? 5 + 2 * k : 0]);
                     }
+#pragma unroll
+                    for (int k = 0; k < 2; k++) mma_f16(c[k * C1], a[d][k], B[b][2 * k], B[b][2 * k + 1]);
+                }
 #pragma unroll
                 for (int k = 0; k <= C1; k++) {
                     const float sl = scale_of<F, QUIRK>(p, lo, hl, b, k), sh = scale_of<F, QUIRK>(p, hi, hh, b, k);
@@ -480,6 +510,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
                 dst[8] = v1;
             } else {
                 dst += 2 * t * 16 + g;
+                acc[0] *= down; acc[1] *= down1; acc[2] *= down; acc[3] *= down1;
                 if (u) { acc[0] += dst[0]; acc[1] += dst[16]; acc[2] += dst[8]; acc[3] += dst[24]; }
                 dst[0] = acc[0];
                 dst[16] = acc[1];
@@ -504,20 +535,18 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         const int row = ((pairs ? tile0 >> 1 : tile0) + o) * 16 + r;
         if (m >= p.M || row >= p.N) continue;
         float f = 1.f;
-        if (NT) f = __ldcg(p.xf + m);
-        else if (p.nw) {
+        if (NT == 0 && p.nw) {
             float q = 0.f;
             for (int w = 0; w < active; w++) q += squares[w * 4 + m];
             f = 1.0f / sqrtf(q / (float)p.K + p.eps);
         }
         const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
-        float v = 0.f, v2 = 0.f;
-        for (int w = 0; w < active; w++) v += src[w * (COLS * 16)];
+        float v = warp_sums<COLS>(src, active);
         v *= f;
         float* out = p.y + (size_t)m * p.N + row;
         if (pairs) {
-            for (int w = 0; w < active; w++) v2 += src[(W + w) * (COLS * 16)];
-            *out = (v / (1.0f + expf(-v))) * (v2 * f);
+            const float v2 = warp_sums<COLS>(src + W * (COLS * 16), active) * f;
+            *out = (v / (1.0f + expf(-v))) * v2;
         } else if (p.epi == EPI_ACCUM) *out += v;
         else *out = v;
     }
@@ -526,7 +555,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
 // ---- 9 to 32 rows of x --------------------------------------------------------------------------------------------------------
 // A warp has 16 columns (two products) of x and a share of K. CG = 1: sixteen shares; CG = 2 (17 rows of x and more): eight, whose
 // weights two warps read, each for its own columns.
-template <int F, int CG, int T, bool QUIRK>
+template <int F, int CG, int T, bool QUIRK, bool DEEP>
 __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, NT = 2, COLS = 16 * CG, W = kWarps / CG;
@@ -559,6 +588,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
     if (F == CMLB200_NF4) asm volatile("griddepcontrol.wait;" ::: "memory");
     issue(0);
     if (stages > 1) issue(1);
+    uint32_t* const tmem = reinterpret_cast<uint32_t*>(smem + p.extra);
+    if (DEEP) {
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(tmem)) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     float acc[T][NT][4];
@@ -575,9 +614,34 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         for (int j = 0; j < NT; j++) { nh[j] = __ldcg(src + j * 64); nl[j] = __ldcg(src + j * 64 + 32); }
     };
     if (my_units) fetch(share * 8);
+    // exponent fields of what undoes the scaling of the warp's columns, unit after unit
+    uint8_t* const fields = smem + p.extra + 16 + warp * (16 * ((units + W - 1) / W));
+    for (int i = lane; i < 4 * my_units; i += 32) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.xf + (size_t)(share + (i >> 2) * W) * COLS + 16 * cg + 4 * (i & 3)));
+        *reinterpret_cast<uint32_t*>(fields + 4 * i) = (__float_as_uint(v.x) >> 23) | (__float_as_uint(v.y) >> 23 << 8) | (__float_as_uint(v.z) >> 23 << 16) |
+                                                       (__float_as_uint(v.w) >> 23 << 24);
+    }
+    __syncwarp();
+    auto undoes = [&](int u) { return lds16(fields + 16 * u + 2 * t) | lds16(fields + 16 * u + 8 + 2 * t) << 16; };     // the thread's four columns
+    // a thread's place in tensor memory: its warp's 32 lanes, 64 columns for each of the four warps of a quadrant
+    const uint32_t totals = DEEP ? *tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * 64u : 0u;
     int buf = 0;
     for (int u = 0; u < my_units; u++) {
         const int un = share + u * W;
+        if (!DEEP && u) {                                       // the sums follow to the unit's scaling, exactly: by 2^40 at most (x_split_kernel)
+            const uint32_t now = undoes(u), before = undoes(u - 1);
+            if (now != before) {
+#pragma unroll
+                for (int j = 0; j < NT; j++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const int at = 8 * (2 * j + k);
+                        const float ratio = power(127u + ((before >> at) & 255u) - ((now >> at) & 255u));
+#pragma unroll
+                        for (int i = 0; i < T; i++) { acc[i][j][k] *= ratio; acc[i][j][k + 2] *= ratio; }
+                    }
+            }
+        }
         if (stages > 1) cp_async_wait<1>();
         else cp_async_wait<0>();
         meet();
@@ -612,14 +676,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
 #pragma unroll
                         for (int v = 0; v < 4; v++) c[k][j][v] = 0.f;
 #pragma unroll
-                for (int k = 0; k < 2; k++)
+                for (int d = kDigits<F> - 1; d >= 0; d--) {     // (as above)
 #pragma unroll
-                    for (int d = 0; d < kDigits<F>; d++) {
-#pragma unroll
-                        for (int j = 0; j < NT; j++) mma_f16(c[k * C1][j], a[d][k], k ? bh[j].z : bh[j].x, k ? bh[j].w : bh[j].y);
+                    for (int k = 0; k < 2; k++)
 #pragma unroll
                         for (int j = 0; j < NT; j++) mma_f16(c[k * C1][j], a[d][k], k ? bl[j].z : bl[j].x, k ? bl[j].w : bl[j].y);
-                    }
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+#pragma unroll
+                        for (int j = 0; j < NT; j++) mma_f16(c[k * C1][j], a[d][k], k ? bh[j].z : bh[j].x, k ? bh[j].w : bh[j].y);
+                }
 #pragma unroll
                 for (int k = 0; k <= C1; k++) {
                     const float sl = scale_of<F, QUIRK>(p, lo, hl, b, k), sh = scale_of<F, QUIRK>(p, hi, hh, b, k);
@@ -644,9 +710,43 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         meet();                                                 // every lane is done with this buffer
         issue(buf);
         if (++buf == stages) buf = 0;
+        if (DEEP) {
+            const uint32_t undo = undoes(u);
+#pragma unroll
+            for (int i = 0; i < T; i++) {
+#pragma unroll
+                for (int j = 0; j < NT; j++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (2 * j + (k & 1))));
+                if (u) tmem_add8(totals + 8 * i, acc[i]);
+                if (u + 1 < my_units) {
+                    tmem_put8(totals + 8 * i, acc[i]);
+#pragma unroll
+                    for (int j = 0; j < NT; j++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
+                }
+            }
+            if (u + 1 < my_units) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
     }
+    if (!DEEP && my_units) {
+        const uint32_t undo = undoes(my_units - 1);
+#pragma unroll
+        for (int i = 0; i < T; i++)
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (2 * j + (k & 1))));
+    }
+    if (DEEP) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cp_async_wait<0>();
+    const uint32_t held = DEEP ? *tmem : 0u;
     __syncthreads();                                            // the rings become the place where the warps' sums meet
+    if (DEEP && warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(held) : "memory");
+    }
     float* part = reinterpret_cast<float*>(smem);               // [T][W][COLS][16]
 #pragma unroll
     for (int i = 0; i < T; i++)
@@ -664,21 +764,25 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         const int r = idx & 15, m = (idx >> 4) % COLS, o = idx / (COLS * 16);
         const int row = ((pairs ? tile0 >> 1 : tile0) + o) * 16 + r;
         if (m >= p.M || row >= p.N) continue;
-        const float f = __ldcg(p.xf + m);
         const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
-        float v = 0.f, v2 = 0.f;
-        for (int w = 0; w < active; w++) v += src[w * (COLS * 16)];
-        v *= f;
+        const float v = warp_sums<COLS>(src, active);
         float* out = p.y + (size_t)m * p.N + row;
         if (pairs) {
-            for (int w = 0; w < active; w++) v2 += src[(W + w) * (COLS * 16)];
-            *out = (v / (1.0f + expf(-v))) * (v2 * f);
+            const float v2 = warp_sums<COLS>(src + W * (COLS * 16), active);
+            *out = (v / (1.0f + expf(-v))) * v2;
         } else if (p.epi == EPI_ACCUM) *out += v;
         else *out = v;
     }
 }
 
 // ---- host side ----------------------------------------------------------------------------------------------------------------------
+// One chain through all of a share's blocks rounds at the size of the result each time. For the formats whose former kernels summed
+// in shorter chains (1.25 to 1.35e-7 of the result off) chains of more than 16 blocks are cut: a unit's sums to those of the units before it, which lie in tensor memory meanwhile, for there are no registers for both.
+// K = 11008, 32 rows: NF4 1.57e-7 in one chain, 1.31e-7 so, Q6_K 1.85 and 1.24e-7. It costs 0.5 to 1 us a launch.
+inline bool split_deep(int type, int units, int W) {
+    return (type == CMLB200_Q6_K || type == CMLB200_NF4 || type == CMLB200_Q8_0) && units > 2 * W;
+}
+
 template <typename Kern>
 int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, const SplitArgs& p) {
     cudaLaunchConfig_t cfg = {};
@@ -696,6 +800,7 @@ int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, c
 }
 
 constexpr size_t kSmemMost = 227 * 1024;
+inline size_t wide_extra(const SplitArgs& p, int CG) { return 16 + (size_t)kWarps * 16 * (((p.K + 255) / 256 + kWarps / CG - 1) / (kWarps / CG)); }
 
 template <int F, int NT, bool QUIRK>
 int run_narrow(SplitArgs& p, cudaStream_t st) {
@@ -714,18 +819,20 @@ int run_narrow(SplitArgs& p, cudaStream_t st) {
     return launch_split(kern, (p.tiles + per - 1) / per, W, smem, st, p);
 }
 
-template <int F, int CG, int T, bool QUIRK>
+template <int F, int CG, int T, bool QUIRK, bool DEEP>
 int run_wide(SplitArgs& p, cudaStream_t st) {
     constexpr size_t stage = (size_t)(kWarps / CG) * T * kTileBytes<F>, sums = (size_t)T * kWarps * 16 * 16 * 4;
-    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage <= kSmemMost ? 2 : 1;
-    const size_t smem = p.stages * stage > sums ? p.stages * stage : sums;
-    auto kern = gemv_split_wide_kernel<F, CG, T, QUIRK>;
+    const size_t extra = wide_extra(p, CG);
+    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage + extra <= kSmemMost ? 2 : 1;
+    p.extra = (int)(p.stages * stage > sums ? p.stages * stage : sums);
+    const size_t smem = p.extra + extra;
+    auto kern = gemv_split_wide_kernel<F, CG, T, QUIRK, DEEP>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
     return launch_split(kern, (p.tiles + T - 1) / T, kWarps, smem, st, p);
 }
 
-template <int F, int CG, bool QUIRK>
+template <int F, int CG, bool QUIRK, bool DEEP>
 int run_wide_t(SplitArgs& p, cudaStream_t st) {
     constexpr int most = kSmemMost / (kWarps / CG * kTileBytes<F>);
     const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
@@ -734,14 +841,22 @@ int run_wide_t(SplitArgs& p, cudaStream_t st) {
     for (int i = 0; i < 4; i++) {
         const int T = choice[i];
         if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
+        if (T > 1 && (size_t)(kWarps / CG) * T * kTileBytes<F> + wide_extra(p, CG) > kSmemMost) continue;
         const int ctas = (p.tiles + T - 1) / T;
         const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
         if (cost < least) { least = cost; best = T; }
     }
-    if constexpr (most >= 5) if (best == 5) return run_wide<F, CG, 5, QUIRK>(p, st);
-    if constexpr (most >= 3) if (best == 3) return run_wide<F, CG, 3, QUIRK>(p, st);
-    if (best == 2) return run_wide<F, CG, 2, QUIRK>(p, st);
-    return run_wide<F, CG, 1, QUIRK>(p, st);
+    if constexpr (most >= 5) if (best == 5) return run_wide<F, CG, 5, QUIRK, DEEP>(p, st);
+    if constexpr (most >= 3) if (best == 3) return run_wide<F, CG, 3, QUIRK, DEEP>(p, st);
+    if (best == 2) return run_wide<F, CG, 2, QUIRK, DEEP>(p, st);
+    return run_wide<F, CG, 1, QUIRK, DEEP>(p, st);
+}
+
+template <int F, int CG, bool QUIRK>
+int run_wide_d(SplitArgs& p, cudaStream_t st) {
+    if constexpr (F == CMLB200_NF4 || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
+        if (split_deep(F, (p.K + 255) / 256, kWarps / CG)) return run_wide_t<F, CG, QUIRK, true>(p, st);
+    return run_wide_t<F, CG, QUIRK, false>(p, st);
 }
 
 template <int F, bool QUIRK>
@@ -749,8 +864,8 @@ int run_split(SplitArgs& p, int nt, cudaStream_t st) {
     switch (nt) {
         case 0: return run_narrow<F, 0, QUIRK>(p, st);
         case 1: return run_narrow<F, 1, QUIRK>(p, st);
-        case 2: return run_wide_t<F, 1, QUIRK>(p, st);
-        default: return run_wide_t<F, 2, QUIRK>(p, st);
+        case 2: return run_wide_d<F, 1, QUIRK>(p, st);
+        default: return run_wide_d<F, 2, QUIRK>(p, st);
     }
 }
 

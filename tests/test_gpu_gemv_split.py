@@ -1,14 +1,14 @@
 """The fp16-split decode kernels (cmlb200_gemv for NF4, Q4_1, Q4_K, Q6_K, larger batches of the others) where their tiles, units
 of columns, warps and batches end, against the dequantised weight in 64 bits.
 
-Bound of an output's error: x enters as two fp16 numbers (2^-22 of every value, once more for what fp16's smallest steps
-cut off), sums of a block and of the blocks are fp32 (2^-24 for each of K / 32 + 32 additions, twice that in the tensor core,
+Bound of an output's error: x enters as two fp16 numbers (2^-23 of every value, once more for what fp16's smallest steps
+cut off of a 256-column unit), sums of a block and of the blocks are fp32 (2^-24 for each of K / 32 + 32 additions, twice that in the tensor core,
 which truncates), all of it relative to the sum of the products' magnitudes."""
 import numpy as np
 import pytest
 import torch
 
-from gpu_util import make_block_stream, make_weight, stream_ptr, to_dev
+from gpu_util import DevQMat, make_block_stream, make_weight, stream_ptr, to_dev
 
 pytestmark = pytest.mark.gpu
 STREAM_TYPES = {"q4_1": 3, "q4_k": 12, "q5_k": 13, "q6_k": 14}
@@ -62,6 +62,52 @@ def test_any_range_of_x(pkg, synth, ob, orc, torch_dev, scale, M):
         x[1] = 0.0                                             # a row without a largest value
         x[2, ::7] *= 1e-4                                      # values of very different sizes in one row
         _check(pkg, W, Wf, x, torch_dev)
+
+
+def _with_zeros(pkg, synth, ob, orc, dev, rng, kind, N, K):
+    """A weight whose first 256 columns are zero."""
+    if kind == "nf4":
+        packed, scales = synth.nf4_weight(rng, N, K, 64)
+        packed = packed.reshape(N, K // 2)
+        packed[:, :128] = 0x77
+        packed = packed.reshape(-1)
+        return DevQMat.from_nf4(pkg, dev, packed, scales, N, K, 64), ob.dequant_nf4(orc, packed, scales, 64, N * K).reshape(N, K)
+    blocks = synth.q8_0_blocks(rng, N, K)
+    b = blocks.reshape(N, K // 32, 34)
+    b[:, :8, 2:] = 0
+    return DevQMat.from_gguf(pkg, dev, pkg.Q8_0, blocks, N, K), ob.dequant_blocks(orc, pkg.Q8_0, blocks, N * K).reshape(N, K)
+
+
+@pytest.mark.parametrize("kind", ["nf4", "q8_0"])
+@pytest.mark.parametrize("K", [2048, 8192, 9216])
+def test_units_of_very_different_sizes(pkg, synth, ob, orc, torch_dev, kind, K):
+    """Large values that meet zero weights take no bits from those in other units of 256 columns."""
+    rng = np.random.default_rng(K)
+    W, Wf = _with_zeros(pkg, synth, ob, orc, torch_dev, rng, kind, 70, K)
+    for M in (3, 7, 12, 30):
+        x = rng.standard_normal((M, K)).astype(np.float32)
+        for m in range(M):
+            x[m, :256] *= 10.0 ** (m % 8)                     # (2^40 lie between the scalings of a row's units at most)
+            x[m, 512:1024] *= 10.0 ** -(m % 5)
+        _check(pkg, W, Wf, x, torch_dev)
+
+
+@pytest.mark.parametrize("K", [1024, 4096, 11008])
+@pytest.mark.parametrize("kind,most", [("nf4", 1.42e-7), ("q6_k", 1.45e-7)])
+def test_error_against_64_bits(pkg, synth, ob, orc, torch_dev, kind, most, K):
+    """What plain fp32 multiply-adds (NF4: 1.17 to 1.34e-7) and 24-bit digits (Q6_K: 1.28 to 1.41e-7) of these inputs give, relative to
+    the norm of the results. 512 x M results: their norm spreads by less than 2 %."""
+    rng = np.random.default_rng(K)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, kind, 512, K)
+    for M in (1, 4, 5, 8, 9, 16, 17, 32):
+        x = rng.standard_normal((4, M, K)).astype(np.float32)
+        off = []
+        for part in x:
+            d_x, d_y = to_dev(part, torch_dev), torch.empty(M, 512, device=torch_dev)
+            pkg.check(pkg.lib.cmlb200_gemv(W.q, d_x.data_ptr(), d_y.data_ptr(), M, stream_ptr()), "gemv")
+            want = part.astype(np.float64) @ Wf.T.astype(np.float64)
+            off.append(np.linalg.norm(d_y.cpu().numpy() - want) / np.linalg.norm(want))
+        assert np.sqrt(np.mean(np.square(off))) <= most, (M, off)
 
 
 def test_streams_keep_their_rows_apart(pkg, synth, ob, orc, torch_dev):
