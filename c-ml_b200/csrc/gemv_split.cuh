@@ -338,6 +338,36 @@ __device__ __forceinline__ void tmem_add8(uint32_t at, float (&v)[2][4]) {
     for (int k = 0; k < 8; k++) v[k >> 2][k & 3] += r[k];
 }
 
+// An output that came out infinite or not a number, once more by plain fp32 multiply-adds: an infinite x is no pair of fp16 numbers
+// (inf - inf), and its products have signs. Formats whose former kernels had those results; rows as they are given.
+template <int F>
+__device__ __noinline__ float plain_dot(const uint8_t* qs, const uint8_t* sc, const float* x, int K, int row, int nf4_shift, int nf4_units) {
+    const int nblk = K / 32, per_row = (nblk >> nf4_shift) / nf4_units;
+    float sum = 0.f;
+    for (int b = 0; b < nblk; b++) {
+        const size_t blk = (size_t)row * nblk + b;
+        const float s = F == CMLB200_NF4 ? reinterpret_cast<const float*>(sc)[(size_t)row * per_row + (b >> nf4_shift) / nf4_units]
+                                         : cml_half_to_float(reinterpret_cast<const uint16_t*>(sc)[blk]);
+        float block = 0.f;
+        for (int k = 0; k < 32; k++) {
+            float w;
+            if (F == CMLB200_Q8_0) w = (float)reinterpret_cast<const int8_t*>(qs)[blk * 32 + k];
+            else if (F == CMLB200_Q4_0) w = (float)(int)((qs[blk * 16 + (k & 15)] >> (k < 16 ? 0 : 4)) & 15) - 8.0f;
+            else w = kNF4[(qs[blk * 16 + (k >> 1)] >> (k & 1 ? 0 : 4)) & 15];
+            block = fmaf(w, x[b * 32 + k], block);
+        }
+        sum = fmaf(block, s, sum);
+    }
+    return sum;
+}
+template <int F>
+__device__ __forceinline__ float finite_or_plain(float v, const SplitArgs& p, int which, int row, int m) {
+    if constexpr (F == CMLB200_NF4 || F == CMLB200_Q8_0 || F == CMLB200_Q4_0)
+        if (!(fabsf(v) <= 3.402823466e38f) && !p.nw)
+            return plain_dot<F>(which ? p.qs2 : p.qs, which ? p.sc2 : p.sc, p.x + (size_t)m * p.K, p.K, row, p.nf4_shift, p.nf4_units);
+    return v;
+}
+
 // ---- up to 8 rows of x ------------------------------------------------------------------------------------------------------
 constexpr int kWarps = 16;
 template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 ? 2 : Lay<F>::ROW == 144 && NT ? 4 : 3;      // items per warp in flight
@@ -542,10 +572,10 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         }
         const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
         float v = warp_sums<COLS>(src, active);
-        v *= f;
+        v = finite_or_plain<F>(v * f, p, 0, row, m);
         float* out = p.y + (size_t)m * p.N + row;
         if (pairs) {
-            const float v2 = warp_sums<COLS>(src + W * (COLS * 16), active) * f;
+            const float v2 = finite_or_plain<F>(warp_sums<COLS>(src + W * (COLS * 16), active) * f, p, 1, row, m);
             *out = (v / (1.0f + expf(-v))) * v2;
         } else if (p.epi == EPI_ACCUM) *out += v;
         else *out = v;
@@ -765,10 +795,10 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         const int row = ((pairs ? tile0 >> 1 : tile0) + o) * 16 + r;
         if (m >= p.M || row >= p.N) continue;
         const float* src = part + (size_t)(o << pairs) * W * (COLS * 16) + m * 16 + r;
-        const float v = warp_sums<COLS>(src, active);
+        const float v = finite_or_plain<F>(warp_sums<COLS>(src, active), p, 0, row, m);
         float* out = p.y + (size_t)m * p.N + row;
         if (pairs) {
-            const float v2 = warp_sums<COLS>(src + W * (COLS * 16), active);
+            const float v2 = finite_or_plain<F>(warp_sums<COLS>(src + W * (COLS * 16), active), p, 1, row, m);
             *out = (v / (1.0f + expf(-v))) * v2;
         } else if (p.epi == EPI_ACCUM) *out += v;
         else *out = v;

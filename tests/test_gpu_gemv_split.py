@@ -110,6 +110,37 @@ def test_error_against_64_bits(pkg, synth, ob, orc, torch_dev, kind, most, K):
         assert np.sqrt(np.mean(np.square(off))) <= most, (M, off)
 
 
+@pytest.mark.parametrize("kind,batches", [("nf4", (1, 4, 5, 8, 9, 16, 17, 32)), ("q8_0", (9, 32))])
+def test_infinities_and_nan(pkg, synth, ob, orc, torch_dev, kind, batches):
+    """Rows of x that are not finite give what fp32 multiply-adds give: infinities with their signs, NaN where an infinity meets a zero
+    weight or one of the other sign; the rows beside them stay as they are."""
+    rng = np.random.default_rng(9)
+    N, K = 130, 2304
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K)
+    for M in batches:
+        x = rng.standard_normal((M, K)).astype(np.float32)
+        clean = x.copy()
+        bad = sorted({0, M - 1})
+        x[0, 300] = np.inf
+        x[M - 1, 7] = -np.inf
+        if M > 4:
+            x[2, [5, 2000]] = np.inf
+            x[3, 1000] = np.nan
+            bad += [2, 3]
+        d_x, d_y = to_dev(x, torch_dev), torch.empty(M, N, device=torch_dev)
+        pkg.check(pkg.lib.cmlb200_gemv(W.q, d_x.data_ptr(), d_y.data_ptr(), M, stream_ptr()), "gemv")
+        got = d_y.cpu().numpy()
+        with np.errstate(invalid="ignore"):
+            want = (x.astype(np.float64)[:, None, :] * Wf.astype(np.float64)[None]).sum(2)
+        assert np.array_equal(got[bad], want[bad].astype(np.float32), equal_nan=True)
+        rest = [m for m in range(M) if m not in bad]
+        assert np.isfinite(got[rest]).all()
+        if rest:
+            d_c, d_z = to_dev(clean, torch_dev), torch.empty(M, N, device=torch_dev)
+            pkg.check(pkg.lib.cmlb200_gemv(W.q, d_c.data_ptr(), d_z.data_ptr(), M, stream_ptr()), "gemv")
+            assert np.array_equal(got[rest], d_z.cpu().numpy()[rest])
+
+
 def test_streams_keep_their_rows_apart(pkg, synth, ob, orc, torch_dev):
     rng = np.random.default_rng(5)
     W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", 4096, 4096)
