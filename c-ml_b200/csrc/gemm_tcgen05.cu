@@ -33,6 +33,7 @@
 // mbarrier is bounded; on expiry the CTA raises a status flag (cmlb200_gemm_status), waits for its
 // copies and MMAs in flight (each has a barrier of its own), frees its tensor memory and returns.
 #include <cuda.h>
+#include <mutex>
 #include <type_traits>
 #include "common.cuh"
 
@@ -561,19 +562,49 @@ int get_encoder(EncodeTiledFn* out) {
 // A call's shape: tiles of 128 weight rows by NX activation rows, the K of a tile shared by `ranks` CTAs
 struct Shape { int NX, ranks; };
 
-// Estimated time (us) of a shape, fitted to 4096x4096, 11008x4096, 4096x11008, 32000x4096 and 1024x4096 at M = 40 .. 2048: waves of
-// tiles, each K / 64 / ranks slabs of `expand` us for the weights and 0.115 for every 256 activation rows, 2.5 us to fill the
-// pipeline and the epilogue; a cluster's sum takes a few us more (NX = 80: 15.0 us with four ranks, 19.1 with two, 27.1 without, 4096x4096). A cluster lies in one
-// GPC (18 SMs, eight of them, counted as seven), so fewer fit than the SMs would hold: 1024x4096 at M = 40 takes 11.3 us as 8 clusters
-// of 8 CTAs and 20.9 as 16 of them
-inline double shape_cost(const Shape& s, int M, int N, int KB, int sms, double expand) {
-    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN), at_once = s.ranks == 1 ? sms : s.ranks > 6 ? sms / 16 : 7 * (sms / 8 / s.ranks);
-    if (s.ranks > 1 && (tiles > at_once || s.NX > B_ROWS)) return 1e30;
-    const double slab = expand + 0.115 * s.NX / 256;
-    const int waves = (tiles + at_once - 1) / at_once;
-    return waves * (((KB + s.ranks - 1) / s.ranks) * slab + 2.5 + 0.006 * s.NX) + (s.ranks > 1 ? 3.2 + 0.02 * s.NX + 0.13 * s.ranks : 0.0);
+// How many clusters of each size run at once, one CTA an SM: a cluster lies in one GPC, and how many SMs those have is the device's
+// own affair. B200: 74 clusters of two, 45, 33, 26, 22, 15, 15 of eight.
+template <typename Kern>
+const int* clusters_at_once(Kern kern, size_t smem) {
+    static int counts[kMaxDevices][9] = {};
+    static std::mutex mutex;
+    std::lock_guard<std::mutex> lock(mutex);
+    int* c = counts[cmlb_device_index()];
+    if (c[1]) return c;
+    const int sms = cmlb_num_sms();
+    for (int ranks = 8; ranks >= 1; ranks--) {                          // (c[1] last)
+        int n = 0;
+        if (ranks == 1) n = sms;
+        else {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(ranks);
+            cfg.blockDim = dim3(THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = ranks;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        }
+        c[ranks] = n;
+    }
+    return c;
 }
-inline Shape pick_shape(int M, int N, int KB, int sms, double expand) {
+
+// Estimated time (us) of a shape: waves of tiles, each K / 64 / ranks slabs of `expand` us for the weights and 0.14 for every 256
+// activation rows, a few us to fill the pipeline and for the epilogue, and for a cluster's sum. Fitted to all shapes of 504 calls (three
+// formats, 640 to 32000 weight rows, 1024 to 14336 columns, 33 to 2048 rows of x): 7 % rms, the shape picked is 0.3 % off the
+// best one on average. 4096x4096, Q4_0, 77 rows: 14.2 us with four ranks (32 of the 33 clusters that fit), 16.0 with three, 27.1 without.
+inline double shape_cost(const Shape& s, int M, int N, int KB, const int* at_once, double expand) {
+    if (!at_once[s.ranks] || (s.ranks > 1 && s.NX > B_ROWS)) return 1e30;
+    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN);
+    const double slab = expand + 0.14 * s.NX / 256;
+    const int waves = (tiles + at_once[s.ranks] - 1) / at_once[s.ranks];
+    return waves * (((KB + s.ranks - 1) / s.ranks) * slab + 3.7 + 0.008 * s.NX + (s.ranks > 1 ? 1.5 + 0.014 * s.NX + 0.25 * s.ranks : 0.0));
+}
+inline Shape pick_shape(int M, int N, int KB, const int* at_once, double expand) {
     Shape best = {16, 1};
     double least = 1e300;
     const int tm0 = (M + 511) / 512, tm1 = (M + 255) / 256;
@@ -581,7 +612,7 @@ inline Shape pick_shape(int M, int N, int KB, int sms, double expand) {
         for (int ranks = 1; ranks <= 8; ranks++) {
             if (ranks > 1 && KB < 2 * ranks) continue;
             const Shape s = {((M + tm - 1) / tm + 15) / 16 * 16, ranks};
-            const double c = shape_cost(s, M, N, KB, sms, expand);
+            const double c = shape_cost(s, M, N, KB, at_once, expand);
             if (c < least) { least = c; best = s; }
         }
     return best;
@@ -641,7 +672,11 @@ int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16
 template <int TYPE>
 int launch_gemm(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, int splits, cudaStream_t st) {
     const int KB = (W->cols + BK - 1) / BK;
-    Shape s = pick_shape(M, W->rows, KB, cmlb_num_sms(), TYPE == CMLB200_Q8_0 ? 0.63 : TYPE == CMLB200_NF4 ? 0.54 : 0.37);
+    auto kern = gemm_kernel<TYPE, false>;
+    static size_t attr[kMaxDevices] = {};
+    const size_t smem = Cfg<TYPE, false>::total + 1024;
+    CMLB_CUDA(cmlb_ensure_smem(kern, smem, attr));
+    Shape s = pick_shape(M, W->rows, KB, clusters_at_once(kern, smem), TYPE == CMLB200_Q8_0 ? 0.53 : TYPE == CMLB200_NF4 ? 0.47 : 0.32);
     if (splits > 0) {                                                    // the caller's choice, as far as a cluster and the slabs go
         const int tm = (M + 255) / 256;
         s.NX = ((M + tm - 1) / tm + 15) / 16 * 16;
