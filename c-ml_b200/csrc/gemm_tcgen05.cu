@@ -190,19 +190,25 @@ __device__ __forceinline__ uint32_t bf162_sub(uint32_t a, uint32_t b) {
 template <int TYPE>
 __device__ __forceinline__ void expand32(const uint4* raw, float scale, uint4 (&out)[4]) {
     if (TYPE == CMLB200_Q8_0) {
+        // (2^15 + q + 128) scale - (2^15 + 128) scale: the second product is exact (20 bits), so the difference is q scale, which is
+        // exact too (19 bits)
+        const float offset = -32896.0f * scale;
         const uint32_t w[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
+        auto each = [&](auto value) {
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            uint32_t o[4];
+            for (int c = 0; c < 4; c++) {
+                uint32_t o[4];
 #pragma unroll
-            for (int p = 0; p < 4; p++) {                // 2^23 + (q + 128) as fp32 has the byte for its last mantissa bits
-                const uint32_t u = w[2 * c + (p >> 1)] ^ 0x80808080u;
-                const float a = (__uint_as_float(__byte_perm(u, 0x4b000000u, p & 1 ? 0x7442 : 0x7440)) - 8388736.0f) * scale;
-                const float b = (__uint_as_float(__byte_perm(u, 0x4b000000u, p & 1 ? 0x7443 : 0x7441)) - 8388736.0f) * scale;
-                o[p] = pack_bf16(a, b);
+                for (int p = 0; p < 4; p++) {            // 2^15 + (q + 128) as fp32 has the byte in its mantissa
+                    const uint32_t u = w[2 * c + (p >> 1)] ^ 0x80808080u;
+                    o[p] = pack_bf16(value(__uint_as_float(__byte_perm(u, 0x47000000u, p & 1 ? 0x7424 : 0x7404))),
+                                     value(__uint_as_float(__byte_perm(u, 0x47000000u, p & 1 ? 0x7434 : 0x7414))));
+                }
+                out[c] = make_uint4(o[0], o[1], o[2], o[3]);
             }
-            out[c] = make_uint4(o[0], o[1], o[2], o[3]);
-        }
+        };
+        if (fabsf(scale) <= 65504.0f) each([&](float v) { return fmaf(v, scale, offset); });
+        else each([&](float v) { return (v - 32896.0f) * scale; });      // infinite weights
     } else if (TYPE == CMLB200_NF4) {
         // word i = bytes 4i..4i+3 = elements 8i..8i+7, the even one in the high nibble. Low and high bytes of the 16 code values
         // as bf16, four to a word; a permute looks up eight entries, a second one picks by the index's top bit

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 from conftest import rel_err_inf
-from gpu_util import gemm_status, make_weight, stream_ptr, to_dev
+from gpu_util import DevQMat, gemm_status, make_weight, stream_ptr, to_dev
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-2
@@ -157,6 +157,31 @@ def test_gemm_output_modes(pkg, synth, ob, orc, torch_dev, M):
     assert pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, 3, buf.data_ptr(), None, stream_ptr()) == -1      # SwiGLU needs the gate
     assert pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, 7, buf.data_ptr(), None, stream_ptr()) == -1
 
+
+
+def test_gemm_q8_0_weights_are_rounded_once(pkg, synth, torch_dev):
+    """Unit vectors through a Q8_0 weight with every quant and scales from the smallest to the largest finite half: outputs are the
+    products, each rounded to bf16 once. An infinite scale stands for infinite weights."""
+    K = N = 256
+    scales = np.array([0x0400, 0x0001, 0x3c00, 0x1234, 0x7bff, 0x2e66, 0xbc01, 0x0000], np.uint16)
+    blocks = np.zeros((N, K // 32, 34), np.uint8)
+    for n in range(N):
+        for b in range(K // 32):
+            blocks[n, b, :2] = np.frombuffer(scales[(n + b) % 8].tobytes(), np.uint8)
+            blocks[n, b, 2:] = (np.arange(32) + 32 * ((n // 8 + b) % 8)).astype(np.uint8)
+    W = DevQMat.from_gguf(pkg, torch_dev, pkg.Q8_0, blocks.reshape(-1), N, K)
+    s = scales.view(np.float16).astype(np.float32)
+    s[1] *= 0.5                                              # C-ML's reading of a subnormal half
+    q = blocks[:, :, 2:].view(np.int8).astype(np.float32)
+    w = (q * s[(np.arange(N)[:, None] + np.arange(K // 32)[None]) % 8][:, :, None]).reshape(N, K)
+    got = _gemm(pkg, synth, W, np.eye(K, dtype=np.float32), N, torch_dev)
+    want = synth.bf16_to_f32(synth.bf16_round(np.ascontiguousarray(w.T))[0].reshape(K, N))
+    assert np.array_equal(got, want)
+    blocks[5, 3, :2] = (0x00, 0x7c)
+    blocks[5, 3, 2:] = np.arange(1, 33)
+    W = DevQMat.from_gguf(pkg, torch_dev, pkg.Q8_0, blocks.reshape(-1), N, K)
+    got = _gemm(pkg, synth, W, np.ones((2, K), np.float32), N, torch_dev)
+    assert (got[:, 5] == np.inf).all() and np.isfinite(np.delete(got, 5, 1)).all()
 
 
 @pytest.fixture(scope="module")
