@@ -325,8 +325,7 @@ int cmlb200_x_digits_(const float* x, int M, int K, uint32_t* xq, cudaStream_t s
 // norm_w first when that is not NULL.
 int cmlb200_gemv_dp4a_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps,
                        const uint32_t* xq, float* y, int M, int epi, cudaStream_t st) {
-    // three rows (the 4-row kernel would need two launches or pad), and Q8_0 from three on: as in gemv.cu
-    if (!xq && M > 2 && (M == 3 || W->type == CMLB200_Q8_0) && cmlb200_gemv_split_ok_(W, W2)) return cmlb200_gemv_split_(W, W2, x, norm_w, eps, y, M, epi, st);
+    if (!xq && cmlb200_gemv_split_faster_(W, W2, M, epi)) return cmlb200_gemv_split_(W, W2, x, norm_w, eps, y, M, epi, st);
     // more rows of x than one launch of the 4-row kernel takes for this shape: the 8-row kernel streams the weight once
     if (!xq && M > 2 && M <= 8 && (M > 4 || cmlb200_gemv_mma_rows_(W, W2, epi) < M) && cmlb200_gemv_mma8_ok_(W, W2, epi)) return cmlb200_gemv_mma8_(W, W2, x, norm_w, eps, y, M, epi, st);
     if (cmlb200_gemv_mma_ok_(W, W2, epi)) return cmlb200_gemv_mma_(W, W2, xq ? nullptr : x, norm_w, eps, xq, y, M, epi, st);

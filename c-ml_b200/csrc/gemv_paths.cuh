@@ -25,6 +25,9 @@ bool cmlb200_gemv_split_ok_(const cmlb200_qmat* W, const cmlb200_qmat* W2);
 int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const float* x, const uint16_t* norm_w, float eps, float* y, int M, int epi,
                         cudaStream_t st);
 
+// gemv.cu: whether they are the faster ones for so many rows of x
+bool cmlb200_gemv_split_faster_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M, int epi);
+
 // gemv_kquant.cu: Q4_1 / Q4_K / Q5_K / Q6_K weights straight from the GGUF block stream
 bool cmlb200_is_kquant_type_(int type);
 int cmlb200_gemv_kquant_(const cmlb200_qmat* W, const float* x, float* y, int M, int accumulate, cudaStream_t st);

@@ -48,3 +48,13 @@ def test_misaligned_quants_of_the_second_weight_are_refused(pkg):
     assert pkg.lib.cmlb200_gemv_swiglu(gate, up, 5 * BASE, 6 * BASE, 1, None) == -1
     assert pkg.lib.cmlb200_gemv_rmsnorm(gate, up, 5 * BASE, 7 * BASE, 1e-5, 6 * BASE, 1, 2, None) == -1
     assert b"aligned" in pkg.lib.cmlb200_last_error()
+
+
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("rows,cols", [(4096, 1024), (12288, 4096), (4096, 11008), (32000, 4096), (2048, 8192)])
+@pytest.mark.parametrize("M", range(1, 9))
+def test_normalised_rows_go_where_plain_rows_go(pkg, kind, rows, cols, M):
+    """One rule for both entry points (the sources of gemv_dp4a.cu hold the launches of both its kernels and no other)."""
+    W = pair(pkg, kind, rows, cols)[0]
+    plain = route(pkg, lambda: pkg.lib.cmlb200_gemv(W, 5 * BASE, 6 * BASE, M, None))
+    assert route(pkg, lambda: pkg.lib.cmlb200_gemv_rmsnorm(W, None, 5 * BASE, 7 * BASE, 1e-5, 6 * BASE, M, 0, None)) == plain
