@@ -9,7 +9,8 @@
 // sub-block costs 24 dp4a per row of x; the fp16 / 6-bit / int8 scales, minima and offsets of the
 // formats are applied once per sub-block in fp32. Q4_K / Q5_K follow C-ML's own nibble order (each
 // 32-element sub-block in 16 consecutive bytes, src/core/gguf_quant.c:174-187), not ggml's.
-// Left with columns that are no whole 256 and very long rows: the fp16-split kernels (gemv_split.cuh) take the others.
+// Left with columns that are no whole 256, with 131,072 columns and more, and with one row of x where columns are few (Q5_K: at
+// one row always): the fp16-split kernels (gemv_split.cuh) take the others (cmlb200_gemv_split_faster_).
 #include "common.cuh"
 #include "gemv_paths.cuh"
 

@@ -21,8 +21,9 @@
 //
 // What bounds it: instructions. 50 a block of 16 x 32 weights at M = 1 (10 to unpack, 6 to address and load, 2 products, 8 to apply the
 // scales, the rest the rows of x), 65 a warp and block at M = 32, at an issue rate of 0.42 to 0.66 a scheduler; tensor pipe 41 % busy
-// at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers) beat eight with 255: 8.2
-// against 10.4 us at M = 1, 16.1 against 14.7 at M = 32 but 9.9 against 11.4 at M = 16 (Q4_0 11008x4096, 4096x4096). More chains of
+// at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers) beat eight with 255 up to
+// 16 rows: 8.2 against 10.4 us at M = 1 (Q4_0 11008x4096), 9.9 against 11.4 at M = 16 (4096x4096). At M = 32 eight were the faster
+// ones (14.7 against 16.1 us, 4096x4096); that form is not built. More chains of
 // products (the block's halves apart) cost more additions than they hid: 14.3 against 12.9 us at M = 8. Times: gemv.cu.
 #pragma once
 #include "common.cuh"

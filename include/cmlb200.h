@@ -207,7 +207,7 @@ int cmlb200_gemm_bf16(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t*
 int cmlb200_gemm_bf16_ex(const cmlb200_qmat* W, const uint16_t* d_x_bf16, int M, int mode, void* d_out, const uint16_t* d_gate_bf16,
                          void* stream);
 /* Same, with the number of K splits chosen by the caller (1 = none): a cluster of the largest power of two CTAs up to
- * `splits`, 8 and half the 64-wide slabs of K shares a tile; the partial sums meet in distributed shared memory. */
+ * `splits`, 8 and the number of 64-wide slabs of K shares a tile; the partial sums meet in distributed shared memory. */
 int cmlb200_gemm_bf16_splitk(const cmlb200_qmat* W, const uint16_t* d_x_bf16, uint16_t* d_y_bf16, int M,
                              int splits, void* stream);
 /* Synchronises the device and reports whether a bounded wait inside the tensor-core kernel
