@@ -260,7 +260,8 @@ __device__ __forceinline__ void expand32(const uint4* raw, float scale, uint4 (&
 //                                                            src/nn/llama.c:126-155; gate may be the output array)
 enum { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_ACC_F32 = 2, GEMM_SWIGLU_BF16 = 3 };
 // CNT finished values of one weight row (neighbouring activation rows; `count` of them exist), `at` the first one's place. What
-// they are multiplied with is loaded first, so that the loads are in flight together; what they are added to is not loaded at all.
+// they are multiplied with or added to is loaded first, so that the loads are in flight together. (Reductions in global memory,
+// which load nothing, make zeros of sums below 2^-126.)
 template <int CNT>
 __device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int mode, size_t at, int N, int count, const float (&v)[CNT]) {
     if (mode == GEMM_SWIGLU_BF16) {
@@ -279,14 +280,23 @@ __device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int
 #pragma unroll
         for (int j = 0; j < CNT; j++, o += N)
             if (j < count) *o = __float2bfloat16_rn(v[j]);
+    } else if (mode == GEMM_ACC_F32) {
+        float* o = static_cast<float*>(out) + at;
+#pragma unroll
+        for (int k = 0; k < CNT; k += 8) {                           // eight loads in flight: sixteen spill more registers
+            float h[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (k + j < count) h[j] = o[(size_t)j * N];
+#pragma unroll
+            for (int j = 0; j < 8; j++, o += N)
+                if (k + j < count) *o = h[j] + v[k + j];
+        }
     } else {
         float* o = static_cast<float*>(out) + at;
 #pragma unroll
         for (int j = 0; j < CNT; j++, o += N)
-            if (j < count) {
-                if (mode == GEMM_ACC_F32) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"(v[j]) : "memory");
-                else *o = v[j];
-            }
+            if (j < count) *o = v[j];
     }
 }
 

@@ -159,6 +159,19 @@ def test_gemm_output_modes(pkg, synth, ob, orc, torch_dev, M):
 
 
 
+@pytest.mark.parametrize("M", [48, 200, 300])
+def test_gemm_residual_below_the_normal_range(pkg, synth, ob, orc, torch_dev, M):
+    """A residual of subnormal numbers is added to, not flushed: with a cluster's sum, one tile of rows, and two."""
+    rng = np.random.default_rng(M)
+    N, K = 384, 1024
+    W, _ = make_weight(pkg, synth, ob, orc, torch_dev, rng, "q4_0", N, K)
+    d_x = torch.zeros(M, K, dtype=torch.bfloat16, device=torch_dev)
+    h0 = (rng.standard_normal((M, N)) * 1e-39).astype(np.float32)
+    h = to_dev(h0, torch_dev)
+    pkg.check(pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, 2, h.data_ptr(), None, stream_ptr()), "acc_f32")
+    assert np.array_equal(h.cpu().numpy(), h0) and np.count_nonzero(h0) > 0
+
+
 def test_gemm_q8_0_weights_are_rounded_once(pkg, synth, torch_dev):
     """Unit vectors through a Q8_0 weight with every quant and scales from the smallest to the largest finite half: outputs are the
     products, each rounded to bf16 once. An infinite scale stands for infinite weights."""
