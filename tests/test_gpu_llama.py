@@ -419,6 +419,37 @@ def test_models_with_other_block_types_match_oracle(pkg, tmp_path, torch_dev, gt
         pkg.lib.cml_llama_free(m)
 
 
+# 17 units of 256 columns (one more than the warps of a CTA that share a row), inner and vocabulary rows that end inside a tile of 16
+WIDE = dict(vocab=250, hidden=4352, inter=512, layers=1, heads=34, kv_heads=2, max_seq=64)
+
+
+@pytest.mark.parametrize("gtype", [2, 3, 7, 12, 13, 14])
+def test_normalised_products_of_every_batch_match_oracle(pkg, tmp_path, torch_dev, gtype):
+    """RMS norm within the projections of 1 to 32 rows: Q/K/V and the vocabulary, gate and up as one launch (up to 8 rows) and as two, in
+    each block format; as a prompt's rows, and as one new token for each of several sequences."""
+    rng = np.random.default_rng(950 + gtype)
+    path = tmp_path / f"wide_type{gtype}.gguf"
+    store = build(entry, rng, WIDE, path, qtype=gtype, wscale=0.02)
+    orc = OracleLlama(entry, WIDE, store, qtype=gtype, rope_all_heads=1, mask_absolute=1)
+    tokens = rng.integers(0, WIDE["vocab"], 32).astype(np.int32)
+    want = orc.forward(tokens)                                 # causal: the rows of a shorter prompt are its first rows
+    for M in (1, 3, 4, 5, 8, 9, 16, 17, 32):
+        m = device_model(pkg, WIDE, path, flags=pkg.KV_FP32)
+        try:
+            assert rel_err_inf(dev_forward(pkg, m, tokens[:M]), want[:M]) <= 2e-3
+        finally:
+            pkg.lib.cml_llama_free(m)
+    for B in (4, 8, 12):
+        m = device_model(pkg, WIDE, path, flags=pkg.KV_FP32, max_batch=B)
+        try:
+            for b in range(B):                                 # sequence b holds the first b + 1 tokens; its next one is the prompt's
+                assert pkg.lib.cml_llama_prefill_sequence(m, b, pkg.np_ptr(tokens), b + 1) == 0
+            got = pkg.tensor_to_numpy(pkg.lib.cml_llama_forward_batch(m, pkg.np_ptr(tokens[1:B + 1].copy()), B))
+            assert rel_err_inf(got, want[1:B + 1]) <= 2e-3
+        finally:
+            pkg.lib.cml_llama_free(m)
+
+
 def _greedy_reference_tokens(pkg, path, prompt, n):
     """n greedy tokens of the model at `path` after `prompt`, one cml_llama_forward per token."""
     m = device_model(pkg, TINY, path)
