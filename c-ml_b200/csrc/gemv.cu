@@ -19,8 +19,14 @@
 //         that are no whole 256 and short rows at M = 1: 16 warps share the 256-column units of a row, Q6_K 4608x1536 6.3 | 5.5).
 //         Q8_0 7424x3840: 4 9.3 | 8.7
 //   Q5_K  11008x4096: 1 15.2 | 14.9, 2 15.8 | 23.5, 32 49.8 | 189.5; 1024x4096: 1 4.6 | 5.5
+// Pairs of up to three rows (SwiGLU; two launches of the alternative): not with up to 4,096 columns where a CTA's row tiles would be more
+// than six, for they go in rounds then whose last is short (Q8_0 of two rows and up to 2,048 columns: four). 4096 columns, RMS norm first:
+//   Q8_0 M = 2  2048 rows 7.2 | 10.4, 6144 12.6 | 17.7, 11008 24.5 | 22.7, 14336 35.4 | 30.6, 32000 62.4 | 57.2, 8192x8192 33.9 | 51.2,
+//               5632x2048 11.7 | 9.7; Q4_0 M = 3  6144 11.2 | 13.9, 11008 21.5 | 20.2, 14336 31.6 | 25.7, 8192x8192 30.0 | 31.7
 bool cmlb200_gemv_split_faster_(const cmlb200_qmat* W, const cmlb200_qmat* W2, int M, int epi) {
     if (!cmlb200_gemv_split_ok_(W, W2)) return false;
+    if (W2 && ((W->type == CMLB200_Q8_0 && M == 2) || (W->type == CMLB200_Q4_0 && M == 3)) && W->cols <= 4096 &&
+        (W->rows + 15) / 16 * 2 > (W->type == CMLB200_Q8_0 && W->cols <= 2048 ? 4 : 6) * cmlb_num_sms()) return false;
     switch (W->type) {
         case CMLB200_Q4_0: return M > 8 || M == 3;
         case CMLB200_Q8_0: return M > 4 || M == 3 || (M > 1 && cmlb200_gemv_mma_rows_(W, W2, epi) < M);

@@ -58,3 +58,14 @@ def test_normalised_rows_go_where_plain_rows_go(pkg, kind, rows, cols, M):
     W = pair(pkg, kind, rows, cols)[0]
     plain = route(pkg, lambda: pkg.lib.cmlb200_gemv(W, 5 * BASE, 6 * BASE, M, None))
     assert route(pkg, lambda: pkg.lib.cmlb200_gemv_rmsnorm(W, None, 5 * BASE, 7 * BASE, 1e-5, 6 * BASE, M, 0, None)) == plain
+
+
+@pytest.mark.parametrize("kind,M,rows,cols,split", [
+    ("q8_0", 2, 6144, 4096, True), ("q8_0", 2, 11008, 4096, False), ("q8_0", 2, 8192, 8192, True), ("q8_0", 2, 3072, 2048, True), ("q8_0", 2, 5632, 2048, False),
+    ("q4_0", 3, 6144, 4096, True), ("q4_0", 3, 14336, 4096, False), ("q4_0", 3, 5632, 2048, True), ("q4_0", 3, 4096, 11008, True), ("q8_0", 3, 14336, 4096, True)])
+def test_pairs_of_few_rows_of_x(pkg, kind, M, rows, cols, split):
+    """Pairs with more row tiles than fit one round of CTAs stay with the digit kernels, with and without the norm."""
+    gate, up = pair(pkg, kind, rows, cols)
+    taken = [route(pkg, lambda: pkg.lib.cmlb200_gemv_swiglu(gate, up, 5 * BASE, 6 * BASE, M, None)),
+             route(pkg, lambda: pkg.lib.cmlb200_gemv_rmsnorm(gate, up, 5 * BASE, 7 * BASE, 1e-5, 6 * BASE, M, 2, None))]
+    assert [t == "gemv_split.cuh" for t in taken] == [split, split]
