@@ -38,11 +38,8 @@ __device__ __forceinline__ float out_scale(const cmlb200_attn& a) { return a.out
 // grid = (tiles, heads). tiles[i] = {first row, rows (1..64), sequence slot, position of the first row}.
 // DV: room for value columns. DK: 0, or the padded key size, and then DV is the padded value size. SCORED: scores come from
 // a.scores, so there are neither queries nor keys.
-// Three CTAs an SM where keys and values have 128 columns at most: values have one stage (the next tile's are requested when this
-// one's have been used, and come while its scores are made), keys two.
-// A prompt of 2,000 tokens through four layers of 16 heads: 1,744 us with two stages of both and one CTA an SM, 1,688 so.
 template <int DV, int DK, bool SCORED>
-__global__ void __launch_bounds__(TILE_THREADS, DV <= 128 && DK <= 128 && !SCORED ? 3 : 1)
+__global__ void __launch_bounds__(TILE_THREADS)
 attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int ld, const int4* __restrict__ tiles, __nv_bfloat16* __restrict__ out,
                        int out_ld) {
     extern __shared__ __align__(16) __half sm[];
@@ -67,22 +64,19 @@ attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int 
     const __half* vp = static_cast<const __half*>(a.v_pool) + (size_t)kh * dv;
     const int kstride = a.kv_heads * dk, vstride = a.kv_heads * dv;
 
-    // the keys, or the values, of tile it; a group of copies of its own, empty past the last tile
-    auto load = [&](int it, bool keys) {
-        if (it < ntiles) {
-            const int kt = tile_start(it), n16 = (keys ? dk : dv) >> 3, stride = keys ? kstride : vstride, L = keys ? LK : LV;
-            const __half* src = keys ? kp : vp;
-            __half* dst = keys ? Ks + (it & 1) * KT * LK : Vs + (SCORED ? (it & 1) * KT * LV : 0);
-            for (int row = threadIdx.x >> 3; row < KT; row += TILE_THREADS / 8) {
-                const int key = min(kt + row, p_last);     // rows past the end repeat the last key (masked below)
-                const size_t slot = ((size_t)table[key >> shift] << shift) + (key & (a.block_size - 1));
-                for (int c = threadIdx.x & 7; c < n16; c += 8) cp16(smem_addr(dst + row * L + c * 8), src + slot * stride + c * 8);
-            }
+    auto load = [&](int it) {
+        const int kt = tile_start(it), st = it & 1;
+        const int kc = dk >> 3, vc = dv >> 3;
+        for (int row = threadIdx.x >> 3; row < KT; row += TILE_THREADS / 8) {
+            const int key = min(kt + row, p_last);     // rows past the end repeat the last key (masked below)
+            const size_t slot = ((size_t)table[key >> shift] << shift) + (key & (a.block_size - 1));
+            if (!SCORED)
+                for (int c = threadIdx.x & 7; c < kc; c += 8) cp16(smem_addr(Ks + (st * KT + row) * LK + c * 8), kp + slot * kstride + c * 8);
+            for (int c = threadIdx.x & 7; c < vc; c += 8) cp16(smem_addr(Vs + (st * KT + row) * LV + c * 8), vp + slot * vstride + c * 8);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (!SCORED) load(0, true);
-    load(0, false);
+    load(0);
     if (!SCORED) {
         const float qs = a.scale * kLog2e;
         for (int r = warp; r < QT; r += TILE_THREADS / 32) {
@@ -103,27 +97,27 @@ attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int 
     float m0 = sink, m1 = m0, l0 = 0.f, l1 = 0.f;
     // score of key kt + c from position q: dot - slope (q - kt - c). The part that depends on the column alone
     // is what the accumulators start from; the rest is one constant per row and tile.
-    const float bias0 = slope * (float)(2 * t), bias1 = slope * (float)(2 * t + 1), bias8 = slope * 8.0f;
+    float bias[KT / 8][2];
+#pragma unroll
+    for (int i = 0; i < KT / 8; i++) { bias[i][0] = slope * (float)(i * 8 + 2 * t); bias[i][1] = slope * (float)(i * 8 + 2 * t + 1); }
     const uint32_t q_base = smem_addr(Qs + (warp * 16 + (lane & 15)) * LK + (lane >> 4) * 8);
     const float* scores = SCORED ? a.scores + (((size_t)blockIdx.x * a.heads + h) * QT + r0) * a.scores_ld : nullptr;
 
     for (int it = 0; it < ntiles; it++) {
-        if (SCORED) {
-            load(it + 1, false);
+        if (it + 1 < ntiles) {
+            load(it + 1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
-            load(it + 1, true);                             // in flight: this tile's keys, its values, the next one's keys
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
         const int kt = tile_start(it), st = it & 1;
         // nothing of this tile is in reach of this warp's rows: before all they see, or past the last row
         const bool active = w_first <= w_last && kt <= w_last && (kt + KT - 1 >= w_lo || kt < a.keep);
-        uint32_t pa[KT / 16][4];
         if (active) {
             float s[KT / 8][4];
 #pragma unroll
-            for (int i = 0; i < KT / 8; i++) { s[i][0] = s[i][2] = fmaf(bias8, (float)i, bias0); s[i][1] = s[i][3] = fmaf(bias8, (float)i, bias1); }
+            for (int i = 0; i < KT / 8; i++) { s[i][0] = bias[i][0]; s[i][1] = bias[i][1]; s[i][2] = bias[i][0]; s[i][3] = bias[i][1]; }
             if constexpr (SCORED) {
                 const float* src = scores + kt - k_lo + 2 * t;
 #pragma unroll
@@ -178,6 +172,7 @@ attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int 
 #pragma unroll
                 for (int i = 0; i < DV / 8; i++) { o[i][0] *= c0; o[i][1] *= c0; o[i][2] *= c1; o[i][3] *= c1; }
             }
+            uint32_t pa[KT / 16][4];
 #pragma unroll
             for (int i = 0; i < KT / 8; i++) {
                 const float e0 = ex2(s[i][0] - g0), e1 = ex2(s[i][1] - g0), e2 = ex2(s[i][2] - g1), e3 = ex2(s[i][3] - g1);
@@ -186,13 +181,7 @@ attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int 
                 pa[i >> 1][(i & 1) * 2] = pack_h2(e0, e1);
                 pa[i >> 1][(i & 1) * 2 + 1] = pack_h2(e2, e3);
             }
-        }
-        if (!SCORED) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncthreads();
-        }
-        if (active) {
-            const uint32_t v_base = smem_addr(Vs + ((SCORED ? st * KT : 0) + (lane & 15)) * LV + (lane >> 4) * 8);
+            const uint32_t v_base = smem_addr(Vs + (st * KT + (lane & 15)) * LV + (lane >> 4) * 8);
 #pragma unroll
             for (int j = 0; j < KT / 16; j++) {
 #pragma unroll
@@ -207,7 +196,6 @@ attention_tiles_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int 
             }
         }
         __syncthreads();                                // this stage may be refilled
-        if (!SCORED) load(it + 1, false);
     }
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
@@ -605,7 +593,7 @@ extern "C" int cmlb200_attention_tiles(const cmlb200_attn* a, const float* d_qkv
     CMLB_REQUIRE(((uintptr_t)d_tiles & 15) == 0, "cmlb200_attention_tiles: the tile list must be 16-byte aligned");
     const bool scored = a->scores != nullptr;
     CMLB_REQUIRE(!scored || (a->scores_ld % 64 == 0 && ((uintptr_t)a->scores & 15) == 0), "cmlb200_attention_tiles: score stride %d", a->scores_ld);
-    const size_t smem = 2 * ((scored ? 0 : (size_t)(QT + 2 * KT) * (a->dim_ld + 8)) + (size_t)(scored ? 2 : 1) * KT * (a->vdim_ld + 8));
+    const size_t smem = 2 * ((scored ? 0 : (size_t)(QT + 2 * KT) * (a->dim_ld + 8)) + (size_t)2 * KT * (a->vdim_ld + 8));
     CMLB_REQUIRE(smem <= 227 * 1024, "cmlb200_attention_tiles: head sizes %d / %d do not fit shared memory", a->dim, a->vdim);
     cudaStream_t st = as_stream(stream);
     const dim3 grid(tiles, a->heads);
