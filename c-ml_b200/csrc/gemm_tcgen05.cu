@@ -27,7 +27,7 @@
 //   Q4_0  a byte permute drops two nibbles into the mantissas of two bf16 halves (0x43nn = 128 + n), one packed subtract gives
 //         n - 8 exactly, one packed multiply applies the block scale
 //   NF4   the two bytes of a code value by byte permutes over a table of 16 in registers, one packed multiply by the block scale
-//   Q8_0  convert, multiply in fp32, round once
+//   Q8_0  a byte permuted into an fp32 mantissa, one multiply-add, rounded once
 // Q4_0 and NF4 therefore round twice (scale or code value to bf16, then the product); the path's
 // tolerance is 1e-2 of the largest output. No cluster multicast is used. Every wait on an
 // mbarrier is bounded; on expiry the CTA raises a status flag (cmlb200_gemm_status), waits for its
