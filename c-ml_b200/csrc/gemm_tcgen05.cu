@@ -54,18 +54,18 @@ constexpr int AHEAD = 3;                        // slabs whose packed weights a 
 constexpr uint32_t SPIN_LIMIT = CML_GEMM_SPIN_LIMIT;
 constexpr uint32_t DRAIN_LIMIT = 1u << 22;
 
-// A group always comes back to the same stages, so a parity wait is never two phases from its barrier.
-// WIDE (NX > 256): activations come in boxes of 256 rows of a ring of their own, two a slab; otherwise a stage holds both operands.
-template <int TYPE, bool WIDE> struct Cfg {
+// A group always comes back to the same stages, so a parity wait is never two phases from its barrier. A stage holds both operands of a
+// slab. PAIR: two boxes of activations, of which a CTA holds half the rows each.
+template <int TYPE, bool PAIR> struct Cfg {
     static constexpr int RAWB = (TYPE == CMLB200_Q8_0) ? 64 : 32;       // packed bytes per row and slab
     static constexpr int GROUPS = 2, GROUP_WARPS = DQ_WARPS / GROUPS;
-    static constexpr int STAGES = 4;                                    // expanded weights
-    static constexpr int BSTAGES = WIDE ? 5 : STAGES;                   // boxes of activations
+    static constexpr int STAGES = 4, BOXES = PAIR ? 2 : 1;
+    static constexpr int BOX_BYTES = PAIR ? B_BYTES / 2 : B_BYTES;
     // offsets from the 1024-byte aligned base
     static constexpr int a_off = 0;
     static constexpr int b_off = STAGES * A_BYTES;
-    static constexpr int bar_off = b_off + BSTAGES * B_BYTES;
-    static constexpr int nbars = 2 * STAGES + 2 * BSTAGES + 2;
+    static constexpr int bar_off = b_off + STAGES * B_BYTES;
+    static constexpr int nbars = 3 * STAGES + 2;
     static constexpr int total = bar_off + 8 * nbars + 32;
     static_assert(total + 1024 <= 227 * 1024, "the stages do not fit shared memory");
 };
@@ -151,14 +151,31 @@ __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
     return d;
 }
 
+// PAIR: for both CTAs of a pair, from the first one's issuing lane; a commit arrives at the barrier of either
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
+    if (PAIR)
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
+    else
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
 }
+template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    if (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// Arrives at the same barrier of the pair's first CTA. What the arrival stands for lies in this SM's own memory, which its half of the
+// MMA reads: released for the CTA. (A release for the cluster holds the warp up for 1,400 cycles, and a slab with it.)
+__device__ __forceinline__ void mbar_arrive_first(uint32_t bar) {
+    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %0, 0;\n mbarrier.arrive.shared::cluster.b64 _, [a];\n}\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&f)[16]) {
     uint32_t r[16];
@@ -314,18 +331,17 @@ struct GemmArgs {
     int mode, M, N, K, NX, tiles_m, tiles, nf4_block, nf4_shift;
 };
 
-template <int TYPE, bool WIDE>
+template <int TYPE, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
-    using C = Cfg<TYPE, WIDE>;
-    constexpr int STAGES = C::STAGES, BST = C::BSTAGES, RAWB = C::RAWB;
+    using C = Cfg<TYPE, PAIR>;
+    constexpr int STAGES = C::STAGES, RAWB = C::RAWB;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem), bars = sbase + C::bar_off;
-    auto full_a = [&](int s) { return bars + 8 * s; };
-    auto empty_a = [&](int s) { return bars + 8 * (STAGES + s); };
-    auto full_b = [&](int s) { return bars + 8 * (2 * STAGES + s); };
-    auto empty_b = [&](int s) { return bars + 8 * (2 * STAGES + BST + s); };
+    auto full_a = [&](int s) { return bars + 8 * s; };               // (a pair's first CTA: and all that the second one has for the slab)
+    auto full_b = [&](int s) { return bars + 8 * (STAGES + s); };
+    auto empty = [&](int s) { return bars + 8 * (2 * STAGES + s); };
     const uint32_t done_bar = bars + 8 * (C::nbars - 2), free_bar = bars + 8 * (C::nbars - 1);      // accumulators finished / read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::bar_off + 8 * C::nbars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::bar_off + 8 * C::nbars + 8);
@@ -337,28 +353,37 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
     uint32_t rank, ranks;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    // a pair has 256 weight rows of a tile, 128 in either CTA, and either holds half of the activations that both multiply with
+    const int second = PAIR ? (int)rank : 0, BM = PAIR ? 2 * BN : BN;
     const int first_tile = blockIdx.x / ranks, step = gridDim.x / ranks;
+    if (PAIR) { rank = 0; ranks = 1; }
     const int kb0 = KB * rank / ranks, kb1 = KB * (rank + 1) / ranks, nkb = kb1 - kb0;
     const int my_tiles = first_tile < p.tiles ? (p.tiles - first_tile + step - 1) / step : 0, slabs = my_tiles * nkb;
     uint32_t tmem_cols = 32;
     while ((int)tmem_cols < p.NX) tmem_cols <<= 1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), C::GROUP_WARPS); mbar_init(empty_a(s), 1); }
-        for (int s = 0; s < BST; s++) { mbar_init(full_b(s), 1); mbar_init(empty_b(s), 1); }
+        for (int s = 0; s < STAGES; s++) { mbar_init(full_a(s), C::GROUP_WARPS + (PAIR && !second ? 1 : 0)); mbar_init(full_b(s), 1); mbar_init(empty(s), 1); }
         mbar_init(done_bar, 1);
-        mbar_init(free_bar, DQ_WARPS);
+        mbar_init(free_bar, PAIR ? 2 * DQ_WARPS : DQ_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");      // its barriers and columns, too
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
@@ -366,68 +391,64 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         // ---------------- TMA producer: activation slabs (operand B) ----------------
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            // not WIDE: a stage's box and expanded weights are free together; counters instead of divisions
-            const int boxes = WIDE ? 2 : 1, total = slabs * boxes;
-            int bi = 0, s = 0, kb = kb0, tile = first_tile, upper = 0;
+            int it = 0, s = 0, kb = kb0, tile = first_tile;              // counters instead of divisions
             uint32_t phase = 1;
-            for (; bi < total; bi++) {
-                const uint32_t bar = full_b(s);
-                if (!mbar_wait(WIDE ? empty_b(s) : empty_a(s), phase, abort_flag, 1)) break;
+            for (; it < slabs; it++) {
+                const uint32_t bar = full_b(s), to = sbase + C::b_off + s * B_BYTES;
+                const int y = (tile % p.tiles_m) * p.NX;
+                if (!mbar_wait(empty(s), phase, abort_flag, 1)) break;
                 mbar_expect_tx(bar, (uint32_t)n_lo * BK * 2);
-                tma_load_2d(sbase + C::b_off + s * B_BYTES, &xmap, kb * BK, (tile % p.tiles_m) * p.NX + upper * B_ROWS, bar);
-                if (++s == BST) { s = 0; phase ^= 1; }
-                if (WIDE) upper ^= 1;
-                if (upper == 0 && ++kb == kb1) { kb = kb0; tile += step; }
+                if (PAIR) {
+                    tma_load_2d(to, &xmap, kb * BK, y + second * (n_lo / 2), bar);
+                    tma_load_2d(to + C::BOX_BYTES, &xmap, kb * BK, y + B_ROWS + second * (n_hi / 2), bar);
+                } else tma_load_2d(to, &xmap, kb * BK, y, bar);
+                if (++s == STAGES) { s = 0; phase ^= 1; }
+                if (++kb == kb1) { kb = kb0; tile += step; }
             }
-            for (int i = max(0, bi - BST); i < bi; i++) mbar_drain(full_b(i % BST), (i / BST) & 1);   // no copy outlives its CTA
+            for (int i = max(0, it - STAGES); i < it; i++) mbar_drain(full_b(i % STAGES), (i / STAGES) & 1);      // no copy outlives its CTA
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: the warp stays converged, an elected lane issues ----
-        const uint32_t ibase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 4) << 24);
+        const uint32_t ibase = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);
         const uint32_t idesc = ibase | ((uint32_t)(n_lo >> 3) << 17), idesc_hi = ibase | ((uint32_t)(n_hi >> 3) << 17);
         bool ok = true;
-        int s = 0, sb = 0, seg = 0;
-        uint32_t phase = 0, phase_b = 0;
+        int s = 0, seg = 0;
+        uint32_t phase = 0;
+        // (the boxes first: they are there earlier, so their wait hides behind the expansion's)
+        auto slab_there = [&]() { return warp_wait(full_b(s), phase, abort_flag, 4) && warp_wait(full_a(s), phase, abort_flag, 3); };
+        if (PAIR && second) {                                              // tells the first CTA what has come to this one
+            for (int it = 0; it < slabs && ok; it++) {
+                ok = slab_there();
+                if (ok && lane == 0) mbar_arrive_first(full_a(s));
+                __syncwarp();
+                if (++s == STAGES) { s = 0; phase ^= 1; }
+            }
+            seg = my_tiles;
+        }
+        const bool issues = !(PAIR && second);
         for (; seg < my_tiles && ok; seg++) {
             if (seg) ok = warp_wait(free_bar, (seg - 1) & 1, abort_flag, 7);
             for (int i = 0; i < nkb && ok; i++) {
-                // (the box first: it is there earlier, so its wait hides behind the expansion's)
-                ok = (WIDE || warp_wait(full_b(s), phase, abort_flag, 4)) && warp_wait(full_a(s), phase, abort_flag, 3);
+                ok = slab_there();
                 if (!ok) break;
-                const uint64_t adesc = make_desc_sw128(sbase + C::a_off + s * A_BYTES);
-                auto half = [&](int b, uint32_t acc, uint32_t id) {
-                    const uint64_t bdesc = make_desc_sw128(sbase + C::b_off + b * B_BYTES);
+                const uint64_t adesc = make_desc_sw128(sbase + C::a_off + s * A_BYTES), bdesc = make_desc_sw128(sbase + C::b_off + s * B_BYTES);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < BK / 16; kk++)               // 32 bytes inside the swizzle row per K=16 step
-                        umma_f16(acc, adesc + (uint64_t)(2 * kk), bdesc + (uint64_t)(2 * kk), id, (i | kk) ? 1u : 0u);
-                };
-                if (WIDE) {
+                    for (int box = 0; box < C::BOXES; box++)
 #pragma unroll
-                    for (int upper = 0; upper < 2; upper++) {
-                        ok = ok && warp_wait(full_b(sb), phase_b, abort_flag, 4);
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (ok && elect_one()) {
-                            half(sb, tmem_base + (uint32_t)(upper * B_ROWS), upper ? idesc_hi : idesc);
-                            umma_commit(empty_b(sb));
-                            if (upper) umma_commit(empty_a(s));
-                        }
-                        __syncwarp();
-                        if (++sb == BST) { sb = 0; phase_b ^= 1; }
-                    }
-                } else {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (elect_one()) {
-                        half(s, tmem_base, idesc);
-                        umma_commit(empty_a(s));
-                    }
-                    __syncwarp();
+                        for (int kk = 0; kk < BK / 16; kk++)               // 32 bytes inside the swizzle row per K=16 step
+                            umma_f16<PAIR>(tmem_base + (uint32_t)(box * B_ROWS), adesc + (uint64_t)(2 * kk), bdesc + (uint64_t)(box * (C::BOX_BYTES >> 4) + 2 * kk),
+                                           box ? idesc_hi : idesc, (i | kk) ? 1u : 0u);
+                    umma_commit<PAIR>(empty(s));
                 }
+                __syncwarp();
                 if (++s == STAGES) { s = 0; phase ^= 1; }
             }
-            if (elect_one()) umma_commit(done_bar);      // arrives once every MMA issued so far has retired
+            if (elect_one()) umma_commit<PAIR>(done_bar);      // arrives once every MMA issued so far has retired
             __syncwarp();
         }
-        if (!ok && seg > 0) mbar_drain(done_bar, (seg - 1) & 1);          // tensor memory and the stages outlive the MMAs
+        if (issues && !ok && seg > 0) mbar_drain(done_bar, (seg - 1) & 1);          // tensor memory and the stages outlive the MMAs
     } else {
         // ---------------- weight expansion (operand A), then epilogue ----------------
         const int dqw = warp - 2, grp = dqw / C::GROUP_WARPS, tg = (dqw % C::GROUP_WARPS) * 32 + lane;
@@ -445,7 +466,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         uint32_t fblk = 0;
         auto place = [&]() {
             while (fkb >= kb1) { fkb -= nkb; ftile += step; }
-            fblk = (uint32_t)min(ftile / p.tiles_m * BN + row, p.N - 1) * (uint32_t)row_blocks + 2u * (uint32_t)fkb + (uint32_t)h;
+            fblk = (uint32_t)min(ftile / p.tiles_m * BM + second * BN + row, p.N - 1) * (uint32_t)row_blocks + 2u * (uint32_t)fkb + (uint32_t)h;
         };
         place();
         uint4 raw[AHEAD][RAWB / 32];
@@ -479,7 +500,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
             expand32<TYPE>(r, f, out);                                // (past the end of a row: zeros meet zero-filled activations)
             fetch(r, sc);
             const int s = it % STAGES;
-            ok = warp_wait(empty_a(s), ((it / STAGES) & 1) ^ 1, abort_flag, 5);
+            ok = warp_wait(empty(s), ((it / STAGES) & 1) ^ 1, abort_flag, 5);
             if (!ok) return;
 #pragma unroll
             for (int c = 0; c < 4; c++) *reinterpret_cast<uint4*>(a_row[c] + s * A_BYTES) = out[c];
@@ -494,7 +515,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         float* const own = reinterpret_cast<float*>(smem);           // [NX][128]: this CTA's sums, where the stages were
         int it = grp, slot = 0, ends = 0;                            // this group's next slab, its slot, the slab behind the tile
         for (int seg = 0; seg < my_tiles && ok; seg++) {
-            const int tile = first_tile + seg * step, n0 = tile / p.tiles_m * BN, m0 = (tile % p.tiles_m) * p.NX;
+            const int tile = first_tile + seg * step, n0 = tile / p.tiles_m * BM + second * BN, m0 = (tile % p.tiles_m) * p.NX;
             ends += nkb;
             for (; it < ends && ok; it += C::GROUPS) {
                 if (slot == 0) slab(raw[0], scale[0], it);
@@ -520,7 +541,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(free_bar);
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_first(free_bar);
+                else mbar_arrive(free_bar);
+            }
         }
     }
     if (ranks > 1) {                                                 // one tile, its K over the cluster: CTA r adds and finishes its share of the columns
@@ -552,9 +576,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody reads or arrives there any more
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
 
@@ -576,7 +602,7 @@ int get_encoder(EncodeTiledFn* out) {
 }
 
 // A call's shape: tiles of 128 weight rows by NX activation rows, the K of a tile shared by `ranks` CTAs
-struct Shape { int NX, ranks; };
+struct Shape { int NX, ranks; bool pair; };
 
 // How many clusters of each size run at once, one CTA an SM: a cluster lies in one GPC, and how many SMs those have is the device's
 // own affair. B200: 74 clusters of two, 45, 33, 26, 22, 15, 15 of eight.
@@ -614,34 +640,40 @@ const int* clusters_at_once(Kern kern, size_t smem) {
 // formats, 640 to 32000 weight rows, 1024 to 14336 columns, 33 to 2048 rows of x): 7 % rms, the shape picked is 0.3 % off the
 // best one on average. 4096x4096, Q4_0, 77 rows: 14.2 us with four ranks (32 of the 33 clusters that fit), 16.0 with three, 27.1 without.
 inline double shape_cost(const Shape& s, int M, int N, int KB, const int* at_once, double expand) {
-    if (!at_once[s.ranks] || (s.ranks > 1 && s.NX > B_ROWS)) return 1e30;
-    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + BN - 1) / BN);
+    const int together = s.pair ? 2 : s.ranks, rows = s.pair ? 2 * BN : BN;
+    if (!at_once[together] || (s.ranks > 1 && s.NX > B_ROWS)) return 1e30;
+    const int tiles = ((M + s.NX - 1) / s.NX) * ((N + rows - 1) / rows);
     const double slab = expand + 0.14 * s.NX / 256;
-    const int waves = (tiles + at_once[s.ranks] - 1) / at_once[s.ranks];
+    const int waves = (tiles + at_once[together] - 1) / at_once[together];
     return waves * (((KB + s.ranks - 1) / s.ranks) * slab + 3.7 + 0.008 * s.NX + (s.ranks > 1 ? 1.5 + 0.014 * s.NX + 0.25 * s.ranks : 0.0));
 }
 inline Shape pick_shape(int M, int N, int KB, const int* at_once, double expand) {
-    Shape best = {16, 1};
+    Shape best = {16, 1, false};
     double least = 1e300;
     const int tm0 = (M + 511) / 512, tm1 = (M + 255) / 256;
     for (int tm = tm0; tm <= tm1 + min(tm1 + 1, 8); tm++)
         for (int ranks = 1; ranks <= 8; ranks++) {
             if (ranks > 1 && KB < 2 * ranks) continue;
-            const Shape s = {((M + tm - 1) / tm + 15) / 16 * 16, ranks};
+            Shape s = {((M + tm - 1) / tm + 15) / 16 * 16, ranks, false};
+            if (s.NX > B_ROWS) {
+                if (ranks > 1) continue;
+                s.NX = max((s.NX + 31) / 32 * 32, B_ROWS + 32);            // (a pair's MMA has whole 32 columns)
+                s.pair = true;
+            }
             const double c = shape_cost(s, M, N, KB, at_once, expand);
             if (c < least) { least = c; best = s; }
         }
     return best;
 }
 
-template <int TYPE, bool WIDE>
-int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, const Shape& shape, cudaStream_t st) {
-    using C = Cfg<TYPE, WIDE>;
+template <int TYPE, bool PAIR>
+int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, const Shape& shape, int pairs_at_once, cudaStream_t st) {
+    using C = Cfg<TYPE, PAIR>;
     const int N = W->rows, K = W->cols;
     GemmArgs a = {};
     a.NX = shape.NX;
     a.tiles_m = (M + a.NX - 1) / a.NX;
-    a.tiles = (N + BN - 1) / BN * a.tiles_m;
+    a.tiles = (N + (PAIR ? 2 : 1) * BN - 1) / ((PAIR ? 2 : 1) * BN) * a.tiles_m;
     a.qs = (const uint8_t*)W->qs;
     a.scales = W->scales;
     a.out = y;
@@ -658,18 +690,19 @@ int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16
     CUtensorMap xmap;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)min(a.NX, B_ROWS)};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)min(a.NX, B_ROWS) / (PAIR ? 2 : 1)};
     const cuuint32_t estr[2] = {1, 1};
     CUresult cr = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)x, dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CMLB_REQUIRE(cr == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with %d (x must be 16-byte aligned, K*2 a multiple of 16)", (int)cr);
-    auto kern = gemm_kernel<TYPE, WIDE>;
+    auto kern = gemm_kernel<TYPE, PAIR>;
     static size_t attr[kMaxDevices] = {};
     const size_t smem = C::total + 1024;
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, attr));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(shape.ranks > 1 ? a.tiles * shape.ranks : min(a.tiles, cmlb_num_sms())));
+    const int ranks = PAIR ? 2 : shape.ranks;
+    cfg.gridDim = dim3((unsigned)(PAIR ? 2 * min(a.tiles, pairs_at_once) : ranks > 1 ? a.tiles * ranks : min(a.tiles, cmlb_num_sms())));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -677,7 +710,7 @@ int launch_tiles(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = shape.ranks;
+    at[1].val.clusterDim.x = ranks;
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 2;
@@ -692,14 +725,16 @@ int launch_gemm(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_
     static size_t attr[kMaxDevices] = {};
     const size_t smem = Cfg<TYPE, false>::total + 1024;
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, attr));
-    Shape s = pick_shape(M, W->rows, KB, clusters_at_once(kern, smem), TYPE == CMLB200_Q8_0 ? 0.53 : TYPE == CMLB200_NF4 ? 0.47 : 0.32);
+    const int* at_once = clusters_at_once(kern, smem);
+    Shape s = pick_shape(M, W->rows, KB, at_once, TYPE == CMLB200_Q8_0 ? 0.53 : TYPE == CMLB200_NF4 ? 0.47 : 0.32);
     if (splits > 0) {                                                    // the caller's choice, as far as a cluster and the slabs go
         const int tm = (M + 255) / 256;
         s.NX = ((M + tm - 1) / tm + 15) / 16 * 16;
         s.ranks = 1;
+        s.pair = false;
         while (2 * s.ranks <= splits && 2 * s.ranks <= KB && s.ranks < 8) s.ranks *= 2;
     }
-    return s.NX > B_ROWS ? launch_tiles<TYPE, true>(W, x, y, gate, mode, M, s, st) : launch_tiles<TYPE, false>(W, x, y, gate, mode, M, s, st);
+    return s.pair ? launch_tiles<TYPE, true>(W, x, y, gate, mode, M, s, at_once[2], st) : launch_tiles<TYPE, false>(W, x, y, gate, mode, M, s, 0, st);
 }
 
 int gemm_entry(const cmlb200_qmat* W, const uint16_t* x, void* y, const uint16_t* gate, int mode, int M, int ctas, void* stream) {
