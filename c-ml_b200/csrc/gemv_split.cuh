@@ -403,8 +403,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         }
         cp_async_commit();
     };
-    // weights do not depend on the launch before (NF4 ones may: it may have quantized them)
-    if (F == CMLB200_NF4) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // weights do not depend on the launch before: the kernel that quantizes them on the device ends before its successor begins
 #pragma unroll
     for (int i = 0; i < RING; i++) issue(i);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -616,7 +615,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         if (CG == 1) __syncwarp();
         else asm volatile("bar.sync %0, %1;" ::"r"(share + 1), "n"(32 * CG) : "memory");
     };
-    if (F == CMLB200_NF4) asm volatile("griddepcontrol.wait;" ::: "memory");
     issue(0);
     if (stages > 1) issue(1);
     uint32_t* const tmem = reinterpret_cast<uint32_t*>(smem + p.extra);
