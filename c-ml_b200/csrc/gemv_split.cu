@@ -95,8 +95,7 @@ x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int k = 0; k < 8; k++) { e[k] *= up; s += e[k]; }
-#pragma unroll
-        for (int k = 0; k < 4; k++) split2(e[4 * (k >> 1) + (k & 1)], e[4 * (k >> 1) + (k & 1) + 2], hi[k], lo[k]);
+        split8<CONTIG>(e, hi, lo);
         const int blk = i >> 2, t = i & 3;
         uint4* dst = planes + ((size_t)(blk * NT + j) * 2) * 32 + g * 4 + t;
         dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);

@@ -35,10 +35,13 @@ enum { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2 };
 
 // Shared memory of one weight row's 256-column unit: bytes of quants (and headers) as they lie in memory, block scales
 // behind them. Row strides are odd multiples of 16 bytes (mod 128), so eight rows hit eight bank groups.
+constexpr int kNF4Fine = CMLB200_NF4 + 1;
+template <int F> constexpr bool kNF4Like = F == CMLB200_NF4 || F == kNF4Fine;
 template <int F> struct Lay;
 template <> struct Lay<CMLB200_Q4_0> { static constexpr int ROW = 144, CH = 8, SC = 128; };
 template <> struct Lay<CMLB200_Q8_0> { static constexpr int ROW = 272, CH = 16, SC = 256; };
-template <> struct Lay<CMLB200_NF4> { static constexpr int ROW = 176, CH = 8, SC = 128; };
+template <> struct Lay<CMLB200_NF4> { static constexpr int ROW = 144, CH = 8, SC = 128; };         // blocks of 64 and more
+template <> struct Lay<kNF4Fine> { static constexpr int ROW = 176, CH = 8, SC = 128; };            // of 32: eight scales
 template <> struct Lay<CMLB200_Q4_1> { static constexpr int ROW = 176, CH = 10, SC = 0; };
 template <> struct Lay<CMLB200_Q4_K> { static constexpr int ROW = 144, CH = 9, SC = 0; };
 template <> struct Lay<CMLB200_Q5_K> { static constexpr int ROW = 176, CH = 11, SC = 0; };
@@ -57,6 +60,7 @@ struct SplitArgs {
     float* y;
     float eps;
     int N, K, M, tiles, per_cta, stages, epi;
+    int lut;                       // NF4: where in shared memory the table of codes lies (whole 16 bytes)
     int extra;                     // 9 rows and more: where in shared memory the address of tensor memory and the scalings go
     int nf4_shift;                 // log2 of how many 32-column blocks one NF4 scale covers, 3 at most
     int nf4_units;                 // units one covers, 1 at least
@@ -143,7 +147,7 @@ __device__ __forceinline__ void issue_tile(const SplitArgs& p, const Pieces<F>& 
         }
     } else {
         const int left = nblk - un * 8;                                      // blocks of the unit that exist
-        const int have = F == CMLB200_Q8_0 ? 2 * left : F == CMLB200_Q4_0 || F == CMLB200_NF4 ? left : CH;
+        const int have = F == CMLB200_Q8_0 ? 2 * left : F == CMLB200_Q4_0 || kNF4Like<F> ? left : CH;
 #pragma unroll 1
         for (int c = lane; c < 16 * CH; c += 32) {
             const int r = c / CH, ch = c % CH;
@@ -153,7 +157,7 @@ __device__ __forceinline__ void issue_tile(const SplitArgs& p, const Pieces<F>& 
     }
     if (F == CMLB200_Q4_0 || F == CMLB200_Q8_0) {
         if (lane < 16) cp_async16(dst + lane * ROW + Lay<F>::SC, sc + 2 * ((size_t)min(row0 + lane, last) * nblk + (size_t)un * 8));
-    } else if (F == CMLB200_NF4) {                                          // absmax: one for a few blocks, or for units
+    } else if (kNF4Like<F>) {                                          // absmax: one for a few blocks, or for units
         const int ws = 3 - p.nf4_shift, words = 1 << ws, per_row = (nblk >> p.nf4_shift) / p.nf4_units, first = (un << ws) / p.nf4_units;
         for (int c = lane; c < 16 * words; c += 32) {
             const int r = c >> ws, k = c & (words - 1);
@@ -166,9 +170,9 @@ __device__ __forceinline__ void issue_tile(const SplitArgs& p, const Pieces<F>& 
 
 // ---- weights: ring -> A operands --------------------------------------------------------------------------------------
 // A thread (g, t) = (lane / 4, lane % 4) of the product holds rows g and g + 8. Of a 32-column block it takes columns 4t .. 4t+3
-// and 16+4t .. 16+4t+3 (NF4: 8t .. 8t+7), in the order (0,2) (1,3) (4,6) (5,7) of the eight; the B operands have the same order,
+// and 16+4t .. 16+4t+3 in the order (0,2) (1,3) (4,6) (5,7) of the eight, of NF4 8t .. 8t+7 as they are; the B operands have the same order,
 // and the order of columns inside a product is free. a[0], a[1]: the two m16n8k16 of the block; NF4: two digits of the value.
-template <int F> constexpr int kDigits = F == CMLB200_NF4 ? 2 : 1;
+template <int F> constexpr int kDigits = kNF4Like<F> ? 2 : 1;
 
 // 4-bit formats: word w holds the eight nibbles of one row
 __device__ __forceinline__ void nibbles(uint32_t w, uint32_t magic, uint32_t (&h)[4]) {
@@ -180,7 +184,7 @@ __device__ __forceinline__ void nibbles(uint32_t w, uint32_t magic, uint32_t (&h
 }
 
 template <int F>
-__device__ __forceinline__ void row_regs(Shared at, int b, int t, uint32_t w0, uint32_t w1, uint32_t off, uint32_t (&h)[kDigits<F>][4]) {
+__device__ __forceinline__ void row_regs(Shared at, int b, int t, uint32_t w0, uint32_t w1, uint32_t off, Shared lut, uint32_t (&h)[kDigits<F>][4]) {
     if constexpr (F == CMLB200_Q4_0 || F == CMLB200_Q4_1 || F == CMLB200_Q4_K) {     // q - 8 from 1024 + q and 1024 + 16 q
         uint32_t n[4];
         nibbles(w0, 0x64006400u, n);
@@ -205,35 +209,45 @@ __device__ __forceinline__ void row_regs(Shared at, int b, int t, uint32_t w0, u
     } else if constexpr (F == CMLB200_Q6_K) {                   // q - 32 from 1024 + q
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-            const uint32_t q = lds16(at + off + 16 * b + 8 * k + 2 * t), hb = at[off + 128 + 8 * b + 4 * k + t];
-            const uint32_t w = __byte_perm(q, 0, 0x4140), hh = hb | (hb << 16);
-            const uint32_t e = and_or(w, 0x000f000fu, 0x64006400u), o = and_or(w >> 4, 0x000f000fu, 0x64006400u);
-            h[0][2 * k] = hadd2u(e | ((hh << 4) & 0x00000030u) | (hh & 0x00300000u), 0xe420e420u);              // - 1056
-            h[0][2 * k + 1] = hadd2u(o | ((hh << 2) & 0x00000030u) | ((hh >> 2) & 0x00300000u), 0xe420e420u);
+            // a byte's four pairs of high bits: to the places beside the nibbles by a multiplication, two at a time
+            const uint32_t q = lds16(at + off + 16 * b + 8 * k + 2 * t), hb = at[off + 128 + 8 * b + 4 * k + t], w = __byte_perm(q, 0, 0x4140);
+            h[0][2 * k] = hadd2u(and_or(hb * 0x00010010u, 0x00300030u, and_or(w, 0x000f000fu, 0x64006400u)), 0xe420e420u);              // - 1056
+            h[0][2 * k + 1] = hadd2u(and_or(hb * 0x00004004u, 0x00300030u, and_or(w >> 4, 0x000f000fu, 0x64006400u)), 0xe420e420u);
         }
-    } else {                                                    // NF4: 10000 times the code = 128 a + b, digits by byte table look-ups
-        // a + 128 and b + 128 of the 16 codes (|b| <= 64), four to a word
-        constexpr uint32_t A0 = 0x61574a32u, A1 = 0x8079726au, A2 = 0x9a938d86u, A3 = 0xceb8aca2u;
-        constexpr uint32_t B0 = 0x937d4e70u, B1 = 0x80714864u, B2 = 0xb39d499cu, B3 = 0x90be7ab7u;
+    } else {                                                    // NF4: 10000 times the code = 128 a + b; a byte's two codes from a table
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const uint32_t w = k ? w0 >> 16 : w0;
-            const uint32_t s = w & 0x7777u, pick = and_or(w >> 1, 0x4444u, 0x3210u);
-            const uint32_t va = __byte_perm(__byte_perm(A0, A1, s), __byte_perm(A2, A3, s), pick);
-            const uint32_t vb = __byte_perm(__byte_perm(B0, B1, s), __byte_perm(B2, B3, s), pick);
-            // bytes: columns 1, 0, 3, 2. 1024 + (a + 128) -> a * 2^-7, 1024 + (b + 128) -> b * 2^-14
-            h[0][2 * k] = hfma2u(__byte_perm(va, 0x64646464u, 0x4341), 0x20002000u, 0xc880c880u);
-            h[0][2 * k + 1] = hfma2u(__byte_perm(va, 0x64646464u, 0x4240), 0x20002000u, 0xc880c880u);
-            h[1][2 * k] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4341), 0x04000400u, 0xac80ac80u);
-            h[1][2 * k + 1] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4240), 0x04000400u, 0xac80ac80u);
+        for (int k = 0; k < 4; k++) {
+            const uint2 v = *reinterpret_cast<const uint2*>(lut + ((k ? w0 >> (8 * k - 7) : w0 << 7) & 0x7f80u));
+            h[0][k] = v.x;
+            h[1][k] = v.y;
         }
     }
+}
+
+// NF4: for every byte the two codes (the high nibble's first) as fp16 numbers a 2^-7, then b 2^-14: 8 bytes, a copy for each lane of half a
+// warp, so that lanes with different bytes read different banks. Beside 10 byte permutes and 4 multiplications for 4 codes (ALU: two cycles
+// each) it takes 2 shifts, 2 masks and a load: 4096x4096, a launch's products of 4 rows 9,000 cycles before.
+constexpr int kLutBytes = 256 * 128;
+__device__ __forceinline__ void fill_lut(uint8_t* lut) {
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+        uint32_t digits[2] = {0u, 0u};
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+            const int v = __float2int_rn(kNF4[(i >> (n ? 1 : 5)) & 15] * 10000.0f), b = ((v + 64) & 127) - 64, a = (v - b) >> 7;
+            digits[0] |= (uint32_t)__half_as_ushort(__float2half_rn((float)a * 0x1p-7f)) << (16 * n);
+            digits[1] |= (uint32_t)__half_as_ushort(__float2half_rn((float)b * 0x1p-14f)) << (16 * n);
+        }
+        const uint4 v = make_uint4(digits[0], digits[1], digits[0], digits[1]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(lut + (i >> 1) * 128 + (i & 1) * 64 + 16 * k) = v;
+    }
+    __syncthreads();
 }
 
 // The words of block b that row_regs wants (row at shared address `at`)
 template <int F>
 __device__ __forceinline__ void row_words(Shared at, int b, int t, uint32_t& w0, uint32_t& w1) {
-    if (F == CMLB200_Q4_0 || F == CMLB200_NF4) w0 = lds32(at + 16 * b + 4 * t);
+    if (F == CMLB200_Q4_0 || kNF4Like<F>) w0 = lds32(at + 16 * b + 4 * t);
     else if (F == CMLB200_Q8_0) { w0 = lds32(at + 32 * b + 4 * t); w1 = lds32(at + 32 * b + 16 + 4 * t); }
     else if (F == CMLB200_Q4_1) w0 = lds32(at + 20 * b + 4 + 4 * t);
     else if (F == CMLB200_Q4_K) w0 = lds32(at + 16 + 16 * b + 4 * t);
@@ -241,12 +255,12 @@ __device__ __forceinline__ void row_words(Shared at, int b, int t, uint32_t& w0,
 }
 
 template <int F>
-__device__ __forceinline__ void block_regs(Shared lo, Shared hi, int b, int t, uint32_t off_lo, uint32_t off_hi, uint32_t (&a)[kDigits<F>][2][4]) {
+__device__ __forceinline__ void block_regs(Shared lo, Shared hi, int b, int t, uint32_t off_lo, uint32_t off_hi, Shared lut, uint32_t (&a)[kDigits<F>][2][4]) {
     uint32_t w0 = 0, w1 = 0, v0 = 0, v1 = 0, r[kDigits<F>][4], s[kDigits<F>][4];
     row_words<F>(lo, b, t, w0, w1);
     row_words<F>(hi, b, t, v0, v1);
-    row_regs<F>(lo, b, t, w0, w1, off_lo, r);
-    row_regs<F>(hi, b, t, v0, v1, off_hi, s);
+    row_regs<F>(lo, b, t, w0, w1, off_lo, lut, r);
+    row_regs<F>(hi, b, t, v0, v1, off_hi, lut, s);
 #pragma unroll
     for (int d = 0; d < kDigits<F>; d++)
 #pragma unroll
@@ -278,6 +292,9 @@ __device__ __forceinline__ void head_of(const SplitArgs& p, Shared at, int row, 
     }
 }
 
+// Byte n of w as a float: 2^23 and the byte, less 2^23 (a permute and an addition; a shift, a mask and a conversion take twice the cycles)
+__device__ __forceinline__ float byte_of(uint32_t w, int n) { return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + (uint32_t)n)) - 8388608.0f; }
+
 // Scale of block b (Q6_K: of its half `k`)
 template <int F, bool QUIRK>
 __device__ __forceinline__ float scale_of(const SplitArgs& p, Shared at, const Head& h, int b, int k) {
@@ -285,17 +302,17 @@ __device__ __forceinline__ float scale_of(const SplitArgs& p, Shared at, const H
         const uint16_t s = (uint16_t)lds16(at + Lay<F>::SC + 2 * b);
         return QUIRK ? cml_half_to_float(s) : __half2float(__ushort_as_half(s));
     }
-    if (F == CMLB200_NF4) return ldsf(at + Lay<F>::SC + 4 * (b >> p.nf4_shift)) * kNF4Unit;
+    if (kNF4Like<F>) return ldsf(at + Lay<F>::SC + 4 * (b >> p.nf4_shift)) * kNF4Unit;
     if (F == CMLB200_Q4_1) return cml_half_to_float((uint16_t)lds16(at + 20 * b));
     if (F == CMLB200_Q6_K) return h.d * (float)(int)(int8_t)at[h.off + 192 + 2 * b + k];
-    return h.d * (float)(((b < 4 ? h.s0 : h.s1) >> (8 * (b & 3))) & 255u);
+    return h.d * byte_of(b < 4 ? h.s0 : h.s1, b & 3);
 }
 
 // What block b adds per sum of x: its minimum, and what the centring of its quants took off
 template <int F>
 __device__ __forceinline__ float offset_of(Shared at, const Head& h, int b, float scale) {
     if (F == CMLB200_Q4_1) return fmaf(8.0f, scale, cml_half_to_float((uint16_t)lds16(at + 20 * b + 2)));
-    const float mn = h.m * (float)(((b < 4 ? h.m0 : h.m1) >> (8 * (b & 3))) & 255u);
+    const float mn = h.m * byte_of(b < 4 ? h.m0 : h.m1, b & 3);
     return fmaf(F == CMLB200_Q5_K ? 16.0f : 8.0f, scale, -mn);
 }
 
@@ -314,6 +331,15 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// Eight values in the order of the product's columns
+template <bool CONTIG> __device__ __forceinline__ void split8(const float (&e)[8], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = CONTIG ? 2 * k : 4 * (k >> 1) + (k & 1), j = CONTIG ? i + 1 : i + 2;
+        split2(e[i], e[j], hi[k], lo[k]);
+    }
 }
 
 // One output's sums of the warps, in four chains: fewer roundings one upon the other than in a row
@@ -347,7 +373,7 @@ __device__ __noinline__ float plain_dot(const uint8_t* qs, const uint8_t* sc, co
     float sum = 0.f;
     for (int b = 0; b < nblk; b++) {
         const size_t blk = (size_t)row * nblk + b;
-        const float s = F == CMLB200_NF4 ? reinterpret_cast<const float*>(sc)[(size_t)row * per_row + (b >> nf4_shift) / nf4_units]
+        const float s = kNF4Like<F> ? reinterpret_cast<const float*>(sc)[(size_t)row * per_row + (b >> nf4_shift) / nf4_units]
                                          : cml_half_to_float(reinterpret_cast<const uint16_t*>(sc)[blk]);
         float block = 0.f;
         for (int k = 0; k < 32; k++) {
@@ -363,7 +389,7 @@ __device__ __noinline__ float plain_dot(const uint8_t* qs, const uint8_t* sc, co
 }
 template <int F>
 __device__ __forceinline__ float finite_or_plain(float v, const SplitArgs& p, int which, int row, int m) {
-    if constexpr (F == CMLB200_NF4 || F == CMLB200_Q8_0 || F == CMLB200_Q4_0)
+    if constexpr (kNF4Like<F> || F == CMLB200_Q8_0 || F == CMLB200_Q4_0)
         if (!(fabsf(v) <= 3.402823466e38f) && !p.nw)
             return plain_dot<F>(which ? p.qs2 : p.qs, which ? p.sc2 : p.sc, p.x + (size_t)m * p.K, p.K, row, p.nf4_shift, p.nf4_units);
     return v;
@@ -371,7 +397,7 @@ __device__ __forceinline__ float finite_or_plain(float v, const SplitArgs& p, in
 
 // ---- up to 8 rows of x ------------------------------------------------------------------------------------------------------
 constexpr int kWarps = 16;
-template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 ? 2 : Lay<F>::ROW == 144 && NT ? 4 : 3;      // items per warp in flight
+template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 || F == kNF4Fine ? 2 : Lay<F>::ROW == 144 && NT ? 4 : 3;      // items per warp in flight
 constexpr int kOwnBytes = 16 + 4 * 8 * 4;                                // NT = 0: a warp's scaling and block sums of its rows, behind the operands
 constexpr int kXBytes = 2 * 8 * 4 * 16;                                  // operands of one row and unit: [hi, lo][block][t]
 
@@ -406,6 +432,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
     // weights do not depend on the launch before: the kernel that quantizes them on the device ends before its successor begins
 #pragma unroll
     for (int i = 0; i < RING; i++) issue(i);
+    if (kNF4Like<F>) fill_lut(smem + p.lut);
+    Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
@@ -418,20 +446,28 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         if (NT == 0) {
             // one row at a time, eight columns a lane: block lane/4, the columns of thread t = lane%4 of the product
             __syncwarp();
+            const int c0 = un * 256 + g * 32 + (kNF4Like<F> ? 8 : 4) * t, c1 = kNF4Like<F> ? c0 + 4 : c0 + 16;
+            const bool real = un * 8 + g < nblk;
+            float4 xa[4], xc[4];                                // every row is on its way before the first is looked at
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                xa[m] = xc[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (m < p.M && real) {
+                    xa[m] = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c0));
+                    xc[m] = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c1));
+                }
+            }
+            uint2 na = make_uint2(0u, 0u), nc = na;
+            if (p.nw && real) {
+                na = *reinterpret_cast<const uint2*>(p.nw + c0);
+                nc = *reinterpret_cast<const uint2*>(p.nw + c1);
+            }
 #pragma unroll
             for (int m = 0; m < 4; m++) {
                 if (m >= p.M) break;
-                float e[8];
-                const int c0 = un * 256 + g * 32 + (F == CMLB200_NF4 ? 8 : 4) * t, c1 = F == CMLB200_NF4 ? c0 + 4 : c0 + 16;
-                float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
-                if (un * 8 + g < nblk) {
-                    a = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c0));
-                    c = __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)m * p.K + c1));
-                }
-                e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w; e[4] = c.x; e[5] = c.y; e[6] = c.z; e[7] = c.w;
-                if (p.nw && un * 8 + g < nblk) {
-                    const uint2 v = *reinterpret_cast<const uint2*>(p.nw + c0), w = *reinterpret_cast<const uint2*>(p.nw + c1);
-                    const uint32_t h[4] = {v.x, v.y, w.x, w.y};
+                float e[8] = {xa[m].x, xa[m].y, xa[m].z, xa[m].w, xc[m].x, xc[m].y, xc[m].z, xc[m].w};
+                if (p.nw && real) {
+                    const uint32_t h[4] = {na.x, na.y, nc.x, nc.y};
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[k]));
@@ -449,8 +485,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
                 uint32_t hi[4], lo[4];
 #pragma unroll
                 for (int k = 0; k < 8; k++) { e[k] *= up; sum += e[k]; }
-#pragma unroll
-                for (int k = 0; k < 4; k++) split2(e[4 * (k >> 1) + (k & 1)], e[4 * (k >> 1) + (k & 1) + 2], hi[k], lo[k]);
+                split8<kNF4Like<F>>(e, hi, lo);
                 uint4* dst = reinterpret_cast<uint4*>(xs + m * kXBytes) + lane;
                 dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 dst[32] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -500,7 +535,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
 #pragma unroll
             for (int b = 0; b < 8; b++) {
                 uint32_t a[kDigits<F>][2][4];
-                block_regs<F>(lo, hi, b, t, hl.off, hh.off, a);
+                block_regs<F>(lo, hi, b, t, hl.off, hh.off, lut, a);
                 float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 constexpr int C1 = F == CMLB200_Q6_K ? 1 : 0;   // Q6_K: a scale for each half
 #pragma unroll
@@ -617,6 +652,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
     };
     issue(0);
     if (stages > 1) issue(1);
+    if (kNF4Like<F>) fill_lut(smem + p.lut);
+    Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
     uint32_t* const tmem = reinterpret_cast<uint32_t*>(smem + p.extra);
     if (DEEP) {
         if (warp == 0) {
@@ -695,7 +732,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
                 head_of<F>(p, lo, row0 + g, un, hl);
                 head_of<F>(p, hi, row0 + g + 8, un, hh);
                 uint32_t a[kDigits<F>][2][4];
-                block_regs<F>(lo, hi, b, t, hl.off, hh.off, a);
+                block_regs<F>(lo, hi, b, t, hl.off, hh.off, lut, a);
                 constexpr int C1 = F == CMLB200_Q6_K ? 1 : 0;
                 float c[C1 + 1][NT][4];
 #pragma unroll
@@ -828,7 +865,7 @@ int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, c
     return CMLB200_OK;
 }
 
-constexpr size_t kSmemMost = 227 * 1024;
+template <int F> constexpr size_t kSmemMost = 227 * 1024 - (kNF4Like<F> ? kLutBytes + 16 : 0);      // besides the table
 inline size_t wide_extra(const SplitArgs& p, int CG) { return 16 + (size_t)kWarps * 16 * (((p.K + 255) / 256 + kWarps / CG - 1) / (kWarps / CG)); }
 
 template <int F, int NT, bool QUIRK>
@@ -841,7 +878,11 @@ int run_narrow(SplitArgs& p, cudaStream_t st) {
     int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
     if (p.epi == EPI_SWIGLU) per = (per + 1) & ~1;
     p.per_cta = per;
-    const size_t smem = (size_t)W * kRing<F, NT> * kTileBytes<F> + (NT == 0 ? (size_t)W * (p.M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * COLS * 16 + W * 4) * sizeof(float);
+    size_t smem = (size_t)W * kRing<F, NT> * kTileBytes<F> + (NT == 0 ? (size_t)W * (p.M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * COLS * 16 + W * 4) * sizeof(float);
+    if (kNF4Like<F>) {
+        p.lut = (int)((smem + 15) / 16 * 16);
+        smem = p.lut + kLutBytes;
+    }
     auto kern = gemv_split_kernel<F, NT, QUIRK>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
@@ -852,9 +893,10 @@ template <int F, int CG, int T, bool QUIRK, bool DEEP>
 int run_wide(SplitArgs& p, cudaStream_t st) {
     constexpr size_t stage = (size_t)(kWarps / CG) * T * kTileBytes<F>, sums = (size_t)T * kWarps * 16 * 16 * 4;
     const size_t extra = wide_extra(p, CG);
-    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage + extra <= kSmemMost ? 2 : 1;
+    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
     p.extra = (int)(p.stages * stage > sums ? p.stages * stage : sums);
-    const size_t smem = p.extra + extra;
+    p.lut = (int)((p.extra + extra + 15) / 16 * 16);
+    const size_t smem = kNF4Like<F> ? (size_t)p.lut + kLutBytes : p.extra + extra;
     auto kern = gemv_split_wide_kernel<F, CG, T, QUIRK, DEEP>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
@@ -863,14 +905,14 @@ int run_wide(SplitArgs& p, cudaStream_t st) {
 
 template <int F, int CG, bool QUIRK, bool DEEP>
 int run_wide_t(SplitArgs& p, cudaStream_t st) {
-    constexpr int most = kSmemMost / (kWarps / CG * kTileBytes<F>);
+    constexpr int most = kSmemMost<F> / (kWarps / CG * kTileBytes<F>);
     const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
     int best = 1;
     double least = 1e30;
     for (int i = 0; i < 4; i++) {
         const int T = choice[i];
         if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
-        if (T > 1 && (size_t)(kWarps / CG) * T * kTileBytes<F> + wide_extra(p, CG) > kSmemMost) continue;
+        if (T > 1 && (size_t)(kWarps / CG) * T * kTileBytes<F> + wide_extra(p, CG) > kSmemMost<F>) continue;
         const int ctas = (p.tiles + T - 1) / T;
         const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
         if (cost < least) { least = cost; best = T; }
@@ -883,7 +925,7 @@ int run_wide_t(SplitArgs& p, cudaStream_t st) {
 
 template <int F, int CG, bool QUIRK>
 int run_wide_d(SplitArgs& p, cudaStream_t st) {
-    if constexpr (F == CMLB200_NF4 || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
+    if constexpr (kNF4Like<F> || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
         if (split_deep(F, (p.K + 255) / 256, kWarps / CG)) return run_wide_t<F, CG, QUIRK, true>(p, st);
     return run_wide_t<F, CG, QUIRK, false>(p, st);
 }
