@@ -256,8 +256,8 @@ attention_one_kernel(const cmlb200_attn a, const float* __restrict__ qkv, int ld
     float* c_l = c_m + RM;
     float* w_acc = c_l + RM;                           // [ONE_WARPS][RM][dv]; the CTA's sums end up in warp 0's part
     __shared__ float2 red[ONE_WARPS];
-    dep_wait();
     dep_trigger();
+    dep_wait();
     const int splits = gridDim.x, rank = blockIdx.x, kh = blockIdx.y / passes, pass = blockIdx.y % passes, r = blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int h0 = kh * group + pass * RM, nh = min(RM, group - pass * RM);

@@ -123,28 +123,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             for (int i = max(0, it - ST); i < it; i++) mbar_wait(full(i % ST), (i / ST) & 1, abort_flag, 2);      // no copy outlives the CTA
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            int it = 0, done = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, done++) {
-                const int b = done & 1;
-                ok = mbar_wait(acc_empty(b), ((done >> 1) & 1) ^ 1, abort_flag, 3);
+        // the whole warp runs the loop and one lane issues: descriptors stay in uniform registers, and a slab's issue (wait, fence, four
+        // MMAs, commit) stays below the 512 cycles that its MMAs take at BN = 256
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        int s = 0, done = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, done++) {
+            const int b = done & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_empty(b), ((done >> 1) & 1) ^ 1, abort_flag, 3));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int k = 0; k < nkb; k++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full(s), phase, abort_flag, 4));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int k = 0; k < nkb; k++, it++) {
-                    const int s = it % ST;
-                    ok = mbar_wait(full(s), (it / ST) & 1, abort_flag, 4);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = make_desc(sbase + s * C::STAGE), bd = make_desc(sbase + s * C::STAGE + A_BYTES);
+                const uint64_t ad = make_desc(sbase + s * C::STAGE), bd = make_desc(sbase + s * C::STAGE + A_BYTES);
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++)
                         umma(tmem_base + (uint32_t)(b * BN), ad + (uint64_t)(2 * kk), bd + (uint64_t)(2 * kk), idesc, (k | kk) ? 1u : 0u);
                     umma_commit(empty(s));
                 }
-                umma_commit(acc_full(b));
+                __syncwarp();
+                if (++s == ST) { s = 0; phase ^= 1; }
             }
+            if (elect_one()) umma_commit(acc_full(b));
+            __syncwarp();
         }
     } else {
         const int q = warp & 3;                         // the quarter of tensor memory's lanes this warp may read

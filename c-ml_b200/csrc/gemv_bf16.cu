@@ -62,8 +62,8 @@ gemv_bf16_kernel(const __nv_bfloat16* __restrict__ W, int ldw, const __nv_bfloat
 #pragma unroll
     for (int u = 0; u < RING; u++) fetch(u, warp + u * GV_WARPS);
     if (!EXPERT) {
-        dep_wait();
         dep_trigger();
+        dep_wait();
     }
     float acc[RT][NB][4];
 #pragma unroll

@@ -7,7 +7,9 @@
 namespace {
 
 // Every kernel of a step is launched so that it may become resident while its predecessor drains;
-// each one waits here before it touches anything an earlier kernel of the stream wrote.
+// each one waits here before it touches anything an earlier kernel of the stream wrote. Kernels that trigger before they wait let their
+// successors request weights that much earlier; a step's first kernels (embedding, advance_tokens) trigger behind their wait, so what a
+// step's rows are (positions, slots) has been written before any later kernel of it begins.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
