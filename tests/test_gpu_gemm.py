@@ -73,6 +73,22 @@ def test_gemm_nf4_config_shape_sampled(pkg, synth, ob, orc, torch_dev, M):
     assert rel_err_inf(got, full) <= TOL
 
 
+@pytest.mark.parametrize("kind", ["nf4", "q4_0", "q8_0"])
+@pytest.mark.parametrize("K", [64, 320])
+@pytest.mark.parametrize("M", [257, 288, 300, 511, 512, 600])
+def test_gemm_pairs_of_ctas_at_their_edges(pkg, synth, ob, orc, torch_dev, kind, K, M):
+    """More than 256 rows over 74 pairs of 256 weight rows (one round, or two with 600 rows), the last pair ragged: the second MMA's
+    smallest and largest number of columns, one slab of K and an odd number of them."""
+    rng = np.random.default_rng(K + M)
+    N = 18900
+    W, Wf = make_weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    _, xr = synth.bf16_round(x)
+    got = _gemm(pkg, synth, W, x, N, torch_dev)
+    want = (to_dev(xr.reshape(x.shape), torch_dev).double() @ to_dev(Wf, torch_dev).double().T).cpu().numpy()
+    assert rel_err_inf(got, want) <= TOL
+
+
 @pytest.mark.parametrize("kind,N,K,M", [("q4_0", 11008, 4096, 512), ("nf4", 4096, 4096, 2000), ("q4_0", 4096, 11008, 2048), ("nf4", 4096, 4096, 4096)])
 def test_gemm_large_shapes_repeated(pkg, synth, ob, orc, torch_dev, kind, N, K, M):
     """LLaMA-sized weights with 512 to 4096 activation rows, incl. a ragged last tile; every output

@@ -70,6 +70,24 @@ def test_residual_norm_forms(pkg, torch_dev, dim, ldy, ldo, out):
         assert (got[:, dim:] == 0).all() and (got[n:] == 0).all()
 
 
+@pytest.mark.parametrize("rows,dim", [(300, 1024), (300, 1028), (300, 2048), (300, 2052), (2, 4), (2, 4096), (2, 4100), (2, 8192), (2, 8196)])
+def test_residual_norm_at_the_edges_of_a_threads_columns(pkg, torch_dev, rows, dim):
+    """256 threads (many rows) and 1,024 hold four or eight columns each; longer rows wait in shared memory."""
+    import torch
+    g = torch.Generator(device=torch_dev).manual_seed(dim)
+    x, y = (torch.randn(rows, dim, device=torch_dev, generator=g) * s for s in (0.3, 0.1))
+    wp, wn = (1 + 0.5 * torch.randn(dim, device=torch_dev, generator=g) for _ in range(2))
+    X, Y, P, N = (t.double().cpu().numpy() for t in (x, y, wp, wn))
+    for post in (True, False):
+        xs, o = x.clone(), torch.zeros(rows, dim, device=torch_dev)
+        pkg.check(pkg.lib.cmlb200_residual_norm(xs.data_ptr(), y.data_ptr(), dim, wp.data_ptr() if post else None, wn.data_ptr(), 1e-2, rows, dim, None,
+                                                o.data_ptr(), pkg.DT_F32, dim, None))
+        sync()
+        want = X + (lo.rms_norm(Y, P, 1e-2) if post else Y)
+        assert np.abs(xs.cpu().numpy() - want).max() < 1e-5
+        assert np.abs(o.cpu().numpy() - lo.rms_norm(want, N, 1e-2)).max() < 2e-5
+
+
 @pytest.mark.parametrize("ff", [16, 33, 250])
 @pytest.mark.parametrize("act", ["gelu", "silu"])
 def test_glu_rows_f32(pkg, torch_dev, ff, act):
