@@ -11,11 +11,11 @@
 #include "gemv_paths.cuh"
 
 // Where the fp16-split kernels (gemv_split.cuh) are the faster ones. us a call, weights from memory, [this | the alternative]:
-//   Q4_0  11008x4096: M = 1 8.3 | 6.7, 3 9.4 | 13.6 (two launches of the alternative), 4 10.0 | 9.4, 8 12.9 | 12.9, 16 19.6 | 24.8,
-//         32 30.1 | 48.3: at 1, 2 and 4 rows the int8-digit kernel fits its columns exactly, from 9 on it makes several passes
-//   Q8_0  4096x4096: 1 5.6 | 4.6, 2 6.3 | 5.1 (4096x11008: 13.5 | 17.9, two launches), 3 6.8 | 9.3, 8 8.8 | 14.1, 32 16.8 | 82.6
-//   NF4 4096x4096: 1 9.5 | 63.5, 4 11.2 | 70.5, 32 26.5 | 562; Q4_K: 1 5.9 | 7.4, 8 9.6 | 22.9, 32 21.0 | 83.8; Q6_K: 1 7.8 | 9.7, 8 10.6 | 27.3,
-//         32 21.6 | 109.9; Q4_1: 1 5.6 | 7.3, 32 18.4 | 79.9 (the alternative of the GGUF types, gemv_kquant.cu, is left with columns
+//   Q4_0  11008x4096: M = 1 8.3 | 6.7, 3 9.6 | 13.6 (two launches of the alternative), 4 10.0 | 9.4, 8 12.9 | 12.9, 16 17.7 | 24.8,
+//         32 27.6 | 48.3: at 1, 2 and 4 rows the int8-digit kernel fits its columns exactly, from 9 on it makes several passes
+//   Q8_0  4096x4096: 1 5.6 | 4.6, 2 6.3 | 5.1 (4096x11008: 13.5 | 17.9, two launches), 3 6.8 | 9.3, 8 7.8 | 14.1, 32 14.5 | 82.6
+//   NF4 4096x4096: 1 7.8 | 63.5, 4 9.6 | 70.5, 32 20.5 | 562; Q4_K: 1 5.9 | 7.4, 8 9.6 | 22.9, 32 21.0 | 83.8; Q6_K: 1 7.4 | 9.7, 8 8.9 | 27.3,
+//         32 21.6 | 109.9; Q4_1: 1 5.8 | 7.3, 32 15.9 | 79.9 (the alternative of the GGUF types, gemv_kquant.cu, is left with columns
 //         that are no whole 256 and short rows at M = 1: 16 warps share the 256-column units of a row, Q6_K 4608x1536 6.3 | 5.5).
 //         Q8_0 7424x3840: 4 9.3 | 8.7
 //   Q5_K  11008x4096: 1 15.2 | 14.9, 2 15.8 | 23.5, 32 49.8 | 189.5; 1024x4096: 1 4.6 | 5.5

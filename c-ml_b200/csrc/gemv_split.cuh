@@ -17,14 +17,16 @@
 //                       warp itself (columns 2r, 2r+1 = hi, lo of row r); NT = 1: 5 to 8 rows, planes from x_split_kernel.
 //                       A warp keeps the B operands of its unit in registers and walks the CTA's row tiles.
 //   gemv_split_wide_kernel   9 to 32 rows: B operands are loaded per block and used by T row tiles whose sums stay in registers;
-//                       16 columns of x a warp, from 17 rows on two warps share a part of K.
+//                       a warp has all columns of x.
 //
-// What bounds it: instructions. 50 a block of 16 x 32 weights at M = 1 (10 to unpack, 6 to address and load, 2 products, 8 to apply the
-// scales, the rest the rows of x), 65 a warp and block at M = 32, at an issue rate of 0.42 to 0.66 a scheduler; tensor pipe 41 % busy
-// at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers) beat eight with 255 up to
-// 16 rows: 8.2 against 10.4 us at M = 1 (Q4_0 11008x4096), 9.9 against 11.4 at M = 16 (4096x4096). At M = 32 eight were the faster
-// ones (14.7 against 16.1 us, 4096x4096); that form is not built. More chains of
-// products (the block's halves apart) cost more additions than they hid: 14.3 against 12.9 us at M = 8. Times: gemv.cu.
+// What bounds it: instructions and the chains between them. A block of 16 x 32 weights at M = 1 takes a thread about 50 (10 to unpack, 6 to
+// address and load, 2 products, 8 to apply the scales, the rest the rows of x); logic operations, permutes and packed halves issue every
+// second cycle; tensor pipe 41 % busy at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers)
+// beat eight with 255 up to 16 rows: 8.2 against 10.4 us at M = 1 (Q4_0 11008x4096), 9.9 against 11.4 at M = 16 (4096x4096); from 17 rows
+// on eight are the faster ones. More chains of products (the block's halves apart) cost more additions than they hid: 14.3 against
+// 12.9 us at M = 8. The same products by tcgen05.mma, weights put into tensor memory block by block, were no faster: a block's sums have a
+// place of their own there and are read back, and every step of that pipeline (a wait, two fences, an arrival, 550 cycles from an
+// MMA to who waits for it) costs more than the mma.sync it saves: 34.5 us at M = 32, 17.4 at M = 16 (Q4_0 11008x4096). Times: gemv.cu.
 #pragma once
 #include "common.cuh"
 #include "mma_util.cuh"
@@ -352,17 +354,17 @@ template <int COLS> __device__ __forceinline__ float warp_sums(const float* src,
 }
 
 // Eight sums of a thread to and from eight columns of tensor memory
-__device__ __forceinline__ void tmem_put8(uint32_t at, const float (&v)[2][4]) {
+__device__ __forceinline__ void tmem_put8(uint32_t at, const float (&v)[4], const float (&w)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
-                 ::"f"(v[0][0]), "f"(v[0][1]), "f"(v[0][2]), "f"(v[0][3]), "f"(v[1][0]), "f"(v[1][1]), "f"(v[1][2]), "f"(v[1][3]), "r"(at) : "memory");
+                 ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "r"(at) : "memory");
 }
-__device__ __forceinline__ void tmem_add8(uint32_t at, float (&v)[2][4]) {
+__device__ __forceinline__ void tmem_add8(uint32_t at, float (&v)[4], float (&w)[4]) {
     float r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "r"(at));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int k = 0; k < 8; k++) v[k >> 2][k & 3] += r[k];
+    for (int k = 0; k < 4; k++) { v[k] += r[k]; w[k] += r[4 + k]; }
 }
 
 // An output that came out infinite or not a number, once more by plain fp32 multiply-adds: an infinite x is no pair of fp16 numbers
@@ -397,6 +399,7 @@ __device__ __forceinline__ float finite_or_plain(float v, const SplitArgs& p, in
 
 // ---- up to 8 rows of x ------------------------------------------------------------------------------------------------------
 constexpr int kWarps = 16;
+template <int NT> constexpr int kShares = 32 / NT;      // warps of a CTA with 8 NT columns of x
 template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 || F == kNF4Fine ? 2 : Lay<F>::ROW == 144 && NT ? 4 : 3;      // items per warp in flight
 constexpr int kOwnBytes = 16 + 4 * 8 * 4;                                // NT = 0: a warp's scaling and block sums of its rows, behind the operands
 constexpr int kXBytes = 2 * 8 * 4 * 16;                                  // operands of one row and unit: [hi, lo][block][t]
@@ -638,13 +641,15 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
 }
 
 // ---- 9 to 32 rows of x --------------------------------------------------------------------------------------------------------
-// A warp has 16 columns (two products) of x and a share of K. CG = 1: sixteen shares; CG = 2 (17 rows of x and more): eight, whose
-// weights two warps read, each for its own columns.
-template <int F, int CG, int T, bool QUIRK, bool DEEP>
-__global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
+// A warp has all columns of x (NT products of eight) and a share of K: sixteen warps up to 16 rows of x, eight with twice the registers
+// beyond, so that weights are unpacked once for 32 rows and the chains of a block's products are four. (Sixteen warps, two of them for
+// a share with half the columns each, took 29.2 us where this takes 27.6: Q4_0 11008x4096, 32 rows; Q4_K 4096x11008 45.4 and 37.5, Q6_K
+// 32000x4096 135 and 101, NF4 4096x4096 25.3 and 20.5.)
+template <int F, int NT, int T, bool QUIRK, bool DEEP>
+__global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, NT = 2, COLS = 16 * CG, W = kWarps / CG;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp / CG, cg = warp % CG, g = lane >> 2, t = lane & 3;
+    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, COLS = 8 * NT, W = kShares<NT>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp, g = lane >> 2, t = lane & 3;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int stages = p.stages;
     Shared rings = smem + share * (stages * T * TB);
@@ -654,21 +659,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
     Pieces<F> pc;
     pc.init(p.K / 32, lane);
     int iss = 0;
-    auto issue = [&](int buf) {                                 // (the warps of a share bring every CG-th tile)
+    auto issue = [&](int buf) {
         if (iss < my_units) {
 #pragma unroll
             for (int i = 0; i < T; i++) {
-                if (CG > 1 && i % CG != cg) continue;
                 const int tile = min(tile0 + i, p.tiles - 1);
                 issue_tile<F>(p, pc, pairs ? tile & 1 : 0, (pairs ? tile >> 1 : tile) * 16, share + iss * W, ring + (buf * T + i) * TB, lane);
             }
             iss++;
         }
         cp_async_commit();
-    };
-    auto meet = [&]() {                                         // the warps of a share
-        if (CG == 1) __syncwarp();
-        else asm volatile("bar.sync %0, %1;" ::"r"(share + 1), "n"(32 * CG) : "memory");
     };
     issue(0);
     if (stages > 1) issue(1);
@@ -695,42 +695,42 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
             for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
     uint4 nh[NT], nl[NT];                                       // B operands of the next block
     auto fetch = [&](int blk) {
-        const uint4* src = p.planes + ((size_t)blk * CG + cg) * (NT * 64) + lane;
+        const uint4* src = p.planes + (size_t)blk * (NT * 64) + lane;
 #pragma unroll
         for (int j = 0; j < NT; j++) { nh[j] = __ldcg(src + j * 64); nl[j] = __ldcg(src + j * 64 + 32); }
     };
     if (my_units) fetch(share * 8);
     // exponent fields of what undoes the scaling of the warp's columns, unit after unit
-    uint8_t* const fields = smem + p.extra + 16 + warp * (16 * ((units + W - 1) / W));
-    for (int i = lane; i < 4 * my_units; i += 32) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.xf + (size_t)(share + (i >> 2) * W) * COLS + 16 * cg + 4 * (i & 3)));
+    uint8_t* const fields = smem + p.extra + 16 + warp * (COLS * ((units + W - 1) / W));
+    constexpr int WORDS = COLS / 4;
+    for (int i = lane; i < WORDS * my_units; i += 32) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.xf + (size_t)(share + i / WORDS * W) * COLS + 4 * (i % WORDS)));
         *reinterpret_cast<uint32_t*>(fields + 4 * i) = (__float_as_uint(v.x) >> 23) | (__float_as_uint(v.y) >> 23 << 8) | (__float_as_uint(v.z) >> 23 << 16) |
                                                        (__float_as_uint(v.w) >> 23 << 24);
     }
     __syncwarp();
-    auto undoes = [&](int u) { return lds16(fields + 16 * u + 2 * t) | lds16(fields + 16 * u + 8 + 2 * t) << 16; };     // the thread's four columns
-    // a thread's place in tensor memory: its warp's 32 lanes, 64 columns for each of the four warps of a quadrant
-    const uint32_t totals = DEEP ? *tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * 64u : 0u;
+    auto undoes = [&](int u, int j) { return lds16(fields + COLS * u + 8 * j + 2 * t); };      // the thread's two columns of product j
+    // a thread's place in tensor memory: its warp's 32 lanes, as many columns for each of the warps of a quadrant
+    const uint32_t totals = DEEP ? *tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * (uint32_t)(1024 / W) : 0u;
     int buf = 0;
     for (int u = 0; u < my_units; u++) {
         const int un = share + u * W;
         if (!DEEP && u) {                                       // the sums follow to the unit's scaling, exactly: by 2^40 at most (x_split_kernel)
-            const uint32_t now = undoes(u), before = undoes(u - 1);
-            if (now != before) {
 #pragma unroll
-                for (int j = 0; j < NT; j++)
+            for (int j = 0; j < NT; j++) {
+                const uint32_t now = undoes(u, j), before = undoes(u - 1, j);
+                if (now == before) continue;
 #pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        const int at = 8 * (2 * j + k);
-                        const float ratio = power(127u + ((before >> at) & 255u) - ((now >> at) & 255u));
+                for (int k = 0; k < 2; k++) {
+                    const float ratio = power(127u + ((before >> (8 * k)) & 255u) - ((now >> (8 * k)) & 255u));
 #pragma unroll
-                        for (int i = 0; i < T; i++) { acc[i][j][k] *= ratio; acc[i][j][k + 2] *= ratio; }
-                    }
+                    for (int i = 0; i < T; i++) { acc[i][j][k] *= ratio; acc[i][j][k + 2] *= ratio; }
+                }
             }
         }
         if (stages > 1) cp_async_wait<1>();
         else cp_async_wait<0>();
-        meet();
+        __syncwarp();
         Shared base = rings + buf * T * TB + g * ROW;
 #pragma unroll 1
         for (int b = 0; b < 8; b++) {
@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
             float2 s32[NT];
             if (kMins<F>) {
 #pragma unroll
-                for (int j = 0; j < NT; j++) s32[j] = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * COLS + 16 * cg + 8 * j + 2 * t));
+                for (int j = 0; j < NT; j++) s32[j] = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * COLS + 8 * j + 2 * t));
             }
 #pragma unroll
             for (int i = 0; i < T; i++) {
@@ -793,20 +793,25 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
                 }
             }
         }
-        meet();                                                 // every lane is done with this buffer
+        __syncwarp();                                           // every lane is done with this buffer
         issue(buf);
         if (++buf == stages) buf = 0;
         if (DEEP) {
-            const uint32_t undo = undoes(u);
 #pragma unroll
             for (int i = 0; i < T; i++) {
 #pragma unroll
-                for (int j = 0; j < NT; j++)
+                for (int j = 0; j < NT; j++) {
+                    const uint32_t undo = undoes(u, j);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (2 * j + (k & 1))));
-                if (u) tmem_add8(totals + 8 * i, acc[i]);
+                    for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (k & 1)));
+                }
+#pragma unroll
+                for (int j = 0; j < NT; j += 2) {
+                    const uint32_t at = totals + (uint32_t)(4 * NT * i + 4 * j);
+                    if (u) tmem_add8(at, acc[i][j], acc[i][j + 1]);
+                    if (u + 1 < my_units) tmem_put8(at, acc[i][j], acc[i][j + 1]);
+                }
                 if (u + 1 < my_units) {
-                    tmem_put8(totals + 8 * i, acc[i]);
 #pragma unroll
                     for (int j = 0; j < NT; j++)
 #pragma unroll
@@ -817,13 +822,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
         }
     }
     if (!DEEP && my_units) {
-        const uint32_t undo = undoes(my_units - 1);
 #pragma unroll
-        for (int i = 0; i < T; i++)
+        for (int j = 0; j < NT; j++) {
+            const uint32_t undo = undoes(my_units - 1, j);
 #pragma unroll
-            for (int j = 0; j < NT; j++)
+            for (int i = 0; i < T; i++)
 #pragma unroll
-                for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (2 * j + (k & 1))));
+                for (int k = 0; k < 4; k++) acc[i][j][k] *= power(undo >> (8 * (k & 1)));
+        }
     }
     if (DEEP) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cp_async_wait<0>();
@@ -838,7 +844,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_wide_kernel(const S
     for (int i = 0; i < T; i++)
 #pragma unroll
         for (int j = 0; j < NT; j++) {
-            float* dst = part + ((size_t)i * W + share) * (COLS * 16) + (16 * cg + 8 * j + 2 * t) * 16 + g;
+            float* dst = part + ((size_t)i * W + share) * (COLS * 16) + (8 * j + 2 * t) * 16 + g;
             dst[0] = acc[i][j][0];
             dst[16] = acc[i][j][1];
             dst[8] = acc[i][j][2];
@@ -886,7 +892,7 @@ int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, c
 }
 
 template <int F> constexpr size_t kSmemMost = 227 * 1024 - (kNF4Like<F> ? kLutBytes + 16 : 0);      // besides the table
-inline size_t wide_extra(const SplitArgs& p, int CG) { return 16 + (size_t)kWarps * 16 * (((p.K + 255) / 256 + kWarps / CG - 1) / (kWarps / CG)); }
+template <int NT> size_t wide_extra(const SplitArgs& p) { return 16 + (size_t)kShares<NT> * 8 * NT * (((p.K + 255) / 256 + kShares<NT> - 1) / kShares<NT>); }
 
 template <int F, int NT, bool QUIRK>
 int run_narrow(SplitArgs& p, cudaStream_t st) {
@@ -909,45 +915,45 @@ int run_narrow(SplitArgs& p, cudaStream_t st) {
     return launch_split(kern, (p.tiles + per - 1) / per, W, smem, st, p);
 }
 
-template <int F, int CG, int T, bool QUIRK, bool DEEP>
+template <int F, int NT, int T, bool QUIRK, bool DEEP>
 int run_wide(SplitArgs& p, cudaStream_t st) {
-    constexpr size_t stage = (size_t)(kWarps / CG) * T * kTileBytes<F>, sums = (size_t)T * kWarps * 16 * 16 * 4;
-    const size_t extra = wide_extra(p, CG);
-    p.stages = (p.K + 255) / 256 > kWarps / CG && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
+    constexpr size_t stage = (size_t)kShares<NT> * T * kTileBytes<F>, sums = (size_t)T * 32 * 8 * 16 * 4;
+    const size_t extra = wide_extra<NT>(p);
+    p.stages = (p.K + 255) / 256 > kShares<NT> && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
     p.extra = (int)(p.stages * stage > sums ? p.stages * stage : sums);
     p.lut = (int)((p.extra + extra + 15) / 16 * 16);
     const size_t smem = kNF4Like<F> ? (size_t)p.lut + kLutBytes : p.extra + extra;
-    auto kern = gemv_split_wide_kernel<F, CG, T, QUIRK, DEEP>;
+    auto kern = gemv_split_wide_kernel<F, NT, T, QUIRK, DEEP>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
-    return launch_split(kern, (p.tiles + T - 1) / T, kWarps, smem, st, p);
+    return launch_split(kern, (p.tiles + T - 1) / T, kShares<NT>, smem, st, p);
 }
 
-template <int F, int CG, bool QUIRK, bool DEEP>
+template <int F, int NT, bool QUIRK, bool DEEP>
 int run_wide_t(SplitArgs& p, cudaStream_t st) {
-    constexpr int most = kSmemMost<F> / (kWarps / CG * kTileBytes<F>);
+    constexpr int most = kSmemMost<F> / (kShares<NT> * kTileBytes<F>);
     const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
     int best = 1;
     double least = 1e30;
     for (int i = 0; i < 4; i++) {
         const int T = choice[i];
         if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
-        if (T > 1 && (size_t)(kWarps / CG) * T * kTileBytes<F> + wide_extra(p, CG) > kSmemMost<F>) continue;
+        if (T > 1 && (size_t)kShares<NT> * T * kTileBytes<F> + wide_extra<NT>(p) > kSmemMost<F>) continue;
         const int ctas = (p.tiles + T - 1) / T;
         const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
         if (cost < least) { least = cost; best = T; }
     }
-    if constexpr (most >= 5) if (best == 5) return run_wide<F, CG, 5, QUIRK, DEEP>(p, st);
-    if constexpr (most >= 3) if (best == 3) return run_wide<F, CG, 3, QUIRK, DEEP>(p, st);
-    if (best == 2) return run_wide<F, CG, 2, QUIRK, DEEP>(p, st);
-    return run_wide<F, CG, 1, QUIRK, DEEP>(p, st);
+    if constexpr (most >= 5) if (best == 5) return run_wide<F, NT, 5, QUIRK, DEEP>(p, st);
+    if constexpr (most >= 3) if (best == 3) return run_wide<F, NT, 3, QUIRK, DEEP>(p, st);
+    if (best == 2) return run_wide<F, NT, 2, QUIRK, DEEP>(p, st);
+    return run_wide<F, NT, 1, QUIRK, DEEP>(p, st);
 }
 
-template <int F, int CG, bool QUIRK>
+template <int F, int NT, bool QUIRK>
 int run_wide_d(SplitArgs& p, cudaStream_t st) {
     if constexpr (kNF4Like<F> || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
-        if (split_deep(F, (p.K + 255) / 256, kWarps / CG)) return run_wide_t<F, CG, QUIRK, true>(p, st);
-    return run_wide_t<F, CG, QUIRK, false>(p, st);
+        if (split_deep(F, (p.K + 255) / 256, kShares<NT>)) return run_wide_t<F, NT, QUIRK, true>(p, st);
+    return run_wide_t<F, NT, QUIRK, false>(p, st);
 }
 
 template <int F, bool QUIRK>
@@ -955,8 +961,8 @@ int run_split(SplitArgs& p, int nt, cudaStream_t st) {
     switch (nt) {
         case 0: return run_narrow<F, 0, QUIRK>(p, st);
         case 1: return run_narrow<F, 1, QUIRK>(p, st);
-        case 2: return run_wide_d<F, 1, QUIRK>(p, st);
-        default: return run_wide_d<F, 2, QUIRK>(p, st);
+        case 2: return run_wide_d<F, 2, QUIRK>(p, st);
+        default: return run_wide_d<F, 4, QUIRK>(p, st);
     }
 }
 
