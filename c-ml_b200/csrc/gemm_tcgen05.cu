@@ -5,24 +5,33 @@
 // triple loop" (src/nn/qlora.c:264-317) and its dequantize-at-load + fp32 matmul
 // (src/core/gguf.c:271-295, src/ops/ir/execution.c:989-1052).
 //
-// A CTA works on a tile of 128 weight rows (the MMA "M" side, operand A) by NX <= 512 activation rows (the MMA "N" side, operand B;
-// two MMAs and two halves of tensor memory above 256), K in slabs of 64. Where the tiles are fewer than the SMs, a cluster of 2 to 8
-// CTAs shares the K of a tile: their sums meet in distributed shared memory, every CTA adds and finishes its part of the columns in
-// rank order (no scratch in global memory, no second launch, the same result every time).
+// A tile is 128 weight rows (the MMA "M" side, operand A) by NX <= 256 activation rows (the MMA "N" side, operand B), or 256 weight rows
+// by 257 to 512 activation rows, which a pair of CTAs shares (cta_group::2: a CTA expands 128 weight rows and holds half of the
+// activations, two MMAs into two halves of tensor memory). K in slabs of 64. Where the small tiles are fewer than the SMs, a cluster
+// of 2 to 8 CTAs shares the K of a tile: their sums meet in distributed shared memory, every CTA adds and finishes its part of the
+// columns in rank order (no scratch in global memory, no second launch, the same result every time).
 //   warp 0      one lane issues TMA tensor loads of the bf16 activation slab (128B swizzle, boxes of up to 256 rows)
-//   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma (128 x 256 x 16, kind::f16)
+//   warp 1      allocates tensor memory; an elected lane (of the pair's first CTA) issues tcgen05.mma (kind::f16, 128 or 256 x NX x 16);
+//               in the second CTA it passes on that the CTA's slab is ready
 //   warps 2..17 expand the packed weights to bf16 in the canonical K-major 128B-swizzled layout the MMA reads, two groups of eight
 //               the slabs in turn; they are the epilogue too: tcgen05.ld, then Y or the cluster's sum
-// What bounds it: the expansion up to 256 activation rows (a slab of 128 x 64 weights takes 0.37 us for Q4_0, 0.54 for NF4, 0.63 for
-// Q8_0, about as long as its instructions at half an instruction a cycle and scheduler), from 512 on expansion and MMA (0.54 us
-// for 128 x 512 x 64) about equally. Hence the tile: as many activation rows as fill the SMs in whole waves (pick_shape).
+// What bounds it: up to 256 activation rows the expansion (a slab of 128 x 64 weights takes 0.37 us for Q4_0, 0.54 for NF4, 0.63 for
+// Q8_0, about as long as its instructions at half an instruction a cycle and scheduler) beside about 4 us to start and 2.5 to 4 for a
+// cluster's sum; above, the MMA: a slab of 256 x 512 x 64 takes a pair 1,090 cycles, the tensor cores 1,024 of them. Pairs halve what an SM
+// reads of the activations (every 128 weight rows used to read all of them: 1.4 GB from L2 at 2,048 rows of 11008x4096) and the
+// expansion per MMA. The issuing warp is the next limit: with a barrier for each box, or an arrival released for the cluster, a slab took
+// 1,440 cycles. Hence the tile: as many activation rows as fill the SMs in whole waves (pick_shape).
 // Packed weights and scales come by plain loads into registers, three slabs of the group ahead. Each thread keeps one
 // block index and no other address, and the issuing warp counts its stages: with 64-bit addresses, zeroed registers and a vote
 // in every wait a slab took 0.60 instead of 0.40 us, with a division per slab in the issuing warp 0.54.
-// us a call, before and after (before: 128 x 512 tiles, four groups fed by TMA, K splits through global memory), weights from memory:
-//   Q4_0 4096x4096    M = 77 22.4 14.6, 512 37.0 25.0, 2048 65.2 55.5      11008x4096  77 43.0 29.0, 512 64.0 55.6, 2048 201 156
-//   Q4_0 4096x11008   M = 77 35.0 24.2, 512 64.0 46.3, 2048 171 141        32000x4096  77 82.0 52.5, 512 130 110, 2048 477 397
-//   NF4 4096x4096     M = 77 22.8 17.4, 512 41.1 30.1, 2048 67.7 59.6      Q8_0 4096x4096  77 22.6 18.8, 512 39.6 33.4, 2048 94.3 68.0
+// The cluster's sum: a thread has four weight rows of a column, reads all ranks' sums in 16-byte pieces that are in flight together, and
+// stores 8 or 16 bytes; one value and one rank after the other, with a last barrier that waited for the stores, it took 1.1 to 2.2 us more
+// (3.5 for NF4 at 511 rows). A table of NF4's code pairs in shared memory instead of permutes was slower (4096x4096 77 rows 17.5 18.2).
+// us a call, weights from memory, before and after the pairs and this sum:
+//   Q4_0 4096x4096    M = 77 15.1 13.9, 512 25.6 23.4, 2048 56.0 49.6      11008x4096  77 31.3 30.8, 512 57.0 49.8, 2048 159 130
+//   Q4_0 4096x11008   M = 77 25.9 24.5, 512 49.0 46.1, 2048 142 124        32000x4096  77 59.7 59.6, 512 111 97.6, 2048 408 357
+//   NF4 4096x4096     M = 77 17.5 16.1, 512 30.1 26.7, 2048 58.8 50.5      Q8_0 4096x4096  77 18.0 17.4, 512 30.8 30.1, 2048 65.6 52.1
+//   Q8_0 7000x5120    M = 600 87.6 53.9
 // Expansion:
 //   Q4_0  a byte permute drops two nibbles into the mantissas of two bf16 halves (0x43nn = 128 + n), one packed subtract gives
 //         n - 8 exactly, one packed multiply applies the block scale
@@ -276,7 +285,8 @@ __device__ __forceinline__ void expand32(const uint4* raw, float scale, uint4 (&
 //   GEMM_SWIGLU_BF16 silu(gate[i]) * value stored as bf16   (the up projection finishing SwiGLU,
 //                                                            src/nn/llama.c:126-155; gate may be the output array)
 enum { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_ACC_F32 = 2, GEMM_SWIGLU_BF16 = 3 };
-// CNT finished values of one weight row (neighbouring activation rows; `count` of them exist), `at` the first one's place. What
+// CNT finished values `N` places apart (neighbouring activation rows of one weight row; or, 1 apart, the other way round), of which
+// `count` exist, `at` the first one's place. What
 // they are multiplied with or added to is loaded first, so that the loads are in flight together. (Reductions in global memory,
 // which load nothing, make zeros of sums below 2^-126.)
 template <int CNT>
@@ -301,12 +311,14 @@ __device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int
         float* o = static_cast<float*>(out) + at;
 #pragma unroll
         for (int k = 0; k < CNT; k += 8) {                           // eight loads in flight: sixteen spill more registers
-            float h[8];
+            constexpr int B = CNT < 8 ? CNT : 8;
+            static_assert(CNT % B == 0, "whole batches");
+            float h[B];
 #pragma unroll
-            for (int j = 0; j < 8; j++)
+            for (int j = 0; j < B; j++)
                 if (k + j < count) h[j] = o[(size_t)j * N];
 #pragma unroll
-            for (int j = 0; j < 8; j++, o += N)
+            for (int j = 0; j < B; j++, o += N)
                 if (k + j < count) *o = h[j] + v[k + j];
         }
     } else {
@@ -315,6 +327,28 @@ __device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int
         for (int j = 0; j < CNT; j++, o += N)
             if (j < count) *o = v[j];
     }
+}
+
+// The same of four neighbouring weight rows in one activation row, all there, in memory aligned to them
+__device__ __forceinline__ void finish4(void* out, const __nv_bfloat16* gate, int mode, size_t at, float (&v)[4]) {
+    if (mode == GEMM_ACC_F32 || mode == GEMM_OUT_F32) {
+        float4* const o = reinterpret_cast<float4*>(static_cast<float*>(out) + at);
+        float4 h = make_float4(v[0], v[1], v[2], v[3]);
+        if (mode == GEMM_ACC_F32) {
+            h = *o;
+            h.x += v[0]; h.y += v[1]; h.z += v[2]; h.w += v[3];
+        }
+        *o = h;
+        return;
+    }
+    if (mode == GEMM_SWIGLU_BF16) {
+        const uint2 w = *reinterpret_cast<const uint2*>(gate + at);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
+        const float g[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] *= g[e] / (1.0f + expf(-g[e]));
+    }
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + at) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
 }
 
 __device__ __forceinline__ uint4 ld_weights(const uint4* p) {        // the row's next slabs come into L2 along with it
@@ -548,31 +582,51 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
         }
     }
     if (ranks > 1) {                                                 // one tile, its K over the cluster: CTA r adds and finishes its share of the columns
-        __syncthreads();
+        __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
         const int n0 = first_tile / p.tiles_m * BN, m0 = (first_tile % p.tiles_m) * p.NX;
         if (warp >= 2 && !*abort_flag) {
-            const int q = warp & 3, part = (warp - 2) >> 2, r = q * 32 + lane;
-            const int per = ((p.NX + (int)ranks - 1) / (int)ranks + 1) & ~1, c_end = min(p.NX, ((int)rank + 1) * per);
-            for (int c0 = (int)rank * per + part * 8; c0 < c_end; c0 += 32) {
-                float v[8];
+            const int cols = min(p.NX, p.M - m0), per = (cols + (int)ranks - 1) / (int)ranks, c0 = (int)rank * per;
+            const int r = lane * 4, quads = n0 + r < p.N ? (min(cols, c0 + per) - c0) * 32 : 0;      // four weight rows of a column each
+            const bool whole = p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0 && ((uintptr_t)p.gate & 7) == 0;
+            auto add = [&](auto most) {
+                constexpr int R = decltype(most)::value, Q = 8 / R;
+                for (int i = (warp - 2) * 32 + lane; i < quads; i += Q * DQ_THREADS) {
+                    float x[Q][R][4];
 #pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = 0.f;
-                for (uint32_t k = 0; k < ranks; k++) {
-                    uint32_t at;
-                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(sbase + (uint32_t)(c0 * 128 + r) * 4u), "r"(k));
+                    for (int j = 0; j < Q; j++)
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (c0 + j < c_end) {
-                            float x;
-                            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at + (uint32_t)j * 512u) : "memory");
-                            v[j] += x;
-                        }
+                        for (int k = 0; k < R; k++)
+                            if (i + j * DQ_THREADS < quads && k < (int)ranks) {
+                                uint32_t at;
+                                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(sbase + (uint32_t)((c0 * 32 + i + j * DQ_THREADS) * 16)), "r"(k));
+                                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                                             : "=f"(x[j][k][0]), "=f"(x[j][k][1]), "=f"(x[j][k][2]), "=f"(x[j][k][3]) : "r"(at) : "memory");
+                            }
+#pragma unroll
+                    for (int j = 0; j < Q; j++) {
+                        const int at = i + j * DQ_THREADS;
+                        if (at >= quads) break;
+                        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (int k = 0; k < R; k++)
+                            if (k < (int)ranks)
+#pragma unroll
+                                for (int e = 0; e < 4; e++) v[e] += x[j][k][e];
+                        const size_t to = (size_t)(m0 + c0 + (at >> 5)) * p.N + n0 + r;
+                        if (whole) finish4(p.out, p.gate, p.mode, to, v);
+                        else finish(p.out, p.gate, p.mode, to, 1, p.N - n0 - r, v);
+                    }
                 }
-                if (n0 + r < p.N) finish(p.out, p.gate, p.mode, (size_t)(m0 + c0) * p.N + n0 + r, p.N, min(min(8, c_end - c0), p.M - m0 - c0), v);
-            }
+            };
+            if (ranks <= 2) add(std::integral_constant<int, 2>());
+            else if (ranks <= 4) add(std::integral_constant<int, 4>());
+            else add(std::integral_constant<int, 8>());
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // Nobody leaves while its sums are read. Every value read has been used by now, and nobody in the cluster reads what was stored:
+        // no release, which would wait for those stores.
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -637,8 +691,10 @@ const int* clusters_at_once(Kern kern, size_t smem) {
 
 // Estimated time (us) of a shape: waves of tiles, each K / 64 / ranks slabs of `expand` us for the weights and 0.14 for every 256
 // activation rows, a few us to fill the pipeline and for the epilogue, and for a cluster's sum. Fitted to all shapes of 504 calls (three
-// formats, 640 to 32000 weight rows, 1024 to 14336 columns, 33 to 2048 rows of x): 7 % rms, the shape picked is 0.3 % off the
-// best one on average. 4096x4096, Q4_0, 77 rows: 14.2 us with four ranks (32 of the 33 clusters that fit), 16.0 with three, 27.1 without.
+// formats, 640 to 32000 weight rows, 1024 to 14336 columns, 33 to 2048 rows of x) before there were pairs and with a sum that took 1 to 2
+// us more: 7 % rms then, the shape picked 0.3 % off the best one on average. What the sum takes now (about 1.2 + 0.009 NX + 0.15 ranks)
+// would change the pick of one call in twenty, by 1 to 5 % of the estimate, less than its error. 4096x4096, Q4_0, 77 rows: 13.9 us
+// with four ranks (32 of the 33 clusters that fit); with the former sum 14.2, 16.0 with three, 27.1 without.
 inline double shape_cost(const Shape& s, int M, int N, int KB, const int* at_once, double expand) {
     const int together = s.pair ? 2 : s.ranks, rows = s.pair ? 2 * BN : BN;
     if (!at_once[together] || (s.ranks > 1 && s.NX > B_ROWS)) return 1e30;

@@ -175,6 +175,39 @@ def test_gemm_output_modes(pkg, synth, ob, orc, torch_dev, M):
 
 
 
+@pytest.mark.parametrize("N,K,M,offset", [(384, 128, 33, 0), (384, 1024, 77, 0), (384, 1024, 77, 1), (130, 1024, 45, 0), (1031, 512, 255, 0), (4, 256, 1, 0)])
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_gemm_cluster_sums_at_their_edges(pkg, synth, ob, orc, torch_dev, mode, N, K, M, offset):
+    """What a cluster adds, four weight rows at a time: rows that are no whole fours, outputs off their alignment, every epilogue,
+    and nothing written beside them. Twice rounded weights (2^-9 each) and a bf16 output: 3 x 2^-9 of the norm of the outputs."""
+    rng = np.random.default_rng(1700 + N + M)
+    W, Wf = make_weight(pkg, synth, ob, orc, torch_dev, rng, "q4_0", N, K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    xb, xr = synth.bf16_round(x)
+    want = xr.reshape(x.shape).astype(np.float64) @ Wf.T.astype(np.float64)
+    first = rng.standard_normal((M, N)).astype(np.float32)
+    bf16 = mode in (0, 3)
+    if mode == 3:
+        fb, fr = synth.bf16_round(first)
+        g = fr.reshape(first.shape).astype(np.float64)
+        want, fill = g / (1.0 + np.exp(-g)) * want, fb.reshape(-1)
+    else:
+        fill = np.zeros(M * N, np.uint16) if bf16 else first.reshape(-1)
+    buf = np.concatenate([fill[:1]] * 8 + [fill] + [fill[:1]] * 8)
+    buf = np.roll(buf, offset)
+    d = to_dev(buf, torch_dev)
+    at = d.data_ptr() + (8 + offset) * buf.itemsize
+    d_x = to_dev(xb.reshape(x.shape), torch_dev)
+    pkg.check(pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, mode, at, at if mode == 3 else None, stream_ptr()), "gemm")
+    torch.cuda.synchronize()
+    assert gemm_status(pkg) == 0
+    out = d.cpu().numpy()
+    got = out[8 + offset:8 + offset + M * N]
+    got = (synth.bf16_to_f32(got) if bf16 else got).reshape(M, N)
+    assert np.linalg.norm(got - (first if mode == 2 else 0) - want) <= 3 * 2.0 ** -9 * np.linalg.norm(want)
+    assert np.array_equal(out[:8 + offset], buf[:8 + offset]) and np.array_equal(out[8 + offset + M * N:], buf[8 + offset + M * N:])
+
+
 @pytest.mark.parametrize("M", [48, 200, 300])
 def test_gemm_residual_below_the_normal_range(pkg, synth, ob, orc, torch_dev, M):
     """A residual of subnormal numbers is added to, not flushed: with a cluster's sum, one tile of rows, and two."""
