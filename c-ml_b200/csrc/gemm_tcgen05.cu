@@ -27,7 +27,11 @@
 // The cluster's sum: a thread has four weight rows of a column, reads all ranks' sums in 16-byte pieces that are in flight together, and
 // stores 8 or 16 bytes; one value and one rank after the other, with a last barrier that waited for the stores, it took 1.1 to 2.2 us more
 // (3.5 for NF4 at 511 rows). A table of NF4's code pairs in shared memory instead of permutes was slower (4096x4096 77 rows 17.5 18.2).
-// us a call, weights from memory, before and after the pairs and this sum:
+// What an output is multiplied with or added to is requested before the wait for the accumulators or with the cluster's sums, then a
+// batch ahead; requested with the batch itself, it put a memory latency into each: SwiGLU 11008x4096 77 rows 34.3 31.1, 512 67.7 62.3,
+// 2048 174 158 (without SwiGLU 30.8, 49.2, 130: the rest is the division and exponential of every output), onto a residual 4096x11008
+// 512 48.4 45.5, 4096x4096 512 25.4 22.6, stored as fp32 4096x4096 77 13.9 12.9.
+// us a call, weights from memory, bf16 output, before and after the pairs and this sum:
 //   Q4_0 4096x4096    M = 77 15.1 13.9, 512 25.6 23.4, 2048 56.0 49.6      11008x4096  77 31.3 30.8, 512 57.0 49.8, 2048 159 130
 //   Q4_0 4096x11008   M = 77 25.9 24.5, 512 49.0 46.1, 2048 142 124        32000x4096  77 59.7 59.6, 512 111 97.6, 2048 408 357
 //   NF4 4096x4096     M = 77 17.5 16.1, 512 30.1 26.7, 2048 58.8 50.5      Q8_0 4096x4096  77 18.0 17.4, 512 30.8 30.1, 2048 65.6 52.1
@@ -285,70 +289,62 @@ __device__ __forceinline__ void expand32(const uint4* raw, float scale, uint4 (&
 //   GEMM_SWIGLU_BF16 silu(gate[i]) * value stored as bf16   (the up projection finishing SwiGLU,
 //                                                            src/nn/llama.c:126-155; gate may be the output array)
 enum { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_ACC_F32 = 2, GEMM_SWIGLU_BF16 = 3 };
-// CNT finished values `N` places apart (neighbouring activation rows of one weight row; or, 1 apart, the other way round), of which
-// `count` exist, `at` the first one's place. What
-// they are multiplied with or added to is loaded first, so that the loads are in flight together. (Reductions in global memory,
-// which load nothing, make zeros of sums below 2^-126.)
+// CNT finished values `step` places apart (neighbouring activation rows of one weight row; or, 1 apart, the other way round), of which
+// `count` exist, `at` the first one's place. What they are multiplied with or added to comes first, by a call of its own, so that
+// those loads are in flight together and beside others. (Reductions in global memory, which load nothing, make zeros of sums below 2^-126.)
 template <int CNT>
-__device__ __forceinline__ void finish(void* out, const __nv_bfloat16* gate, int mode, size_t at, int N, int count, const float (&v)[CNT]) {
+__device__ __forceinline__ void operands(const void* out, const __nv_bfloat16* gate, int mode, size_t at, int step, int count, uint32_t (&w)[CNT]) {
     if (mode == GEMM_SWIGLU_BF16) {
-        __nv_bfloat16 o[CNT];
 #pragma unroll
         for (int j = 0; j < CNT; j++)
-            if (j < count) o[j] = gate[at + (size_t)j * N];
+            if (j < count) w[j] = reinterpret_cast<const uint16_t*>(gate)[at + (size_t)j * step];
+    } else if (mode == GEMM_ACC_F32) {
 #pragma unroll
         for (int j = 0; j < CNT; j++)
-            if (j < count) {
-                const float g = __bfloat162float(o[j]);
-                static_cast<__nv_bfloat16*>(out)[at + (size_t)j * N] = __float2bfloat16_rn((g / (1.0f + expf(-g))) * v[j]);
-            }
-    } else if (mode == GEMM_OUT_BF16) {
+            if (j < count) w[j] = static_cast<const uint32_t*>(out)[at + (size_t)j * step];
+    }
+}
+template <int CNT>
+__device__ __forceinline__ void combine(int mode, const uint32_t (&w)[CNT], float (&v)[CNT]) {
+    if (mode == GEMM_SWIGLU_BF16) {
+#pragma unroll
+        for (int j = 0; j < CNT; j++) {
+            const float g = __uint_as_float(w[j] << 16);
+            v[j] *= g / (1.0f + expf(-g));
+        }
+    } else if (mode == GEMM_ACC_F32) {
+#pragma unroll
+        for (int j = 0; j < CNT; j++) v[j] += __uint_as_float(w[j]);
+    }
+}
+template <int CNT>
+__device__ __forceinline__ void store(void* out, int mode, size_t at, int step, int count, const float (&v)[CNT]) {
+    if (mode == GEMM_OUT_BF16 || mode == GEMM_SWIGLU_BF16) {
         __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
 #pragma unroll
-        for (int j = 0; j < CNT; j++, o += N)
+        for (int j = 0; j < CNT; j++, o += step)
             if (j < count) *o = __float2bfloat16_rn(v[j]);
-    } else if (mode == GEMM_ACC_F32) {
-        float* o = static_cast<float*>(out) + at;
-#pragma unroll
-        for (int k = 0; k < CNT; k += 8) {                           // eight loads in flight: sixteen spill more registers
-            constexpr int B = CNT < 8 ? CNT : 8;
-            static_assert(CNT % B == 0, "whole batches");
-            float h[B];
-#pragma unroll
-            for (int j = 0; j < B; j++)
-                if (k + j < count) h[j] = o[(size_t)j * N];
-#pragma unroll
-            for (int j = 0; j < B; j++, o += N)
-                if (k + j < count) *o = h[j] + v[k + j];
-        }
     } else {
         float* o = static_cast<float*>(out) + at;
 #pragma unroll
-        for (int j = 0; j < CNT; j++, o += N)
+        for (int j = 0; j < CNT; j++, o += step)
             if (j < count) *o = v[j];
     }
 }
-
 // The same of four neighbouring weight rows in one activation row, all there, in memory aligned to them
-__device__ __forceinline__ void finish4(void* out, const __nv_bfloat16* gate, int mode, size_t at, float (&v)[4]) {
-    if (mode == GEMM_ACC_F32 || mode == GEMM_OUT_F32) {
-        float4* const o = reinterpret_cast<float4*>(static_cast<float*>(out) + at);
-        float4 h = make_float4(v[0], v[1], v[2], v[3]);
-        if (mode == GEMM_ACC_F32) {
-            h = *o;
-            h.x += v[0]; h.y += v[1]; h.z += v[2]; h.w += v[3];
-        }
-        *o = h;
-        return;
-    }
+__device__ __forceinline__ void operands4(const void* out, const __nv_bfloat16* gate, int mode, size_t at, uint32_t (&w)[4]) {
     if (mode == GEMM_SWIGLU_BF16) {
-        const uint2 w = *reinterpret_cast<const uint2*>(gate + at);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
-        const float g[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-        for (int e = 0; e < 4; e++) v[e] *= g[e] / (1.0f + expf(-g[e]));
+        const uint2 g = *reinterpret_cast<const uint2*>(gate + at);
+        w[0] = g.x & 0xffffu; w[1] = g.x >> 16; w[2] = g.y & 0xffffu; w[3] = g.y >> 16;
+    } else if (mode == GEMM_ACC_F32) {
+        const uint4 h = *reinterpret_cast<const uint4*>(static_cast<const uint32_t*>(out) + at);
+        w[0] = h.x; w[1] = h.y; w[2] = h.z; w[3] = h.w;
     }
-    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + at) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+}
+__device__ __forceinline__ void store4(void* out, int mode, size_t at, const float (&v)[4]) {
+    if (mode == GEMM_OUT_BF16 || mode == GEMM_SWIGLU_BF16)
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + at) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    else *reinterpret_cast<float4*>(static_cast<float*>(out) + at) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 __device__ __forceinline__ uint4 ld_weights(const uint4* p) {        // the row's next slabs come into L2 along with it
@@ -557,6 +553,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                 else slab(raw[2], scale[2], it);
                 slot = slot == 2 ? 0 : slot + 1;
             }
+            const int r = q * 32 + lane, there = ranks == 1 && n0 + r < p.N ? p.M - m0 : 0;
+            auto place = [&](int c) { return (size_t)(m0 + c) * p.N + n0 + r; };
+            uint32_t w[16];
+            auto ahead = [&](int c) { operands(p.out, p.gate, p.mode, place(c), p.N, min(p.NX, there) - c, w); };
+            ahead(part * 16);
             ok = ok && warp_wait(done_bar, seg & 1, abort_flag, 6);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // ---- D[n][m] (lane = weight row, column = activation row) -> Y[m][n], or into shared memory for the cluster
@@ -564,9 +565,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                 for (int c0 = part * 16; c0 < p.NX; c0 += 64) {
                     float f[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, f);
-                    const int r = q * 32 + lane;
                     if (ranks == 1) {
-                        if (n0 + r < p.N) finish(p.out, p.gate, p.mode, (size_t)(m0 + c0) * p.N + n0 + r, p.N, min(p.NX - c0, p.M - m0 - c0), f);
+                        combine(p.mode, w, f);
+                        ahead(c0 + 64);
+                        store(p.out, p.mode, place(c0), p.N, min(p.NX, there) - c0, f);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 16; j++) own[(c0 + j) * 128 + r] = f[j];
@@ -593,6 +595,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                 constexpr int R = decltype(most)::value, Q = 8 / R;
                 for (int i = (warp - 2) * 32 + lane; i < quads; i += Q * DQ_THREADS) {
                     float x[Q][R][4];
+                    uint32_t w[Q][4];
+                    auto place = [&](int at) { return (size_t)(m0 + c0 + (at >> 5)) * p.N + n0 + r; };
+#pragma unroll
+                    for (int j = 0; j < Q; j++)
+                        if (i + j * DQ_THREADS < quads) {
+                            if (whole) operands4(p.out, p.gate, p.mode, place(i + j * DQ_THREADS), w[j]);
+                            else operands(p.out, p.gate, p.mode, place(i + j * DQ_THREADS), 1, p.N - n0 - r, w[j]);
+                        }
 #pragma unroll
                     for (int j = 0; j < Q; j++)
 #pragma unroll
@@ -613,9 +623,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs p) {
                             if (k < (int)ranks)
 #pragma unroll
                                 for (int e = 0; e < 4; e++) v[e] += x[j][k][e];
-                        const size_t to = (size_t)(m0 + c0 + (at >> 5)) * p.N + n0 + r;
-                        if (whole) finish4(p.out, p.gate, p.mode, to, v);
-                        else finish(p.out, p.gate, p.mode, to, 1, p.N - n0 - r, v);
+                        combine(p.mode, w[j], v);
+                        if (whole) store4(p.out, p.mode, place(at), v);
+                        else store(p.out, p.mode, place(at), 1, p.N - n0 - r, v);
                     }
                 }
             };
