@@ -117,6 +117,14 @@ x_split_kernel(const float* __restrict__ x, const __half* __restrict__ nw, float
 
 constexpr int kMaxUnits = 512;                               // K < 131072
 
+// One chain through all of a share's blocks rounds at the size of the result each time. For the formats whose former kernels summed
+// in shorter chains (1.25 to 1.35e-7 of the result off) chains of more than 16 blocks are cut: a unit's sums to those of the units before
+// it, which lie in tensor memory meanwhile, for there are no registers for both. Scalings need not follow one another there.
+// K = 11008, 32 rows: NF4 1.57e-7 in one chain, 1.31e-7 so, Q6_K 1.85 and 1.24e-7. It costs 0.5 to 1 us a launch.
+bool split_deep(int type, int units, int W) {
+    return (type == CMLB200_Q6_K || type == CMLB200_NF4 || type == CMLB200_Q8_0) && units > 2 * W;
+}
+
 }  // namespace
 
 // Weights the kernels take: whole 16-byte rows of quants and whole 256-column units of scales, or (NF4) blocks of 32, 64, 128
@@ -168,7 +176,8 @@ int cmlb200_gemv_split_(const cmlb200_qmat* W, const cmlb200_qmat* W2, const flo
         p.sums = sums;
         p.xf = xf;
         const int shares = nt == 4 ? kWarps / 2 : kWarps, units = (p.K + 255) / 256;
-        const bool follow = nt > 1 && units > shares && !split_deep(W->type, units, shares);
+        p.deep = nt > 1 && split_deep(W->type, units, shares);
+        const bool follow = nt > 1 && units > shares && !p.deep;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(8 * nt);
         cfg.blockDim = dim3(512);

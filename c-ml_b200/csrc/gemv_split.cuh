@@ -62,6 +62,7 @@ struct SplitArgs {
     float* y;
     float eps;
     int N, K, M, tiles, per_cta, stages, epi;
+    bool deep;                     // split_deep's answer: x_split_kernel and the product have to go by the same one
     int lut;                       // NF4: where in shared memory the table of codes lies (whole 16 bytes)
     int extra;                     // 9 rows and more: where in shared memory the address of tensor memory and the scalings go
     int nf4_shift;                 // log2 of how many 32-column blocks one NF4 scale covers, 3 at most
@@ -868,13 +869,6 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
 }
 
 // ---- host side ----------------------------------------------------------------------------------------------------------------------
-// One chain through all of a share's blocks rounds at the size of the result each time. For the formats whose former kernels summed
-// in shorter chains (1.25 to 1.35e-7 of the result off) chains of more than 16 blocks are cut: a unit's sums to those of the units before it, which lie in tensor memory meanwhile, for there are no registers for both.
-// K = 11008, 32 rows: NF4 1.57e-7 in one chain, 1.31e-7 so, Q6_K 1.85 and 1.24e-7. It costs 0.5 to 1 us a launch.
-inline bool split_deep(int type, int units, int W) {
-    return (type == CMLB200_Q6_K || type == CMLB200_NF4 || type == CMLB200_Q8_0) && units > 2 * W;
-}
-
 template <typename Kern>
 int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, const SplitArgs& p) {
     cudaLaunchConfig_t cfg = {};
@@ -952,7 +946,7 @@ int run_wide_t(SplitArgs& p, cudaStream_t st) {
 template <int F, int NT, bool QUIRK>
 int run_wide_d(SplitArgs& p, cudaStream_t st) {
     if constexpr (kNF4Like<F> || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
-        if (split_deep(F, (p.K + 255) / 256, kShares<NT>)) return run_wide_t<F, NT, QUIRK, true>(p, st);
+        if (p.deep) return run_wide_t<F, NT, QUIRK, true>(p, st);
     return run_wide_t<F, NT, QUIRK, false>(p, st);
 }
 

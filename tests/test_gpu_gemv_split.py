@@ -110,6 +110,28 @@ def test_error_against_64_bits(pkg, synth, ob, orc, torch_dev, kind, most, K):
         assert np.sqrt(np.mean(np.square(off))) <= most, (M, off)
 
 
+@pytest.mark.parametrize("M", [12, 32])
+def test_long_rows_of_nf4_blocks_of_32(pkg, synth, ob, orc, torch_dev, M):
+    """More units of 256 columns than two a warp: no further off 64 bits than blocks of 64 (the bound above), and sums of large units
+    are kept where zero units follow them (scalings of a row then lie further apart than an fp32 factor reaches)."""
+    rng = np.random.default_rng(M)
+    N, K, shares = 512, 11008, 16 if M <= 16 else 8
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", N, K, 32)
+    off = []
+    for _ in range(4):
+        x = rng.standard_normal((M, K)).astype(np.float32)
+        d_x, d_y = to_dev(x, torch_dev), torch.empty(M, N, device=torch_dev)
+        pkg.check(pkg.lib.cmlb200_gemv(W.q, d_x.data_ptr(), d_y.data_ptr(), M, stream_ptr()), "gemv")
+        want = x.astype(np.float64) @ Wf.T.astype(np.float64)
+        off.append(np.linalg.norm(d_y.cpu().numpy() - want) / np.linalg.norm(want))
+    for scale in (1.0, 1e6):
+        x = rng.standard_normal((M, K)).astype(np.float32)
+        x[:, :256 * shares] *= scale
+        x[:, 256 * shares:512 * shares] = 0.0
+        _check(pkg, W, Wf, x, torch_dev)
+    assert np.sqrt(np.mean(np.square(off))) <= 1.42e-7, off
+
+
 @pytest.mark.parametrize("kind,batches", [("nf4", (1, 4, 5, 8, 9, 16, 17, 32)), ("q8_0", (9, 32))])
 def test_infinities_and_nan(pkg, synth, ob, orc, torch_dev, kind, batches):
     """Rows of x that are not finite give what fp32 multiply-adds give: infinities with their signs, NaN where an infinity meets a zero
