@@ -62,11 +62,11 @@ struct SplitArgs {
     float* y;
     float eps;
     int N, K, M, tiles, per_cta, stages, epi;
-    bool deep;                     // split_deep's answer: x_split_kernel and the product have to go by the same one
     int lut;                       // NF4: where in shared memory the table of codes lies (whole 16 bytes)
     int extra;                     // 9 rows and more: where in shared memory the address of tensor memory and the scalings go
     int nf4_shift;                 // log2 of how many 32-column blocks one NF4 scale covers, 3 at most
     int nf4_units;                 // units one covers, 1 at least
+    bool deep;                     // split_deep's answer: x_split_kernel and the product have to go by the same one
 };
 
 // Shared memory through pointers, so that the compiler may order the loads as it likes between the waits
@@ -405,10 +405,10 @@ template <int F, int NT> constexpr int kRing = Lay<F>::ROW > 176 || F == kNF4Fin
 constexpr int kOwnBytes = 16 + 4 * 8 * 4;                                // NT = 0: a warp's scaling and block sums of its rows, behind the operands
 constexpr int kXBytes = 2 * 8 * 4 * 16;                                  // operands of one row and unit: [hi, lo][block][t]
 
-template <int F, int NT, bool QUIRK>
+template <int F, int NT, bool QUIRK, int RING>
 __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, RING = kRing<F, NT>, COLS = NT == 0 ? 4 : 8;
+    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, COLS = NT == 0 ? 4 : 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // shared memory: rings [W][RING][TB] | NT = 0: operands [W][M][kXBytes], scaling and sums [W][kOwnBytes] | sums [per_cta][W][COLS][16] | squares [W][4]
@@ -888,25 +888,43 @@ int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, c
 template <int F> constexpr size_t kSmemMost = 227 * 1024 - (kNF4Like<F> ? kLutBytes + 16 : 0);      // besides the table
 template <int NT> size_t wide_extra(const SplitArgs& p) { return 16 + (size_t)kShares<NT> * 8 * NT * (((p.K + 255) / 256 + kShares<NT> - 1) / kShares<NT>); }
 
-template <int F, int NT, bool QUIRK>
-int run_narrow(SplitArgs& p, cudaStream_t st) {
-    constexpr int COLS = NT == 0 ? 4 : 8;
-    const int units = (p.K + 255) / 256, W = units < kWarps ? units : kWarps, sms = cmlb_num_sms();
-    // as many row tiles a CTA as fill the SMs once, or several times where that would be more than six (5 tiles of 11008 rows:
-    // 8.2 us at M = 1; 3: 11.4, 2: 13.3, for every CTA makes the operands of x again)
-    const int want = (p.tiles + sms - 1) / sms, rounds = (want + 5) / 6;
-    int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
-    if (p.epi == EPI_SWIGLU) per = (per + 1) & ~1;
-    p.per_cta = per;
-    size_t smem = (size_t)W * kRing<F, NT> * kTileBytes<F> + (NT == 0 ? (size_t)W * (p.M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * COLS * 16 + W * 4) * sizeof(float);
+constexpr int kMostTiles = 6;                                            // row tiles of a CTA
+
+// Shared memory of gemv_split_kernel besides NF4's table
+template <int F, int NT> constexpr size_t narrow_smem(int ring, int W, int M, int per) {
+    return (size_t)W * ring * kTileBytes<F> + (NT == 0 ? (size_t)W * (M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * (NT == 0 ? 4 : 8) * 16 + W * 4) * sizeof(float);
+}
+
+template <int F, int NT, bool QUIRK, int RING>
+int launch_narrow(SplitArgs& p, int W, cudaStream_t st) {
+    size_t smem = narrow_smem<F, NT>(RING, W, p.M, p.per_cta);
     if (kNF4Like<F>) {
         p.lut = (int)((smem + 15) / 16 * 16);
         smem = p.lut + kLutBytes;
     }
-    auto kern = gemv_split_kernel<F, NT, QUIRK>;
+    auto kern = gemv_split_kernel<F, NT, QUIRK, RING>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
-    return launch_split(kern, (p.tiles + per - 1) / per, W, smem, st, p);
+    return launch_split(kern, (p.tiles + p.per_cta - 1) / p.per_cta, W, smem, st, p);
+}
+
+template <int F, int NT, bool QUIRK>
+int run_narrow(SplitArgs& p, cudaStream_t st) {
+    const int units = (p.K + 255) / 256, W = units < kWarps ? units : kWarps, sms = cmlb_num_sms();
+    // as many row tiles a CTA as fill the SMs once, or several times where that would be more than six (5 tiles of 11008 rows:
+    // 8.2 us at M = 1; 3: 11.4, 2: 13.3, for every CTA makes the operands of x again)
+    const int want = (p.tiles + sms - 1) / sms, rounds = (want + kMostTiles - 1) / kMostTiles;
+    int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
+    if (p.epi == EPI_SWIGLU) per = (per + 1) & ~1;
+    p.per_cta = per;
+    // sixteen warps, four rows, six tiles: where that is too much (NF4, blocks of 64 and more), such calls have rings of two
+    // (13824x5120, 4 rows: 25.5 us; without the table, whose place a third item took, 32.4)
+    constexpr int ring = kRing<F, NT>;
+    constexpr bool fits = narrow_smem<F, NT>(ring, kWarps, 4, kMostTiles) <= kSmemMost<F>;
+    static_assert(kMostTiles % 2 == 0 && (fits || narrow_smem<F, NT>(2, kWarps, 4, kMostTiles) <= kSmemMost<F>), "the largest calls do not fit shared memory");
+    if constexpr (!fits)
+        if (narrow_smem<F, NT>(ring, W, p.M, per) > kSmemMost<F>) return launch_narrow<F, NT, QUIRK, 2>(p, W, st);
+    return launch_narrow<F, NT, QUIRK, ring>(p, W, st);
 }
 
 template <int F, int NT, int T, bool QUIRK, bool DEEP>

@@ -52,6 +52,38 @@ def test_nf4_blocks_and_partial_units(pkg, synth, ob, orc, torch_dev, block, K, 
     _check(pkg, W, Wf, rng.standard_normal((M, K)).astype(np.float32), torch_dev)
 
 
+@pytest.mark.parametrize("M", [3, 4, 5, 32])
+@pytest.mark.parametrize("N,K,block", [(13824, 5120, 64), (28352, 3904, 64), (11904, 3872, 32)])
+def test_nf4_six_row_tiles_a_cta(pkg, synth, ob, orc, torch_dev, N, K, block, M):
+    """What needs most shared memory: six row tiles for each of sixteen warps, the table of codes beside them."""
+    rng = np.random.default_rng(N + M)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", N, K, block)
+    X, F = to_dev(rng.standard_normal((M, K)).astype(np.float32), torch_dev), to_dev(Wf, torch_dev).double()
+    y = torch.empty(M, N, device=torch_dev)
+    pkg.check(pkg.lib.cmlb200_gemv(W.q, X.data_ptr(), y.data_ptr(), M, stream_ptr()), "gemv")
+    want, size = X.double() @ F.T, X.double().abs() @ F.abs().T
+    assert ((y.double() - want).abs() <= (2.0 ** -21 + (K / 32 + 32) * 2.0 ** -23) * size).all()
+
+
+@pytest.mark.parametrize("M", [4, 8])
+@pytest.mark.parametrize("N,K", [(4800, 3904), (11008, 4096)])
+def test_nf4_swiglu_of_large_pairs(pkg, synth, ob, orc, torch_dev, N, K, M):
+    """Six row tiles a CTA of the two weights in turn. The error of silu(g) u is at most 1.1 |u| of g's and |silu(g)| of u's, and 2^-20 of
+    the value for the exponential, the division and the product."""
+    rng = np.random.default_rng(N + M)
+    (G, Gf), (U, Uf) = (_weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", N, K) for _ in range(2))
+    X = to_dev(rng.standard_normal((M, K)).astype(np.float32), torch_dev)
+    y = torch.empty(M, N, device=torch_dev)
+    pkg.check(pkg.lib.cmlb200_gemv_swiglu(G.q, U.q, X.data_ptr(), y.data_ptr(), M, stream_ptr()), "swiglu")
+    off, of = 2.0 ** -21 + (K / 32 + 32) * 2.0 ** -23, []
+    for f in (Gf, Uf):
+        F = to_dev(f, torch_dev).double()
+        of.append((X.double() @ F.T, off * (X.double().abs() @ F.abs().T)))
+    (g, dg), (u, du) = of
+    silu = g / (1 + torch.exp(-g))
+    assert ((y.double() - silu * u).abs() <= 1.1 * dg * (u.abs() + du) + silu.abs() * du + 2.0 ** -20 * (silu * u).abs()).all()
+
+
 @pytest.mark.parametrize("scale", [1e-30, 1e-6, 1e6, 1e30])
 @pytest.mark.parametrize("M", [3, 7, 20])
 def test_any_range_of_x(pkg, synth, ob, orc, torch_dev, scale, M):
