@@ -54,6 +54,7 @@ _sig("cmlb200_unrepack_gguf", ci, ci, vp, vp, ci, ci, vp)
 _sig("cmlb200_gguf_dequantize", ci, ci, vp, vp, sz, vp)
 _sig("cmlb200_dequant_qmat", ci, C.POINTER(QMat), vp, vp)
 _sig("cmlb200_dequantize_nf4", ci, vp, vp, ci, ci, sz, vp, vp)
+_sig("cmlb200_quantize_nf4", ci, vp, sz, ci, vp, vp, vp)
 _sig("cmlb200_gemv", ci, C.POINTER(QMat), vp, vp, ci, vp)
 _sig("cmlb200_gemv_noalloc", ci, C.POINTER(QMat), vp, vp, ci, vp)
 _sig("cmlb200_gemv_accum", ci, C.POINTER(QMat), vp, vp, ci, vp)

@@ -176,10 +176,6 @@ __global__ void nf4_codes_kernel(const float* __restrict__ x, size_t numel, int 
     }
 }
 
-// Ends a chain of launches whose results the kernel behind it may read before its dependency wait: it begins when they are written, and
-// nothing begins before it has ended.
-__global__ void settle_kernel() {}
-
 inline int grid_for(size_t work, int threads) {
     size_t g = (work + threads - 1) / threads;
     size_t cap = (size_t)cmlb_num_sms() * 16;
@@ -255,8 +251,6 @@ extern "C" int cmlb200_quantize_nf4(const float* d_x, size_t numel, int block, u
     nf4_absmax_kernel<<<grid_for(nblocks, 128), 128, 0, as_stream(stream)>>>(d_x, numel, block, d_scales, nblocks);
     CMLB_LAUNCH_CHECK();
     nf4_codes_kernel<<<grid_for((numel + 1) / 2, 256), 256, 0, as_stream(stream)>>>(d_x, numel, block, d_scales, d_packed);
-    CMLB_LAUNCH_CHECK();
-    settle_kernel<<<1, 32, 0, as_stream(stream)>>>();            // products request weights ahead of their dependency wait
     CMLB_LAUNCH_CHECK();
     return CMLB200_OK;
 }

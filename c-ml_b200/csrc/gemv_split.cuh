@@ -10,7 +10,7 @@
 // Error against 64 bits on N(0,1) inputs: 1.2e-7 to 2e-7 of the result's norm, as the int8-digit kernels have.
 //
 // Work: item = 16 weight rows x 256 columns; the warps of a CTA share K (a warp takes every W-th 256-column unit), each
-// with a ring of its own that cp.async fills, the first items before the launch waits for its predecessor. Sums of the
+// with a ring of its own that cp.async fills, the first items (but NF4's) before the launch waits for its predecessor. Sums of the
 // warps meet in shared memory and are added in warp order, so results do not depend on timing.
 //
 //   gemv_split_kernel   up to 8 rows of x. NT = 0: up to 4 rows, made into hi / lo columns of ONE 8-column product by the
@@ -433,12 +433,15 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
         }
         cp_async_commit();
     };
-    // weights do not depend on the launch before: the kernel that quantizes them on the device ends before its successor begins
+    // weights do not depend on the launch before, but NF4 ones may: it may have quantized them, or written their scales
+    if (kNF4Like<F>) {
+        fill_lut(smem + p.lut);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
 #pragma unroll
     for (int i = 0; i < RING; i++) issue(i);
-    if (kNF4Like<F>) fill_lut(smem + p.lut);
     Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!kNF4Like<F>) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
     int buf = 0;
@@ -671,9 +674,12 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
         }
         cp_async_commit();
     };
+    if (kNF4Like<F>) {                                          // (as above)
+        fill_lut(smem + p.lut);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
     issue(0);
     if (stages > 1) issue(1);
-    if (kNF4Like<F>) fill_lut(smem + p.lut);
     Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
     uint32_t* const tmem = reinterpret_cast<uint32_t*>(smem + p.extra);
     if (DEEP) {

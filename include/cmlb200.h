@@ -53,7 +53,11 @@ extern "C" {
  *   scales Q8_0/Q4_0: rows*(cols/32) fp16, row-major (the `d` of each block).
  *          NF4 : rows*cols/block fp32 absmax values.
  * Both planes must be 16-byte aligned; cols must be a multiple of 32 (and of
- * `block` for NF4) so that every row starts on a 16-byte boundary. */
+ * `block` for NF4) so that every row starts on a 16-byte boundary.
+ * NF4 weights are read in stream order. Weights in the other formats, which no kernel of this
+ * library writes, are constants to cmlb200_gemv and its relatives: they may be read before the
+ * kernel launched just before the call has ended. A program that writes such weights with a kernel
+ * of its own puts a synchronisation or a copy on that stream between that kernel and the call. */
 typedef struct cmlb200_qmat {
     int type;
     int rows;

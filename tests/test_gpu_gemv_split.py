@@ -213,3 +213,56 @@ def test_streams_keep_their_rows_apart(pkg, synth, ob, orc, torch_dev):
             pkg.check(pkg.lib.cmlb200_gemv(W.q, x.data_ptr(), y.data_ptr(), 16, s.cuda_stream), "gemv")
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(alone, out))
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("M", [1, 4, 8, 32])
+def test_nf4_weights_written_by_the_launch_before(pkg, torch_dev, captured, M):
+    """NF4 weights quantized, or given new scales by another product (whose successors begin early), right before the product that reads
+    them: the same bits as with a synchronisation between, in order and captured."""
+    lib, N, K, block = pkg.lib, 1024, 4096, 64
+    g = torch.Generator(torch_dev).manual_seed(M)
+    qs, scales = torch.zeros(N * K // 2, dtype=torch.uint8, device=torch_dev), torch.zeros(N * K // block, device=torch_dev)
+    W = pkg.QMat(pkg.NF4, N, K, block, qs.data_ptr(), scales.data_ptr(), 0, None)
+    maker_qs = torch.randint(0, 256, (4096 * 2048,), dtype=torch.uint8, device=torch_dev, generator=g)
+    maker_sc = (torch.rand(4096 * 2048 // 32, device=torch_dev, generator=g) * 0.01).half()
+    maker = pkg.QMat(pkg.Q8_0, 4096, 2048, 32, maker_qs.data_ptr(), maker_sc.data_ptr(), 0, None)     # 16 x 4096 results: the scales
+    sources = [(torch.randn(N, K, device=torch_dev, generator=g), torch.randn(16, 2048, device=torch_dev, generator=g)) for _ in range(6)]
+    x = torch.randn(M, K, device=torch_dev, generator=g)
+    w, h, y = torch.empty(N, K, device=torch_dev), torch.empty(16, 2048, device=torch_dev), [torch.empty(M, N, device=torch_dev) for _ in range(2)]
+
+    def run(stream, between):
+        pkg.check(lib.cmlb200_quantize_nf4(w.data_ptr(), N * K, block, qs.data_ptr(), scales.data_ptr(), stream), "quantize")
+        between()
+        pkg.check(lib.cmlb200_gemv(W, x.data_ptr(), y[0].data_ptr(), M, stream), "gemv")
+        between()
+        pkg.check(lib.cmlb200_gemv(maker, h.data_ptr(), scales.data_ptr(), 16, stream), "scales")
+        between()
+        pkg.check(lib.cmlb200_gemv(W, x.data_ptr(), y[1].data_ptr(), M, stream), "gemv")
+
+    stream, want = torch.cuda.Stream(), []
+    for a, b in sources:
+        w.copy_(a)
+        h.copy_(b)
+        torch.cuda.synchronize()
+        run(stream.cuda_stream, torch.cuda.synchronize)
+        torch.cuda.synchronize()
+        want.append([t.clone() for t in y])
+    graph = torch.cuda.CUDAGraph()
+    if captured:
+        with torch.cuda.graph(graph, stream=stream):
+            run(stream.cuda_stream, lambda: None)
+    torch.cuda.synchronize()
+    got = []
+    with torch.cuda.stream(stream):
+        for a, b in sources * 3:
+            w.copy_(a)
+            h.copy_(b)
+            if captured:
+                graph.replay()
+            else:
+                run(stream.cuda_stream, lambda: None)
+            got.append([t.clone() for t in y])
+    torch.cuda.synchronize()
+    for i, pair in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(pair, want[i % len(want)])), i
