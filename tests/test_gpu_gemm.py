@@ -208,6 +208,32 @@ def test_gemm_cluster_sums_at_their_edges(pkg, synth, ob, orc, torch_dev, mode, 
     assert np.array_equal(out[:8 + offset], buf[:8 + offset]) and np.array_equal(out[8 + offset + M * N:], buf[8 + offset + M * N:])
 
 
+@pytest.mark.parametrize("N,K,M", [(18900, 320, 300), (18821, 64, 257), (18821, 128, 511), (18900, 64, 600)])
+@pytest.mark.parametrize("mode", [1, 2, 3])
+def test_gemm_pairs_of_ctas_with_every_epilogue(pkg, synth, ob, orc, torch_dev, mode, N, K, M):
+    """fp32 output, a residual, SwiGLU in place, of 74 pairs of CTAs (with 600 rows twice) whose last one ends in its second CTA's first
+    rows or in their middle, and nothing written beside them. Bound as with clusters."""
+    rng = np.random.default_rng(N + M + mode)
+    W, Wf = make_weight(pkg, synth, ob, orc, torch_dev, rng, "q4_0", N, K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    xb, xr = synth.bf16_round(x)
+    d_x = to_dev(xb.reshape(x.shape), torch_dev)
+    want = to_dev(xr.reshape(x.shape), torch_dev).double() @ to_dev(Wf, torch_dev).double().T
+    first = torch.randn(16 + M * N, device=torch_dev, generator=torch.Generator(torch_dev).manual_seed(M))
+    first = first.to(torch.bfloat16) if mode == 3 else first
+    before = first[8:-8].double().reshape(M, N)
+    if mode == 3:
+        want = before * torch.sigmoid(before) * want
+    out = first.clone()
+    at = out[8:].data_ptr()
+    pkg.check(pkg.lib.cmlb200_gemm_bf16_ex(W.q, d_x.data_ptr(), M, mode, at, at if mode == 3 else None, stream_ptr()), "gemm")
+    torch.cuda.synchronize()
+    assert gemm_status(pkg) == 0
+    got = out[8:-8].double().reshape(M, N)
+    assert ((got - before if mode == 2 else got) - want).norm() <= 3 * 2.0 ** -9 * want.norm()
+    assert torch.equal(out[:8], first[:8]) and torch.equal(out[-8:], first[-8:])
+
+
 @pytest.mark.parametrize("M", [48, 200, 300])
 def test_gemm_residual_below_the_normal_range(pkg, synth, ob, orc, torch_dev, M):
     """A residual of subnormal numbers is added to, not flushed: with a cluster's sum, one tile of rows, and two."""
