@@ -55,9 +55,9 @@ extern "C" {
  * Both planes must be 16-byte aligned; cols must be a multiple of 32 (and of
  * `block` for NF4) so that every row starts on a 16-byte boundary.
  * NF4 weights are read in stream order. Weights in the other formats, which no kernel of this
- * library writes, are constants to cmlb200_gemv and its relatives: they may be read before the
- * kernel launched just before the call has ended. A program that writes such weights with a kernel
- * of its own puts a synchronisation or a copy on that stream between that kernel and the call. */
+ * library writes, are constants to cmlb200_gemv and its relatives: they may be read before kernels
+ * launched ahead of the call have ended. A program that writes such weights with a kernel of its
+ * own puts a synchronisation or a copy on that stream between that kernel and the call. */
 typedef struct cmlb200_qmat {
     int type;
     int rows;
@@ -417,7 +417,8 @@ int cmlb200_ipc_close(void* d_ptr);
 
 /* A dense [rows, cols] weight (rows = out features), row stride `ld` elements. Allocated with rows rounded
  * up to 16 and ld a multiple of 64, the padding zero. dtype CMLB200_DT_F32 or CMLB200_DT_BF16. bias and cap belong to the
- * products with fp32 results (not to the _glu forms and not to the experts'). */
+ * products with fp32 results (not to the _glu forms and not to the experts'). Weights are constants to the _gemv_ forms, as
+ * those of cmlb200_qmat are: a kernel that writes them is followed by a synchronisation or a copy. */
 typedef struct cmlb200_dense {
     int dtype;
     int rows, cols, ld;
@@ -644,7 +645,8 @@ int cmlb200_ring_rows(const cmlb200_attn* a, const float* d_qkv, int ld, const i
  * _tiles (fp16 cache): [tile][heads][64][ld] in units of log2, keys from the tile's first visible one rounded down to 16 on, tiles as in
  * cmlb200_attention_tiles, ld a multiple of 64. _rows: [row][heads][ld], keys from the row's first visible one on; natural
  * units over an fp32 cache, log2 over fp16. max_keys bounds the keys of any row or tile, its own included. _heads: the most
- * heads that _tiles takes. */
+ * heads that _tiles takes. _rows may read positions, slots and the block table before kernels launched ahead have ended: behind a
+ * kernel that writes them comes cmlb200_embed_rows, a synchronisation or a copy first. */
 int cmlb200_talk_scores_tiles(const cmlb200_attn* a, const uint16_t* d_q_f16, const int* d_tiles, int tiles, int max_keys, float* d_scores, int ld, void* stream);
 int cmlb200_talk_scores_rows(const cmlb200_attn* a, const void* d_q, const int* d_row_pos, const int* d_row_slot, int rows, int max_keys, float* d_scores, int ld,
                              void* stream);
