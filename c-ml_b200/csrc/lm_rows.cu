@@ -309,8 +309,8 @@ residual_norm_kernel(float* __restrict__ x, const float* __restrict__ y, int ldy
                      int parts, const int* __restrict__ part_pos, const float* __restrict__ part_w) {
     extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
-    dep_trigger();
     dep_wait();
+    dep_trigger();
     const int r = blockIdx.x;
     auto part_sum = [&](auto zero, int i) {
         auto s = zero;
@@ -389,7 +389,7 @@ residual_norm_kernel(float* __restrict__ x, const float* __restrict__ y, int ldy
 
 // The same where a thread's columns (four at a time, HELD times at most) fit its registers, every row with one of y at most: y, the
 // residual and the weights are requested together, so a row waits for memory once and not three times. 8 rows of 2,048 take 2.4 us
-// behind the launch before where the form above takes 3.1, 2,000 rows 11.4 and 13.
+// where the form above takes 2.8, 2,000 rows 9.2 and 9.5.
 template <typename TO, int HELD>
 __global__ void __launch_bounds__(1024)
 residual_norm_held_kernel(float* __restrict__ x, const float* __restrict__ y, int ldy, const float* __restrict__ w_post, const float* __restrict__ w_next,
@@ -398,8 +398,8 @@ residual_norm_held_kernel(float* __restrict__ x, const float* __restrict__ y, in
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), ones = make_float4(1.f, 1.f, 1.f, 1.f);
     float4 wp[HELD], wn[HELD], v[HELD], o[HELD];
     const int i0 = threadIdx.x * 4, step = blockDim.x * 4, r = blockIdx.x;
-    dep_trigger();
     dep_wait();
+    dep_trigger();
     float* xr = x + (size_t)(idx ? idx[r] : r) * dim;
     float ss = 0.f;
     auto square = [](float4 a, float s) { return fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, s)))); };
@@ -668,7 +668,8 @@ static int launch_residual(float* d_x, const float* d_y, int ldy, const cmlb200_
     // few rows: enough threads that each meets its row once; many rows: small CTAs, several to an SM
     int threads = 256;
     if (rows <= 2 * cmlb_num_sms()) while (threads < 1024 && threads * 4 < dim) threads *= 2;
-    if (vec && !parts && dim <= 8 * threads) {
+    // held in registers: 1,024 threads of them leave an SM no second CTA, so up to one row an SM (296x4096 5.8 us so, 5.4 us in shared memory)
+    if (vec && !parts && dim <= 8 * threads && (threads < 1024 || rows <= cmlb_num_sms())) {
 #define RN_HELD(TO, H) CMLB_CUDA(launch_chain(residual_norm_held_kernel<TO, H>, dim3(rows), dim3(threads), 0, 1, st, d_x, d_y, ldy, d_w_post, d_w_next, eps, dim, d_row_idx, (TO*)d_out, ldo, raw))
         const bool once = dim <= 4 * threads;
         if (out_dtype == CMLB200_DT_BF16) { if (once) RN_HELD(__nv_bfloat16, 1); else RN_HELD(__nv_bfloat16, 2); }

@@ -9,7 +9,8 @@ namespace {
 // Every kernel of a step is launched so that it may become resident while its predecessor drains;
 // each one waits here before it touches anything an earlier kernel of the stream wrote. Kernels that trigger before they wait let their
 // successors request weights that much earlier; a step's first kernels (embedding, advance_tokens) trigger behind their wait, so what a
-// step's rows are (positions, slots) has been written before any later kernel of it begins.
+// step's rows are (positions, slots) has been written before any later kernel of it begins. The residual norm triggers behind its wait: ahead of
+// it, CTAs of the launches behind lay between its own (420 rows of 4,096: 8.3 us, 5.3 so; a decode step of eight sequences 222 us, 217 so).
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
