@@ -645,15 +645,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
 }
 
 // ---- 9 to 32 rows of x --------------------------------------------------------------------------------------------------------
-// A warp has all columns of x (NT products of eight) and a share of K: sixteen warps up to 16 rows of x, eight with twice the registers
-// beyond, so that weights are unpacked once for 32 rows and the chains of a block's products are four. (Sixteen warps, two of them for
-// a share with half the columns each, took 29.2 us where this takes 27.6: Q4_0 11008x4096, 32 rows; Q4_K 4096x11008 45.4 and 37.5, Q6_K
-// 32000x4096 135 and 101, NF4 4096x4096 25.3 and 20.5.)
-template <int F, int NT, int T, bool QUIRK, bool DEEP>
-__global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
+// A warp has NT products of eight columns of x and a share of K. CG = 1: all columns of x, sixteen warps up to 16 rows of x, eight with twice
+// the registers beyond, so that weights are unpacked once for 32 rows and the chains of a block's products are four. CG = 2: sixteen
+// warps, two of them for a share, each with its half of 32 columns; for short rows (kFewUnits). Longer ones of 17 to 32 rows take 29.2 us
+// so where eight warps take 27.6 (Q4_0 11008x4096; Q4_K 4096x11008 45.4 and 37.5, Q6_K 32000x4096 135 and 101).
+template <int F, int NT, int CG, int T, bool QUIRK, bool DEEP>
+__global__ void __launch_bounds__(kShares<NT * CG> * CG * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
+    static_assert(!DEEP || CG == 1, "the place of a warp's sums in tensor memory is that of its share");
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, COLS = 8 * NT, W = kShares<NT>;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp, g = lane >> 2, t = lane & 3;
+    constexpr int ROW = Lay<F>::ROW, TB = kTileBytes<F>, OWN = 8 * NT, COLS = OWN * CG, W = kShares<NT * CG>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp / CG, cg = warp % CG, g = lane >> 2, t = lane & 3;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int stages = p.stages;
     Shared rings = smem + share * (stages * T * TB);
@@ -667,12 +668,17 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
         if (iss < my_units) {
 #pragma unroll
             for (int i = 0; i < T; i++) {
+                if (CG > 1 && i % CG != cg) continue;           // (the warps of a share bring every CG-th tile)
                 const int tile = min(tile0 + i, p.tiles - 1);
                 issue_tile<F>(p, pc, pairs ? tile & 1 : 0, (pairs ? tile >> 1 : tile) * 16, share + iss * W, ring + (buf * T + i) * TB, lane);
             }
             iss++;
         }
         cp_async_commit();
+    };
+    auto meet = [&]() {                                         // the warps of a share
+        if (CG == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(share + 1), "n"(32 * CG) : "memory");
     };
     if (kNF4Like<F>) {                                          // (as above)
         fill_lut(smem + p.lut);
@@ -702,21 +708,21 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
             for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
     uint4 nh[NT], nl[NT];                                       // B operands of the next block
     auto fetch = [&](int blk) {
-        const uint4* src = p.planes + (size_t)blk * (NT * 64) + lane;
+        const uint4* src = p.planes + ((size_t)blk * CG + cg) * (NT * 64) + lane;
 #pragma unroll
         for (int j = 0; j < NT; j++) { nh[j] = __ldcg(src + j * 64); nl[j] = __ldcg(src + j * 64 + 32); }
     };
     if (my_units) fetch(share * 8);
     // exponent fields of what undoes the scaling of the warp's columns, unit after unit
-    uint8_t* const fields = smem + p.extra + 16 + warp * (COLS * ((units + W - 1) / W));
-    constexpr int WORDS = COLS / 4;
+    uint8_t* const fields = smem + p.extra + 16 + warp * (OWN * ((units + W - 1) / W));
+    constexpr int WORDS = OWN / 4;
     for (int i = lane; i < WORDS * my_units; i += 32) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.xf + (size_t)(share + i / WORDS * W) * COLS + 4 * (i % WORDS)));
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.xf + (size_t)(share + i / WORDS * W) * COLS + OWN * cg + 4 * (i % WORDS)));
         *reinterpret_cast<uint32_t*>(fields + 4 * i) = (__float_as_uint(v.x) >> 23) | (__float_as_uint(v.y) >> 23 << 8) | (__float_as_uint(v.z) >> 23 << 16) |
                                                        (__float_as_uint(v.w) >> 23 << 24);
     }
     __syncwarp();
-    auto undoes = [&](int u, int j) { return lds16(fields + COLS * u + 8 * j + 2 * t); };      // the thread's two columns of product j
+    auto undoes = [&](int u, int j) { return lds16(fields + OWN * u + 8 * j + 2 * t); };      // the thread's two columns of product j
     // a thread's place in tensor memory: its warp's 32 lanes, as many columns for each of the warps of a quadrant
     const uint32_t totals = DEEP ? *tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * (uint32_t)(1024 / W) : 0u;
     int buf = 0;
@@ -737,7 +743,7 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
         }
         if (stages > 1) cp_async_wait<1>();
         else cp_async_wait<0>();
-        __syncwarp();
+        meet();
         Shared base = rings + buf * T * TB + g * ROW;
 #pragma unroll 1
         for (int b = 0; b < 8; b++) {
@@ -749,7 +755,7 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
             float2 s32[NT];
             if (kMins<F>) {
 #pragma unroll
-                for (int j = 0; j < NT; j++) s32[j] = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * COLS + 8 * j + 2 * t));
+                for (int j = 0; j < NT; j++) s32[j] = __ldcg(reinterpret_cast<const float2*>(p.sums + (size_t)(un * 8 + b) * COLS + OWN * cg + 8 * j + 2 * t));
             }
 #pragma unroll
             for (int i = 0; i < T; i++) {
@@ -800,7 +806,7 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
                 }
             }
         }
-        __syncwarp();                                           // every lane is done with this buffer
+        meet();                                                 // every lane is done with this buffer
         issue(buf);
         if (++buf == stages) buf = 0;
         if (DEEP) {
@@ -851,7 +857,7 @@ __global__ void __launch_bounds__(kShares<NT> * 32, 1) gemv_split_wide_kernel(co
     for (int i = 0; i < T; i++)
 #pragma unroll
         for (int j = 0; j < NT; j++) {
-            float* dst = part + ((size_t)i * W + share) * (COLS * 16) + (8 * j + 2 * t) * 16 + g;
+            float* dst = part + ((size_t)i * W + share) * (COLS * 16) + (OWN * cg + 8 * j + 2 * t) * 16 + g;
             dst[0] = acc[i][j][0];
             dst[16] = acc[i][j][1];
             dst[8] = acc[i][j][2];
@@ -933,45 +939,53 @@ int run_narrow(SplitArgs& p, cudaStream_t st) {
     return launch_narrow<F, NT, QUIRK, ring>(p, W, st);
 }
 
-template <int F, int NT, int T, bool QUIRK, bool DEEP>
+template <int F, int NT, int CG, int T, bool QUIRK, bool DEEP>
 int run_wide(SplitArgs& p, cudaStream_t st) {
-    constexpr size_t stage = (size_t)kShares<NT> * T * kTileBytes<F>, sums = (size_t)T * 32 * 8 * 16 * 4;
-    const size_t extra = wide_extra<NT>(p);
-    p.stages = (p.K + 255) / 256 > kShares<NT> && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
+    constexpr size_t stage = (size_t)kShares<NT * CG> * T * kTileBytes<F>, sums = (size_t)T * 32 * 8 * 16 * 4;
+    const size_t extra = wide_extra<NT * CG>(p);
+    p.stages = (p.K + 255) / 256 > kShares<NT * CG> && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
     p.extra = (int)(p.stages * stage > sums ? p.stages * stage : sums);
     p.lut = (int)((p.extra + extra + 15) / 16 * 16);
     const size_t smem = kNF4Like<F> ? (size_t)p.lut + kLutBytes : p.extra + extra;
-    auto kern = gemv_split_wide_kernel<F, NT, T, QUIRK, DEEP>;
+    auto kern = gemv_split_wide_kernel<F, NT, CG, T, QUIRK, DEEP>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
-    return launch_split(kern, (p.tiles + T - 1) / T, kShares<NT>, smem, st, p);
+    return launch_split(kern, (p.tiles + T - 1) / T, kShares<NT * CG> * CG, smem, st, p);
 }
 
-template <int F, int NT, bool QUIRK, bool DEEP>
+template <int F, int NT, int CG, bool QUIRK, bool DEEP>
 int run_wide_t(SplitArgs& p, cudaStream_t st) {
-    constexpr int most = kSmemMost<F> / (kShares<NT> * kTileBytes<F>);
+    constexpr int most = kSmemMost<F> / (kShares<NT * CG> * kTileBytes<F>);
     const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
     int best = 1;
     double least = 1e30;
     for (int i = 0; i < 4; i++) {
         const int T = choice[i];
         if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
-        if (T > 1 && (size_t)kShares<NT> * T * kTileBytes<F> + wide_extra<NT>(p) > kSmemMost<F>) continue;
+        if (T > 1 && (size_t)kShares<NT * CG> * T * kTileBytes<F> + wide_extra<NT * CG>(p) > kSmemMost<F>) continue;
         const int ctas = (p.tiles + T - 1) / T;
         const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
         if (cost < least) { least = cost; best = T; }
     }
-    if constexpr (most >= 5) if (best == 5) return run_wide<F, NT, 5, QUIRK, DEEP>(p, st);
-    if constexpr (most >= 3) if (best == 3) return run_wide<F, NT, 3, QUIRK, DEEP>(p, st);
-    if (best == 2) return run_wide<F, NT, 2, QUIRK, DEEP>(p, st);
-    return run_wide<F, NT, 1, QUIRK, DEEP>(p, st);
+    if constexpr (most >= 5) if (best == 5) return run_wide<F, NT, CG, 5, QUIRK, DEEP>(p, st);
+    if constexpr (most >= 3) if (best == 3) return run_wide<F, NT, CG, 3, QUIRK, DEEP>(p, st);
+    if (best == 2) return run_wide<F, NT, CG, 2, QUIRK, DEEP>(p, st);
+    return run_wide<F, NT, CG, 1, QUIRK, DEEP>(p, st);
 }
+
+// Up to so many units of a row, 17 rows of x and more have sixteen warps with half the columns each: of eight, only as many as there are
+// units would work, and the launch is as long as one of those. us, 32 rows, eight warps and sixteen: Q8_0 10000x256 11.5 9.5, Q4_0
+// 17616x1280 27.3 24.7, NF4 20000x512 35.0 26.2, 20000x1536 47.8 41.1; three and four units are even, seven and more are for the eight.
+// Q4_K, Q5_K and Q6_K, whose unpacking costs most, are from three units on (Q6_K 10000x1024 14.1 17.3).
+template <int F> constexpr int kFewUnits = F == CMLB200_Q4_K || F == CMLB200_Q5_K || F == CMLB200_Q6_K ? 2 : 6;
 
 template <int F, int NT, bool QUIRK>
 int run_wide_d(SplitArgs& p, cudaStream_t st) {
     if constexpr (kNF4Like<F> || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
-        if (p.deep) return run_wide_t<F, NT, QUIRK, true>(p, st);
-    return run_wide_t<F, NT, QUIRK, false>(p, st);
+        if (p.deep) return run_wide_t<F, NT, 1, QUIRK, true>(p, st);
+    if constexpr (NT == 4)
+        if ((p.K + 255) / 256 <= kFewUnits<F>) return run_wide_t<F, 2, 2, QUIRK, false>(p, st);
+    return run_wide_t<F, NT, 1, QUIRK, false>(p, st);
 }
 
 template <int F, bool QUIRK>
