@@ -668,8 +668,10 @@ static int launch_residual(float* d_x, const float* d_y, int ldy, const cmlb200_
     // few rows: enough threads that each meets its row once; many rows: small CTAs, several to an SM
     int threads = 256;
     if (rows <= 2 * cmlb_num_sms()) while (threads < 1024 && threads * 4 < dim) threads *= 2;
-    // held in registers: 1,024 threads of them leave an SM no second CTA, so up to one row an SM (296x4096 5.8 us so, 5.4 us in shared memory)
-    if (vec && !parts && dim <= 8 * threads && (threads < 1024 || rows <= cmlb_num_sms())) {
+    // held in registers: 1,024 threads of them leave an SM no second CTA, so up to one row an SM (296x4096 5.8 us so, 5.4 us in shared memory). Many
+    // rows: fewer CTAs fit, which is made up for where a row waits for y and is not too short (2,000 rows of 256 5.8 and 5.6, of 2,048 9.2 and 9.5)
+    const bool held = rows > 2 * cmlb_num_sms() ? d_y && dim >= 768 : threads < 1024 || rows <= cmlb_num_sms();
+    if (vec && !parts && dim <= 8 * threads && held) {
 #define RN_HELD(TO, H) CMLB_CUDA(launch_chain(residual_norm_held_kernel<TO, H>, dim3(rows), dim3(threads), 0, 1, st, d_x, d_y, ldy, d_w_post, d_w_next, eps, dim, d_row_idx, (TO*)d_out, ldo, raw))
         const bool once = dim <= 4 * threads;
         if (out_dtype == CMLB200_DT_BF16) { if (once) RN_HELD(__nv_bfloat16, 1); else RN_HELD(__nv_bfloat16, 2); }
