@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
 // ---- 9 to 32 rows of x --------------------------------------------------------------------------------------------------------
 // A warp has NT products of eight columns of x and a share of K. CG = 1: all columns of x, sixteen warps up to 16 rows of x, eight with twice
 // the registers beyond, so that weights are unpacked once for 32 rows and the chains of a block's products are four. CG = 2: sixteen
-// warps, two of them for a share, each with its half of 32 columns; for short rows (kFewUnits). Longer ones of 17 to 32 rows take 29.2 us
+// warps, two of them for a share, each with its half of 32 columns; for short rows (few_units). Longer ones of 17 to 32 rows take 29.2 us
 // so where eight warps take 27.6 (Q4_0 11008x4096; Q4_K 4096x11008 45.4 and 37.5, Q6_K 32000x4096 135 and 101).
 template <int F, int NT, int CG, int T, bool QUIRK, bool DEEP>
 __global__ void __launch_bounds__(kShares<NT * CG> * CG * 32, 1) gemv_split_wide_kernel(const SplitArgs p) {
@@ -973,18 +973,22 @@ int run_wide_t(SplitArgs& p, cudaStream_t st) {
     return run_wide<F, NT, CG, 1, QUIRK, DEEP>(p, st);
 }
 
-// Up to so many units of a row, 17 rows of x and more have sixteen warps with half the columns each: of eight, only as many as there are
-// units would work, and the launch is as long as one of those. us, 32 rows, eight warps and sixteen: Q8_0 10000x256 11.5 9.5, Q4_0
-// 17616x1280 27.3 24.7, NF4 20000x512 35.0 26.2, 20000x1536 47.8 41.1; three and four units are even, seven and more are for the eight.
-// Q4_K, Q5_K and Q6_K, whose unpacking costs most, are from three units on (Q6_K 10000x1024 14.1 17.3).
-template <int F> constexpr int kFewUnits = F == CMLB200_Q4_K || F == CMLB200_Q5_K || F == CMLB200_Q6_K ? 2 : 6;
+// Rows of few units: 17 rows of x and more have sixteen warps with half the columns each: of eight, only as many as there are units would work,
+// and the launch is as long as one of those. us, 32 rows, eight warps and sixteen: Q8_0 10000x256 11.5 9.5, Q4_0 17616x1280 27.3 24.7, NF4
+// 20000x512 35.0 26.2, 20000x1536 47.8 41.1; three and four units are even, seven and more are for the eight. Q4_K, Q5_K and Q6_K, whose unpacking
+// costs most, are for eight from three units on where a CTA has several row tiles (Q6_K 10000x1024 14.1 17.3; Q4_K 2048x768 8.1 7.4).
+template <int F> bool few_units(const SplitArgs& p) {
+    const int units = (p.K + 255) / 256;
+    const bool heavy = F == CMLB200_Q4_K || F == CMLB200_Q5_K || F == CMLB200_Q6_K;
+    return units <= 2 || (units <= 6 && (!heavy || p.tiles <= cmlb_num_sms()));
+}
 
 template <int F, int NT, bool QUIRK>
 int run_wide_d(SplitArgs& p, cudaStream_t st) {
     if constexpr (kNF4Like<F> || F == CMLB200_Q6_K || F == CMLB200_Q8_0)
         if (p.deep) return run_wide_t<F, NT, 1, QUIRK, true>(p, st);
     if constexpr (NT == 4)
-        if ((p.K + 255) / 256 <= kFewUnits<F>) return run_wide_t<F, 2, 2, QUIRK, false>(p, st);
+        if (few_units<F>(p)) return run_wide_t<F, 2, 2, QUIRK, false>(p, st);
     return run_wide_t<F, NT, 1, QUIRK, false>(p, st);
 }
 
