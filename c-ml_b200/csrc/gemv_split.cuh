@@ -37,13 +37,17 @@ enum { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2 };
 
 // Shared memory of one weight row's 256-column unit: bytes of quants (and headers) as they lie in memory, block scales
 // behind them. Row strides are odd multiples of 16 bytes (mod 128), so eight rows hit eight bank groups.
-constexpr int kNF4Fine = CMLB200_NF4 + 1;
-template <int F> constexpr bool kNF4Like = F == CMLB200_NF4 || F == kNF4Fine;
+// NF4: of blocks of 64 and more, of blocks of 32; both without the table of codes
+constexpr int kNF4Fine = CMLB200_NF4 + 1, kNF4Bare = CMLB200_NF4 + 2, kNF4FineBare = CMLB200_NF4 + 3;
+template <int F> constexpr bool kNF4Like = F >= CMLB200_NF4 && F <= kNF4FineBare;
+template <int F> constexpr bool kTable = F == CMLB200_NF4 || F == kNF4Fine;
 template <int F> struct Lay;
 template <> struct Lay<CMLB200_Q4_0> { static constexpr int ROW = 144, CH = 8, SC = 128; };
 template <> struct Lay<CMLB200_Q8_0> { static constexpr int ROW = 272, CH = 16, SC = 256; };
 template <> struct Lay<CMLB200_NF4> { static constexpr int ROW = 144, CH = 8, SC = 128; };         // blocks of 64 and more
 template <> struct Lay<kNF4Fine> { static constexpr int ROW = 176, CH = 8, SC = 128; };            // of 32: eight scales
+template <> struct Lay<kNF4Bare> : Lay<CMLB200_NF4> {};
+template <> struct Lay<kNF4FineBare> : Lay<kNF4Fine> {};
 template <> struct Lay<CMLB200_Q4_1> { static constexpr int ROW = 176, CH = 10, SC = 0; };
 template <> struct Lay<CMLB200_Q4_K> { static constexpr int ROW = 144, CH = 9, SC = 0; };
 template <> struct Lay<CMLB200_Q5_K> { static constexpr int ROW = 176, CH = 11, SC = 0; };
@@ -217,7 +221,23 @@ __device__ __forceinline__ void row_regs(Shared at, int b, int t, uint32_t w0, u
             h[0][2 * k] = hadd2u(and_or(hb * 0x00010010u, 0x00300030u, and_or(w, 0x000f000fu, 0x64006400u)), 0xe420e420u);              // - 1056
             h[0][2 * k + 1] = hadd2u(and_or(hb * 0x00004004u, 0x00300030u, and_or(w >> 4, 0x000f000fu, 0x64006400u)), 0xe420e420u);
         }
-    } else {                                                    // NF4: 10000 times the code = 128 a + b; a byte's two codes from a table
+    } else if constexpr (!kTable<F>) {                          // NF4: 10000 times the code = 128 a + b, digits by byte table look-ups
+        // a + 128 and b + 128 of the 16 codes (|b| <= 64), four to a word
+        constexpr uint32_t A0 = 0x61574a32u, A1 = 0x8079726au, A2 = 0x9a938d86u, A3 = 0xceb8aca2u;
+        constexpr uint32_t B0 = 0x937d4e70u, B1 = 0x80714864u, B2 = 0xb39d499cu, B3 = 0x90be7ab7u;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t w = k ? w0 >> 16 : w0;
+            const uint32_t s = w & 0x7777u, pick = and_or(w >> 1, 0x4444u, 0x3210u);
+            const uint32_t va = __byte_perm(__byte_perm(A0, A1, s), __byte_perm(A2, A3, s), pick);
+            const uint32_t vb = __byte_perm(__byte_perm(B0, B1, s), __byte_perm(B2, B3, s), pick);
+            // bytes: columns 1, 0, 3, 2. 1024 + (a + 128) -> a * 2^-7, 1024 + (b + 128) -> b * 2^-14
+            h[0][2 * k] = hfma2u(__byte_perm(va, 0x64646464u, 0x4041), 0x20002000u, 0xc880c880u);
+            h[0][2 * k + 1] = hfma2u(__byte_perm(va, 0x64646464u, 0x4243), 0x20002000u, 0xc880c880u);
+            h[1][2 * k] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4041), 0x04000400u, 0xac80ac80u);
+            h[1][2 * k + 1] = hfma2u(__byte_perm(vb, 0x64646464u, 0x4243), 0x04000400u, 0xac80ac80u);
+        }
+    } else {                                                    // a byte's two codes from a table
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const uint2 v = *reinterpret_cast<const uint2*>(lut + ((k ? w0 >> (8 * k - 7) : w0 << 7) & 0x7f80u));
@@ -435,12 +455,12 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_split_kernel(const SplitA
     };
     // weights do not depend on the launch before, but NF4 ones may: it may have quantized them, or written their scales
     if (kNF4Like<F>) {
-        fill_lut(smem + p.lut);
+        if (kTable<F>) fill_lut(smem + p.lut);
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
 #pragma unroll
     for (int i = 0; i < RING; i++) issue(i);
-    Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
+    Shared lut = smem + (kTable<F> ? p.lut + (lane & 15) * 8 : 0);
     if (!kNF4Like<F>) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
@@ -681,12 +701,12 @@ __global__ void __launch_bounds__(kShares<NT * CG> * CG * 32, 1) gemv_split_wide
         else asm volatile("bar.sync %0, %1;" ::"r"(share + 1), "n"(32 * CG) : "memory");
     };
     if (kNF4Like<F>) {                                          // (as above)
-        fill_lut(smem + p.lut);
+        if (kTable<F>) fill_lut(smem + p.lut);
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     issue(0);
     if (stages > 1) issue(1);
-    Shared lut = smem + (kNF4Like<F> ? p.lut + (lane & 15) * 8 : 0);
+    Shared lut = smem + (kTable<F> ? p.lut + (lane & 15) * 8 : 0);
     uint32_t* const tmem = reinterpret_cast<uint32_t*>(smem + p.extra);
     if (DEEP) {
         if (warp == 0) {
@@ -897,7 +917,7 @@ int launch_split(Kern kern, int grid, int warps, size_t smem, cudaStream_t st, c
     return CMLB200_OK;
 }
 
-template <int F> constexpr size_t kSmemMost = 227 * 1024 - (kNF4Like<F> ? kLutBytes + 16 : 0);      // besides the table
+template <int F> constexpr size_t kSmemMost = 227 * 1024 - (kTable<F> ? kLutBytes + 16 : 0);      // besides the table
 template <int NT> size_t wide_extra(const SplitArgs& p) { return 16 + (size_t)kShares<NT> * 8 * NT * (((p.K + 255) / 256 + kShares<NT> - 1) / kShares<NT>); }
 
 constexpr int kMostTiles = 6;                                            // row tiles of a CTA
@@ -907,10 +927,20 @@ template <int F, int NT> constexpr size_t narrow_smem(int ring, int W, int M, in
     return (size_t)W * ring * kTileBytes<F> + (NT == 0 ? (size_t)W * (M * kXBytes + kOwnBytes) : 0) + ((size_t)per * W * (NT == 0 ? 4 : 8) * 16 + W * 4) * sizeof(float);
 }
 
+// Warps and row tiles of a CTA: as many tiles as fill the SMs once, or several times where that would be more than six (5 tiles of
+// 11008 rows: 8.2 us at M = 1; 3: 11.4, 2: 13.3, for every CTA makes the operands of x again)
+struct Narrow { int W, per, rounds; };
+inline Narrow narrow_plan(const SplitArgs& p) {
+    const int units = (p.K + 255) / 256, sms = cmlb_num_sms();
+    const int want = (p.tiles + sms - 1) / sms, rounds = (want + kMostTiles - 1) / kMostTiles;
+    const int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
+    return {units < kWarps ? units : kWarps, p.epi == EPI_SWIGLU ? (per + 1) & ~1 : per, rounds};
+}
+
 template <int F, int NT, bool QUIRK, int RING>
 int launch_narrow(SplitArgs& p, int W, cudaStream_t st) {
     size_t smem = narrow_smem<F, NT>(RING, W, p.M, p.per_cta);
-    if (kNF4Like<F>) {
+    if (kTable<F>) {
         p.lut = (int)((smem + 15) / 16 * 16);
         smem = p.lut + kLutBytes;
     }
@@ -922,13 +952,8 @@ int launch_narrow(SplitArgs& p, int W, cudaStream_t st) {
 
 template <int F, int NT, bool QUIRK>
 int run_narrow(SplitArgs& p, cudaStream_t st) {
-    const int units = (p.K + 255) / 256, W = units < kWarps ? units : kWarps, sms = cmlb_num_sms();
-    // as many row tiles a CTA as fill the SMs once, or several times where that would be more than six (5 tiles of 11008 rows:
-    // 8.2 us at M = 1; 3: 11.4, 2: 13.3, for every CTA makes the operands of x again)
-    const int want = (p.tiles + sms - 1) / sms, rounds = (want + kMostTiles - 1) / kMostTiles;
-    int per = (p.tiles + sms * rounds - 1) / (sms * rounds);
-    if (p.epi == EPI_SWIGLU) per = (per + 1) & ~1;
-    p.per_cta = per;
+    const Narrow n = narrow_plan(p);
+    const int W = n.W, per = p.per_cta = n.per;
     // sixteen warps, four rows, six tiles: where that is too much (NF4, blocks of 64 and more), such calls have rings of two
     // (13824x5120, 4 rows: 25.5 us; without the table, whose place a third item took, 32.4)
     constexpr int ring = kRing<F, NT>;
@@ -946,27 +971,36 @@ int run_wide(SplitArgs& p, cudaStream_t st) {
     p.stages = (p.K + 255) / 256 > kShares<NT * CG> && 2 * stage + extra <= kSmemMost<F> ? 2 : 1;
     p.extra = (int)(p.stages * stage > sums ? p.stages * stage : sums);
     p.lut = (int)((p.extra + extra + 15) / 16 * 16);
-    const size_t smem = kNF4Like<F> ? (size_t)p.lut + kLutBytes : p.extra + extra;
+    const size_t smem = kTable<F> ? (size_t)p.lut + kLutBytes : p.extra + extra;
     auto kern = gemv_split_wide_kernel<F, NT, CG, T, QUIRK, DEEP>;
     static size_t done[kMaxDevices] = {};
     CMLB_CUDA(cmlb_ensure_smem(kern, smem, done));
     return launch_split(kern, (p.tiles + T - 1) / T, kShares<NT * CG> * CG, smem, st, p);
 }
 
-template <int F, int NT, int CG, bool QUIRK, bool DEEP>
-int run_wide_t(SplitArgs& p, cudaStream_t st) {
-    constexpr int most = kSmemMost<F> / (kShares<NT * CG> * kTileBytes<F>);
+// Row tiles of a CTA: waves of CTAs, a CTA as long as its tiles and one and a half more
+template <int F, int N8> constexpr int kMostWide = kSmemMost<F> / (kShares<N8> * kTileBytes<F>);
+template <int F, int N8> int wide_tiles(const SplitArgs& p, double* cost_out) {
     const int sms = cmlb_num_sms(), choice[4] = {1, 2, 3, 5};
     int best = 1;
     double least = 1e30;
     for (int i = 0; i < 4; i++) {
         const int T = choice[i];
-        if (T > most || (p.epi == EPI_SWIGLU && T != 2)) continue;
-        if (T > 1 && (size_t)kShares<NT * CG> * T * kTileBytes<F> + wide_extra<NT * CG>(p) > kSmemMost<F>) continue;
+        if (T > kMostWide<F, N8> || (p.epi == EPI_SWIGLU && T != 2)) continue;
+        if (T > 1 && (size_t)kShares<N8> * T * kTileBytes<F> + wide_extra<N8>(p) > kSmemMost<F>) continue;
         const int ctas = (p.tiles + T - 1) / T;
         const double cost = (double)((ctas + sms - 1) / sms) * (T + 1.5);
         if (cost < least) { least = cost; best = T; }
     }
+    *cost_out = least;
+    return best;
+}
+
+template <int F, int NT, int CG, bool QUIRK, bool DEEP>
+int run_wide_t(SplitArgs& p, cudaStream_t st) {
+    constexpr int most = kMostWide<F, NT * CG>;
+    double cost;
+    const int best = wide_tiles<F, NT * CG>(p, &cost);
     if constexpr (most >= 5) if (best == 5) return run_wide<F, NT, CG, 5, QUIRK, DEEP>(p, st);
     if constexpr (most >= 3) if (best == 3) return run_wide<F, NT, CG, 3, QUIRK, DEEP>(p, st);
     if (best == 2) return run_wide<F, NT, CG, 2, QUIRK, DEEP>(p, st);

@@ -84,6 +84,41 @@ def test_nf4_swiglu_of_large_pairs(pkg, synth, ob, orc, torch_dev, N, K, M):
     assert ((y.double() - silu * u).abs() <= 1.1 * dg * (u.abs() + du) + silu.abs() * du + 2.0 ** -20 * (silu * u).abs()).all()
 
 
+@pytest.mark.parametrize("kind,block", [("q8_0", 32), ("q4_1", 32), ("q6_k", 32), ("nf4", 64), ("nf4", 32)])
+@pytest.mark.parametrize("N,K", [(24, 256), (2400, 512), (80, 768), (4752, 1280), (33, 1536), (49, 1792)])
+def test_short_rows_of_large_batches(pkg, synth, ob, orc, torch_dev, kind, block, N, K):
+    """17 to 32 rows of x where a row's units of columns are fewer than the warps that share them: on both sides of the line."""
+    rng = np.random.default_rng(N + K)
+    W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, kind, N, K, block)
+    for M in (17, 24, 32):
+        _check(pkg, W, Wf, rng.standard_normal((M, K)).astype(np.float32), torch_dev)
+
+
+@pytest.mark.parametrize("N,K,block,M,pair", [(700, 512, 64, 6, False), (4100, 768, 32, 5, False), (20000, 2048, 64, 4, False), (14300, 2048, 32, 8, False),
+                                              (28660, 256, 64, 5, True), (20000, 1024, 32, 7, True), (20000, 1024, 64, 4, True), (9000, 1024, 64, 13, True),
+                                              (5000, 768, 32, 30, True), (10000, 320, 32, 12, False), (10000, 8512, 32, 16, False), (400, 512, 64, 32, False)])
+def test_nf4_codes_with_and_without_the_table(pkg, synth, ob, orc, torch_dev, N, K, block, M, pair):
+    """Where NF4 codes come by byte permutes: a few items a CTA, several CTAs an SM, short pairs, five row tiles of blocks of 32. The bounds are
+    those of test_nf4_swiglu_of_large_pairs."""
+    rng = np.random.default_rng(N + K + M)
+    X = to_dev(rng.standard_normal((M, K)).astype(np.float32), torch_dev)
+    off, of, weights = 2.0 ** -21 + (K / 32 + 32) * 2.0 ** -23, [], []
+    for _ in range(1 + pair):
+        W, Wf = _weight(pkg, synth, ob, orc, torch_dev, rng, "nf4", N, K, block)
+        F = to_dev(Wf, torch_dev).double()
+        weights.append(W)
+        of.append((X.double() @ F.T, off * (X.double().abs() @ F.abs().T)))
+    y = torch.full((M, N), float("nan"), device=torch_dev)
+    if pair:
+        pkg.check(pkg.lib.cmlb200_gemv_swiglu(weights[0].q, weights[1].q, X.data_ptr(), y.data_ptr(), M, stream_ptr()), "swiglu")
+        (g, dg), (u, du) = of
+        silu = g / (1 + torch.exp(-g))
+        assert ((y.double() - silu * u).abs() <= 1.1 * dg * (u.abs() + du) + silu.abs() * du + 2.0 ** -20 * (silu * u).abs()).all()
+    else:
+        pkg.check(pkg.lib.cmlb200_gemv(weights[0].q, X.data_ptr(), y.data_ptr(), M, stream_ptr()), "gemv")
+        assert ((y.double() - of[0][0]).abs() <= of[0][1]).all()
+
+
 @pytest.mark.parametrize("scale", [1e-30, 1e-6, 1e6, 1e30])
 @pytest.mark.parametrize("M", [3, 7, 20])
 def test_any_range_of_x(pkg, synth, ob, orc, torch_dev, scale, M):
