@@ -11,14 +11,14 @@
 #include "gemv_paths.cuh"
 
 // Where the fp16-split kernels (gemv_split.cuh) are the faster ones. us a call, weights from memory, [this | the alternative]:
-//   Q4_0  11008x4096: M = 1 8.3 | 6.7, 3 9.6 | 13.6 (two launches of the alternative), 4 10.0 | 9.4, 8 12.9 | 12.9, 16 17.7 | 24.8,
+//   Q4_0  11008x4096: M = 1 8.3 | 6.7, 3 9.6 | 13.6 (two launches of the alternative), 4 10.0 | 9.4, 8 12.9 | 12.9, 16 17.5 | 24.8,
 //         32 27.6 | 48.3: at 1, 2 and 4 rows the int8-digit kernel fits its columns exactly, from 9 on it makes several passes
-//   Q8_0  4096x4096: 1 5.6 | 4.6, 2 6.3 | 5.1 (4096x11008: 13.5 | 17.9, two launches), 3 6.8 | 9.3, 8 7.8 | 14.1, 32 14.5 | 82.6
-//   NF4 4096x4096: 1 7.8 | 63.5, 4 9.6 | 70.5, 32 20.5 | 562; Q4_K: 1 5.9 | 7.4, 8 9.6 | 22.9, 32 21.0 | 83.8; Q6_K: 1 7.4 | 9.7, 8 8.9 | 27.3,
-//         32 21.6 | 109.9; Q4_1: 1 5.8 | 7.3, 32 15.9 | 79.9 (the alternative of the GGUF types, gemv_kquant.cu, is left with columns
+//   Q8_0  4096x4096: 1 5.6 | 4.6, 2 6.3 | 5.1 (4096x11008: 14.0 | 17.9, two launches), 3 6.9 | 9.3, 8 8.2 | 14.1, 32 14.6 | 82.6
+//   NF4 4096x4096: 1 7.9 | 63.5, 4 9.7 | 70.5, 32 21.6 | 562; Q4_K: 1 5.5 | 7.4, 8 7.7 | 22.9, 32 15.8 | 83.8; Q6_K: 1 7.4 | 9.7, 8 8.8 | 27.3,
+//         32 16.2 | 109.9; Q4_1: 1 5.7 | 7.3, 32 15.5 | 79.9 (the alternative of the GGUF types, gemv_kquant.cu, is left with columns
 //         that are no whole 256 and short rows at M = 1: 16 warps share the 256-column units of a row, Q6_K 4608x1536 6.3 | 5.5).
-//         Q8_0 7424x3840: 4 9.3 | 8.7
-//   Q5_K  11008x4096: 1 15.2 | 14.9, 2 15.8 | 23.5, 32 49.8 | 189.5; 1024x4096: 1 4.6 | 5.5
+//         Q8_0 7424x3840: 4 9.0 | 8.7
+//   Q5_K  11008x4096: 1 15.2 | 14.8, 2 15.5 | 23.5, 32 39.2 | 189.5; 1024x4096: 1 4.6 | 5.4
 // Pairs of up to three rows (SwiGLU; two launches of the alternative): not with up to 4,096 columns where a CTA's row tiles would be more
 // than six, for they go in rounds then whose last is short (Q8_0 of two rows and up to 2,048 columns: four). 4096 columns, RMS norm first:
 //   Q8_0 M = 2  2048 rows 7.2 | 10.4, 6144 12.6 | 17.7, 11008 24.5 | 22.7, 14336 35.4 | 30.6, 32000 62.4 | 57.2, 8192x8192 33.9 | 51.2,

@@ -17,13 +17,13 @@
 //                       warp itself (columns 2r, 2r+1 = hi, lo of row r); NT = 1: 5 to 8 rows, planes from x_split_kernel.
 //                       A warp keeps the B operands of its unit in registers and walks the CTA's row tiles.
 //   gemv_split_wide_kernel   9 to 32 rows: B operands are loaded per block and used by T row tiles whose sums stay in registers;
-//                       a warp has all columns of x.
+//                       a warp has all columns of x, of short rows half of them.
 //
 // What bounds it: instructions and the chains between them. A block of 16 x 32 weights at M = 1 takes a thread about 50 (10 to unpack, 6 to
 // address and load, 2 products, 8 to apply the scales, the rest the rows of x); logic operations, permutes and packed halves issue every
-// second cycle; tensor pipe 41 % busy at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers)
+// second cycle; tensor pipe 44 % busy at M = 32 (mma.sync: 2 cycles a product and SM), DRAM 24 % at M = 1. Sixteen warps (128 registers)
 // beat eight with 255 up to 16 rows: 8.2 against 10.4 us at M = 1 (Q4_0 11008x4096), 9.9 against 11.4 at M = 16 (4096x4096); from 17 rows
-// on eight are the faster ones. More chains of products (the block's halves apart) cost more additions than they hid: 14.3 against
+// on eight are the faster ones, but for short rows. More chains of products (the block's halves apart) cost more additions than they hid: 14.3 against
 // 12.9 us at M = 8. The same products by tcgen05.mma, weights put into tensor memory block by block, were no faster: a block's sums have a
 // place of their own there and are read back, and every step of that pipeline (a wait, two fences, an arrival, 550 cycles from an
 // MMA to who waits for it) costs more than the mma.sync it saves: 34.5 us at M = 32, 17.4 at M = 16 (Q4_0 11008x4096). Times: gemv.cu.
