@@ -709,6 +709,9 @@ const int* clusters_at_once(Kern kern, size_t smem) {
 // us more: 7 % rms then, the shape picked 0.3 % off the best one on average. What the sum takes now (about 1.2 + 0.009 NX + 0.15 ranks)
 // would change the pick of one call in twenty, by 1 to 5 % of the estimate, less than its error. 4096x4096, Q4_0, 77 rows: 13.9 us
 // with four ranks (32 of the 33 clusters that fit); with the former sum 14.2, 16.0 with three, 27.1 without.
+// What it picks above 256 rows, pairs or not, against the best form without pairs (1, 2, 4 or 8 CTAs to a tile; three formats, ten shapes of weights,
+// 257 to 2048 rows, 210 calls): 0.86 of its time on average, 0.68 at 32000x4096 (Q4_0, 512 rows: 99.8 and 128 us; 257: 68.2 and 112); more than 3 %
+// behind it in nine calls, the worst of short K (NF4 4096x1024, 257 rows: 13.8 and 11.9), where a pair's MMA and expansion do not add up as the estimate has it.
 inline double shape_cost(const Shape& s, int M, int N, int KB, const int* at_once, double expand) {
     const int together = s.pair ? 2 : s.ranks, rows = s.pair ? 2 * BN : BN;
     if (!at_once[together] || (s.ranks > 1 && s.NX > B_ROWS)) return 1e30;
